@@ -90,6 +90,31 @@ __device__ __forceinline__ T load_key(const T* p) {
 template <bool INCL, typename T>
 __device__ __forceinline__ bool lt(T a, T b) { return INCL ? (a <= b) : (a < b); }
 
+// if (lt(a, b)) r = imm.  The assignment is a predicated multiply-add r * zero +
+// imm (`zero`: 0, unknown to the compiler): a select would go to the ALU pipe,
+// which the ladder's compares already keep busy.
+template <bool INCL>
+__device__ __forceinline__ void take_if_lt(int& r, int32_t a, int32_t b, int zero, int imm) {
+    if constexpr (INCL)
+        asm("{\n\t.reg .pred p;\n\tsetp.le.s32 p, %1, %2;\n\t@p mad.lo.s32 %0, %0, %3, %4;\n\t}" : "+r"(r) : "r"(a), "r"(b), "r"(zero), "r"(imm));
+    else
+        asm("{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %1, %2;\n\t@p mad.lo.s32 %0, %0, %3, %4;\n\t}" : "+r"(r) : "r"(a), "r"(b), "r"(zero), "r"(imm));
+}
+template <bool INCL>
+__device__ __forceinline__ void take_if_lt(int& r, float a, float b, int zero, int imm) {
+    if constexpr (INCL)
+        asm("{\n\t.reg .pred p;\n\tsetp.le.f32 p, %1, %2;\n\t@p mad.lo.s32 %0, %0, %3, %4;\n\t}" : "+r"(r) : "f"(a), "f"(b), "r"(zero), "r"(imm));
+    else
+        asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, %2;\n\t@p mad.lo.s32 %0, %0, %3, %4;\n\t}" : "+r"(r) : "f"(a), "f"(b), "r"(zero), "r"(imm));
+}
+template <bool INCL>
+__device__ __forceinline__ void take_if_lt(int& r, int64_t a, int64_t b, int zero, int imm) {
+    if constexpr (INCL)
+        asm("{\n\t.reg .pred p;\n\tsetp.le.s64 p, %1, %2;\n\t@p mad.lo.s32 %0, %0, %3, %4;\n\t}" : "+r"(r) : "l"(a), "l"(b), "r"(zero), "r"(imm));
+    else
+        asm("{\n\t.reg .pred p;\n\tsetp.lt.s64 p, %1, %2;\n\t@p mad.lo.s32 %0, %0, %3, %4;\n\t}" : "+r"(r) : "l"(a), "l"(b), "r"(zero), "r"(imm));
+}
+
 // ---------------------------------------------------------------------------
 // 128-byte swizzle.  A TMA tile with CU_TENSOR_MAP_SWIZZLE_128B and a 128-byte
 // inner box row stores 16-byte chunk c of row r at chunk c ^ (r % 8) (smem

@@ -8,25 +8,27 @@
 // memory.  One __syncthreads publishes the claim; after it the warps
 // synchronise only with __syncwarp.
 //
-//  Phase 1, per warp tile (the next tiles' 128-byte-swizzled TMA loads stay
-//  in flight in the warp's ring):
-//   1. in-thread answers over IPT consecutive keys in registers (compare
-//      ladder) -- the in-thread step of apsepKernelSPT (src/apsep.cuh:2701-2707);
-//   2. warp prefix minima over lane minima (src/apsep.cuh:2709-2730);
-//   3. each key without an in-thread answer is classified: answered by an
-//      earlier lane of the tile (X), by an earlier tile of the range (S), or by
-//      nothing in the range (deferred);
-//   4. X keys, spread evenly over the lanes, find their lane by binary lifting
-//      over a 5-level table of lane minima held in registers and their key by
-//      binary search over that lane's suffix minima -- a fixed number of
-//      steps in place of the reference's warp-uniform pointer jumping, spine
-//      walk and cross-warp fallback (src/apsep.cuh:2734-2801);
-//   5. S keys search the warp's RANGE STACK (strict suffix minima of the
-//      range's earlier tiles; its top 32 entries one per lane, a shuffle
-//      search, binary search below), in place of the reference's global
-//      min-tree descent (src/apsep.cuh:2952-2996) for every answer inside the
-//      range;
-//   6. the whole tile leaves shared memory in one TMA store, deferred keys as
+//  Phase 1, per warp tile (the next tile's 128-byte-swizzled TMA load stays in
+//  flight in the warp's ring):
+//   1. whole-tile paths for sorted keys (single arrays);
+//   2. in-thread answers over IPT consecutive keys in registers (compare
+//      ladder) -- the in-thread step of apsepKernelSPT (src/apsep.cuh:2701-2707)
+//      -- and, for a lane's first keys, over the four keys before the lane;
+//   3. minima over lanes (src/apsep.cuh:2709-2730) and the tile's strict suffix
+//      minima;
+//   4. the keys left over, spread evenly over the lanes, find the nearest
+//      earlier lane of the tile that qualifies by binary lifting over a 5-level
+//      table of lane minima held in registers and their key by binary search
+//      over that lane's suffix minima -- a fixed number of steps in place of
+//      the reference's warp-uniform pointer jumping, spine walk and cross-warp
+//      fallback (src/apsep.cuh:2734-2801);
+//   5. keys without an answer in the tile search the warp's RANGE STACK (strict
+//      suffix minima of the range's earlier tiles; its top 32 entries one per
+//      lane, a shuffle search, binary search below), in place of the
+//      reference's global min-tree descent (src/apsep.cuh:2952-2996) for every
+//      answer inside the range; the rest are flagged for phase 2: deferred
+//      (nothing in the range qualifies) or capped (the stack dropped the entry);
+//   6. the whole tile leaves shared memory in one TMA store, flagged keys as
 //      -1; the stack takes the tile's strict suffix minima.
 //  Then the warp publishes its range minimum and the top of its stack, and
 //  reads the exclusive prefix minimum P of the earlier ranges (one handshake
@@ -36,38 +38,57 @@
 //  Phase 2 touches only the flagged keys.  Deferred keys are the range's
 //  prefix minima, non-increasing, so the ones P qualifies form a prefix (the
 //  reference's prefix-min early-out, src/apsep.cuh:2903-2926); each finds
-//  the nearest earlier range whose minimum qualifies and its answer at the
-//  top of that range's published stack, all lanes in parallel.  Everything
-//  else (stacks that dropped entries, lists that overflowed) falls back to a
-//  warp-cooperative search down the min hierarchy (find_left).
+//  the nearest earlier range whose minimum qualifies and its answer in that
+//  range's published stack or its tile, chunk and key minima, 32 keys side by
+//  side (answer_before); capped keys search their own range's tiles
+//  (find_in_tiles).
+//
+//  On random keys the kernel is bound by the latency of its dependent steps
+//  and by issue (4 warps a scheduler; 58 % of issue slots and 50 % of the ALU
+//  pipe busy at 2^25 int32 keys): seeing four predecessors before any query,
+//  one list and one prefix sum per tile, no prefix scan and one query round
+//  took 2^25 uniform keys from 136 to 117 us (2.3 TB/s of useful bytes), the
+//  one-key-per-lane phase 2 with the longer stack and lists a random walk of
+//  2^24 keys (stock span) from 783 to 202 us and of 2^20 keys from 176 to 40.
 #pragma once
 #include "apsep_device.cuh"
 #include "apsep_internal.h"
 
 namespace apsep {
 
-constexpr int kStages = 3;      // TMA ring depth per warp (tiles)
-constexpr int kStackCap = 64;   // range-stack entries kept per warp
+// TMA ring depth per warp (tiles): two for 4-byte keys, one landing while one is
+// worked on (a third measured no gain, and its shared memory holds the longer
+// stack and lists); three for 8-byte keys, whose tiles are 256 keys (ascending
+// float64 keys, 2^26 of them: 207 us with two, 173 us with three).
+template <int KB> constexpr int kStagesOf = KB == 8 ? 3 : 2;
+// Range-stack entries kept per warp.  Random keys leave ~ln(range) suffix minima
+// (10 of 13,800 keys), a random walk ~sqrt(range) (130): with 64 entries every
+// second range of a walk dropped some and sent its keys to phase 2 as capped.
+template <int KB> constexpr int kStackCapOf = KB == 8 ? 128 : 256;
+constexpr int kUpKeep = 64;     // entries a wholly increasing tile leaves on the stack
 constexpr int kXQueries = 3;    // cross-lane queries per lane and round (32 * 3 keys per round)
-constexpr int kDefCap = 64;     // deferred keys listed in shared memory per range
-constexpr int kCapCap = 16;     // capped keys listed in shared memory per range
+// Deferred keys listed in shared memory per range (a random walk's prefix
+// minima, ~sqrt(range) of them, fit; 8-byte keys: what shared memory leaves).
+template <int KB> constexpr int kDefCapOf = KB == 8 ? 128 : 256;
+constexpr int kCapCap = 32;     // capped keys listed in shared memory per range
 
 // Shared memory of one warp (KB: bytes per key).
 template <int IPT, int KB = 4>
 struct WLayout {
     static constexpr int WT = 32 * IPT;                              // keys per warp tile
     static constexpr size_t kV = 0;                                   // T[S][WT], swizzled (TMA dst)
-    static constexpr size_t kO = kV + (size_t)kStages * WT * KB;      // int32[WT], swizzled (TMA src)
+    static constexpr size_t kO = kV + (size_t)kStagesOf<KB> * WT * KB;      // int32[WT], swizzled (TMA src)
     static constexpr size_t kSM = kO + (size_t)WT * 4;                // T[WT], swizzled: lane suffix minima
     static constexpr size_t kList = kSM + (size_t)WT * KB;            // int16[WT]: X keys in order
     static constexpr size_t kStkV = kList + (size_t)WT * 2;           // T[K]
-    static constexpr size_t kStkP = kStkV + (size_t)kStackCap * KB;   // int32[K]
-    static constexpr size_t kDefP = kStkP + (size_t)kStackCap * 4;    // int32[kDefCap]
-    static constexpr size_t kDefV = kDefP + (size_t)kDefCap * 4;      // T[kDefCap]
-    static constexpr size_t kCapP = kDefV + (size_t)kDefCap * KB;     // int32[kCapCap]
+    static constexpr size_t kStkP = kStkV + (size_t)kStackCapOf<KB> * KB;   // int32[K]
+    static constexpr size_t kDefP = kStkP + (size_t)kStackCapOf<KB> * 4;    // int32[kDefCap]
+    static constexpr size_t kDefV = kDefP + (size_t)kDefCapOf<KB> * 4;  // T[kDefCap]
+    static constexpr size_t kCapP = kDefV + (size_t)kDefCapOf<KB> * KB;  // int32[kCapCap]
     static constexpr size_t kCapS = kCapP + (size_t)kCapCap * 4;      // int32[kCapCap]: segment starts
-    static constexpr size_t kBar = (kCapS + (size_t)kCapCap * 4 + 7) / 8 * 8;  // uint64[S]
-    static constexpr size_t kEnd = kBar + (size_t)kStages * 8;
+    static constexpr size_t kPad = (kCapS + (size_t)kCapCap * 4 + 15) / 16 * 16;  // T[4]: pads (lane 0's earlier keys)
+    static constexpr size_t kBar = kPad + 4 * KB;  // uint64[S]
+    static constexpr size_t kEnd = kBar + (size_t)kStagesOf<KB> * 8;
     static constexpr size_t kBytes = (kEnd + 1023) / 1024 * 1024;     // keeps every warp 1024-aligned
     static_assert(kO % 1024 == 0 && kSM % 1024 == 0 && (WT * KB) % 1024 == 0,
                   "swizzled buffers need 1024-byte alignment");
@@ -107,33 +128,12 @@ template <typename T>
 __device__ __forceinline__ T group_min_of(const RangeArgs& a, int g) {
     if constexpr (sizeof(T) == 8) {
         T m = KeyTraits<T>::pad();
-        const int e = min(32 * g + 32, a.num_ranges);
-        for (int i = 32 * g; i < e; i++) m = KeyTraits<T>::vmin(m, range_min<T>(a, i));
+#pragma unroll
+        for (int i = 0; i < 32; i++) m = KeyTraits<T>::vmin(m, range_min<T>(a, min(32 * g + i, a.num_ranges - 1)));
         return m;
     } else {
         return group_key<T>(&a.s.group_min[g]);
     }
-}
-
-// ---------------------------------------------------------------------------
-// Warp-cooperative search: the rightmost position p < limit with
-// lt(d_in[p], q), or -1 (-2 if the published minima contradict each other).
-// Descends a five-level min hierarchy, 32 entries per ballot: groups of 32
-// ranges (group_min) -> ranges (range_state) -> tiles of a range
-// (tile_min) -> 32-key chunks of a tile (chunk_min) -> keys, so an answer
-// any distance away costs a handful of dependent L2 reads.  Every range
-// before the one holding limit-1, and every group before that range's group,
-// must have published; so must the tiles and chunks below limit-1.  Reads of
-// the published arrays go to L2 (ld.cg); the keys are read-only.
-// ---------------------------------------------------------------------------
-// Rightmost index i in [lo, hi] (hi - lo < 32) whose minimum qualifies, or -1.
-template <typename T, bool INCL, typename Load>
-__device__ __forceinline__ int ballot_last(int lo, int hi, T q, Load load) {
-    const int lane = threadIdx.x & 31;
-    const int i = hi - lane;
-    const bool ok = i >= lo && lt<INCL>(load(i), q);
-    const unsigned m = __ballot_sync(0xffffffffu, ok);
-    return m ? hi - (__ffs(m) - 1) : -1;
 }
 
 // Exclusive prefix sum over the warp's lanes of a count c, and the total.
@@ -179,74 +179,238 @@ __device__ __forceinline__ T key_at(const T* d_in, int n, int pos) {
     return load_key<T, KMAP>(d_in + (REV ? n - 1 - pos : pos));
 }
 
-template <typename T, int B, bool INCL, int MAPF = KMAP_NONE, bool REV = false>
-__device__ __noinline__ int find_left(T q, int limit, const T* __restrict__ d_in, const T* __restrict__ tile_min,
-                                      const T* __restrict__ chunk_min, const RangeArgs& a) {
-    constexpr int W = B / 32;
-    static_assert(W <= 32, "a tile's chunks must fit one ballot");
-    const int lane = threadIdx.x & 31;
-    if (limit <= 0) return -1;
-    const int last = limit - 1;
-    const int t = last / B;
-    const int c = (last - t * B) >> 5;
-    {  // 1. the row holding limit-1, positions below limit
-        const int row = t * B + c * 32;
-        const int p = row + lane;
-        const bool ok = p < limit && p >= a.head && lt<INCL>(key_at<T, MAPF, REV>(d_in, a.n, p), q);
-        const unsigned m = __ballot_sync(0xffffffffu, ok);
-        if (m) return row + 31 - __clz(m);
-    }
-    auto tmin = [&](int i) { return __ldcg(&tile_min[i]); };
-    const int tpr = a.tiles_per_range;
-    int s = -1;  // tile holding the answer
-    int cc = ballot_last<T, INCL>(0, c - 1, q, [&](int i) { return __ldcg(&chunk_min[(size_t)t * W + i]); });
-    if (cc >= 0) {
-        s = t;
-    } else {
-        const int R = t / tpr;
-        // 3. earlier tiles of the same range
-        for (int hi = t - 1; hi >= R * tpr && s < 0; hi -= 32) s = ballot_last<T, INCL>(R * tpr, hi, q, tmin);
-        if (s < 0) {
-            // 4. earlier ranges of the same group, then 5. earlier groups
-            auto rmin = [&](int i) { return range_min<T>(a, i); };
-            const int g = R >> 5;
-            int rr = ballot_last<T, INCL>(g * 32, R - 1, q, rmin);
-            if (rr < 0) {
-                int gg = -1;
-                for (int hi = g - 1; hi >= 0 && gg < 0; hi -= 32)
-                    gg = ballot_last<T, INCL>(0, hi, q, [&](int i) { return group_min_of<T>(a, i); });
-                if (gg < 0) return -1;
-                rr = ballot_last<T, INCL>(gg * 32, min(gg * 32 + 31, a.num_ranges - 1), q, rmin);
-                if (rr < 0) return -2;
-            }
-            const int rt1 = min((rr + 1) * tpr, a.num_tiles) - 1;
-            for (int hi = rt1; hi >= rr * tpr && s < 0; hi -= 32) s = ballot_last<T, INCL>(rr * tpr, hi, q, tmin);
-            if (s < 0) return -2;
-        }
-        cc = ballot_last<T, INCL>(0, W - 1, q, [&](int i) { return __ldcg(&chunk_min[(size_t)s * W + i]); });
-        if (cc < 0) return -2;
-    }
-    const int row = s * B + cc * 32;
-    const unsigned m =
-        __ballot_sync(0xffffffffu, row + lane >= a.head && lt<INCL>(key_at<T, MAPF, REV>(d_in, a.n, row + lane), q));
-    return m ? row + 31 - __clz(m) : -2;
+// Phase 2's searches take up to kFew queries one by one, the warp's lanes side by
+// side on 32 entries of a level (one load and a ballot a step), and more of them
+// one per lane (a round of independent loads a step for all): a lone query is
+// three times slower the second way, 32 of them ten times slower the first.
+constexpr int kFew = 4;
+
+// The last of the entries lo..hi (hi - lo < 32) that qualifies, or -1; uniform call.
+template <typename T, bool INCL, typename Load>
+__device__ __forceinline__ int last_of(int lo, int hi, T q, Load load) {
+    const int i = hi - (int)(threadIdx.x & 31);
+    const unsigned m = __ballot_sync(0xffffffffu, i >= lo && lt<INCL>(load(max(i, lo)), q));
+    return m ? hi - (__ffs(m) - 1) : -1;
 }
 
-// The nearest range at or below `hi` whose minimum qualifies for q, or -1:
-// the ranges of hi's group, then the minima of earlier groups, 32 per step.
-// Warp-cooperative; every range and group it reads has published.
-template <typename T, bool INCL>
-__device__ __noinline__ int nearest_range(T q, int hi, const RangeArgs& a) {
-    if (hi < 0) return -1;
-    auto rmin = [&](int i) { return range_min<T>(a, i); };
-    const int g = hi >> 5;
-    const int rr = ballot_last<T, INCL>(g * 32, hi, q, rmin);
-    if (rr >= 0) return rr;
-    for (int ghi = g - 1; ghi >= 0; ghi -= 32) {
-        const int gg = ballot_last<T, INCL>(0, ghi, q, [&](int i) { return group_min_of<T>(a, i); });
-        if (gg >= 0) return ballot_last<T, INCL>(gg * 32, gg * 32 + 31, q, rmin);
+// Search inside one range: each lane with `need` finds the rightmost key that
+// qualifies for its q in its tiles [lo, hi) -- the nearest tile by tile minima,
+// its chunk, its key.  -2 when no tile's minimum qualifies.
+template <typename T, int B, bool INCL, int MAPF = KMAP_NONE, bool REV = false>
+__device__ __noinline__ int find_in_tiles(T q, bool need, int lo, int hi, const T* __restrict__ d_in,
+                                          const RangeArgs& a) {
+    constexpr int W = B / 32;
+    const T* tile_min = (const T*)a.s.tile_min;
+    const T* chunk_min = (const T*)a.s.chunk_min;
+    unsigned nm = __ballot_sync(0xffffffffu, need);
+    if (__popc(nm) <= kFew) {
+        int p = -2;
+        for (; nm; nm &= nm - 1) {
+            const int f = __ffs(nm) - 1;
+            const T qf = __shfl_sync(0xffffffffu, q, f);
+            const int lf = __shfl_sync(0xffffffffu, lo, f), hf = __shfl_sync(0xffffffffu, hi, f);
+            int s = -1;
+            for (int h = hf - 1; h >= lf && s < 0; h -= 32)
+                s = last_of<T, INCL>(max(lf, h - 31), h, qf, [&](int i) { return __ldcg(&tile_min[i]); });
+            if (s < 0) continue;
+            const int c = max(last_of<T, INCL>(0, W - 1, qf, [&](int i) { return __ldcg(&chunk_min[(size_t)s * W + i]); }), 0);
+            const int row = s * B + c * 32;
+            const int k = last_of<T, INCL>(max(row, a.head), row + 31, qf,
+                                           [&](int i) { return key_at<T, MAPF, REV>(d_in, a.n, min(i, a.n - 1)); });
+            if ((int)(threadIdx.x & 31) == f && k >= 0 && k < a.n) p = k;
+        }
+        return p;
     }
-    return -1;
+    int s = -1;
+    for (int t = hi - 1; need && s < 0 && t >= lo; t -= 16) {
+        T m[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) m[k] = __ldcg(&tile_min[max(t - k, lo)]);
+#pragma unroll
+        for (int k = 0; k < 16; k++)
+            if (s < 0 && t - k >= lo && lt<INCL>(m[k], q)) s = t - k;
+    }
+    int p = -2;
+    if (need && s >= 0) {
+        int c = 0;
+#pragma unroll
+        for (int k = 0; k < W; k++)
+            if (lt<INCL>(__ldcg(&chunk_min[(size_t)s * W + k]), q)) c = k;
+        const int row = s * B + c * 32;
+#pragma unroll 1
+        for (int h = 16; h >= 0 && p < 0; h -= 16) {
+            T m[16];
+#pragma unroll
+            for (int k = 0; k < 16; k++) m[k] = key_at<T, MAPF, REV>(d_in, a.n, min(max(row + h + k, a.head), a.n - 1));
+#pragma unroll
+            for (int k = 0; k < 16; k++)
+                if (row + h + k >= a.head && row + h + k < a.n && lt<INCL>(m[k], q)) p = row + h + k;
+        }
+    }
+    __syncwarp();
+    return p;
+}
+
+// Phase 2: each lane with `want` finds the answer of its q before range r (the
+// prefix minimum of the earlier ranges qualifies for it): the
+// nearest range whose minimum qualifies -- by the window of 32 range minima
+// (lane i: range r-1-i; wpm: their running minimum), else by the running minima
+// of the earlier groups (sg, staged in shared memory at the first need) and
+// that group's 32 range minima -- then the topmost qualifying entry of that
+// range's published stack, else its tiles.  -2: the published minima contradict
+// each other.
+template <typename T, int B, bool INCL, int MAPF = KMAP_NONE, bool REV = false>
+__device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, bool& staged,
+                                          const T* __restrict__ d_in, const RangeArgs& a) {
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr int KB = (int)sizeof(T);
+    const int lane = threadIdx.x & 31;
+    int rp = -1;
+    const unsigned wm = __ballot_sync(FULL, want);
+    if (__popc(wm) <= kFew) {
+        int ans = -2;
+        bool miss = false;
+        for (unsigned m = wm; m; m &= m - 1) {
+            const int f = __ffs(m) - 1;
+            const T qf = __shfl_sync(FULL, q, f);
+            const unsigned w = __ballot_sync(FULL, lt<INCL>(wpm, qf));
+            int rf = w ? r - __ffs(w) : -1;
+            if constexpr (KB == 8) {  // no group words: the range minima, 8 groups a step
+                for (int hi = r - 33; hi >= 0 && rf < 0; hi -= 256) {
+                    T u[8];
+#pragma unroll
+                    for (int k = 0; k < 8; k++) u[k] = range_min<T>(a, max(hi - 32 * k - lane, 0));
+#pragma unroll
+                    for (int k = 0; k < 8; k++) {
+                        const unsigned b = __ballot_sync(FULL, hi - 32 * k - lane >= 0 && lt<INCL>(u[k], qf));
+                        if (b && rf < 0) rf = hi - 32 * k - (__ffs(b) - 1);
+                    }
+                }
+            } else {
+                int g = rf >= 0 || r < 33 ? -1 : (r - 33) >> 5, gf = -1;
+                for (; g >= 0 && gf < 0; g -= 32)
+                    gf = last_of<T, INCL>(max(g - 31, 0), g, qf, [&](int i) { return group_min_of<T>(a, i); });
+                if (gf >= 0) rf = last_of<T, INCL>(32 * gf, 32 * gf + 31, qf, [&](int i) { return range_min<T>(a, i); });
+            }
+            int af = -2;
+            if (rf >= 0) {  // the range's published stack top
+                const int cnt = (int)(__ldcg(&a.s.top_cnt[rf]) & 0xffu);
+                const T tk = __ldcg((const T*)a.s.top_key + (size_t)rf * kTopEntries + lane);
+                const int tp = __ldcg(&a.s.top_pos[(size_t)rf * kTopEntries + lane]);
+                const unsigned b = __ballot_sync(FULL, lane < cnt && lt<INCL>(tk, qf));
+                if (b) af = __shfl_sync(FULL, tp, 31 - __clz(b));
+            }
+            if (lane == f) {
+                ans = af;
+                rp = rf;
+                miss = rf >= 0 && af == -2;
+            }
+        }
+        if (__any_sync(FULL, miss)) {
+            const int lo = max(rp, 0) * a.tiles_per_range;
+            const int found =
+                find_in_tiles<T, B, INCL, MAPF, REV>(q, miss, lo, min(lo + a.tiles_per_range, a.num_tiles), d_in, a);
+            if (miss) ans = found;
+        }
+        return ans;
+    }
+    {
+        int lo = -1;  // the nearest lo + 1 ranges do not qualify
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1)
+            if (!lt<INCL>(__shfl_sync(FULL, wpm, lo + s), q)) lo += s;
+        if (lt<INCL>(__shfl_sync(FULL, wpm, lo + 1), q)) rp = max(r - 2 - lo, -1);
+    }
+    if (__any_sync(FULL, want && rp < 0)) {
+        const int ng = r >= 33 ? ((r - 33) >> 5) + 1 : 0;  // groups of earlier ranges (the window's part does not qualify)
+        static_assert(kMaxRanges / 32 == 128, "four groups per lane");
+        if (!staged) {
+            T m[4];
+#pragma unroll
+            for (int j = 0; j < 4; j++) m[j] = 4 * lane + j < ng ? group_min_of<T>(a, 4 * lane + j) : KeyTraits<T>::pad();
+#pragma unroll
+            for (int j = 2; j >= 0; j--) m[j] = KeyTraits<T>::vmin(m[j], m[j + 1]);
+            T x = m[0];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const T y = __shfl_down_sync(FULL, x, o);
+                if (lane + o < 32) x = KeyTraits<T>::vmin(x, y);
+            }
+            const T after = __shfl_down_sync(FULL, x, 1);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 4; j++) sg[4 * lane + j] = lane < 31 ? KeyTraits<T>::vmin(m[j], after) : m[j];
+            __syncwarp();
+            staged = true;
+        }
+        if (want && rp < 0 && ng > 0) {
+            int g = 0;
+#pragma unroll
+            for (int s = 64; s > 0; s >>= 1)
+                if (g + s < ng && lt<INCL>(sg[g + s], q)) g += s;
+#pragma unroll 1
+            for (int h = 16; h >= 0 && rp < 0; h -= 16) {
+                T m[16];
+#pragma unroll
+                for (int k = 0; k < 16; k++) {
+                    const int i = 32 * g + h + k;
+                    if constexpr (KB == 8) m[k] = range_min<T>(a, i);
+                    else m[k] = KeyTraits<T>::from_bits(__ldcg((const uint32_t*)&a.s.range_state[i]));
+                }
+#pragma unroll
+                for (int k = 0; k < 16; k++)
+                    if (lt<INCL>(m[k], q)) rp = 32 * g + h + k;
+            }
+        }
+    }
+    int ans = -2;
+    if (want && rp >= 0) {
+        // rp's published stack top, keys and positions in one round of loads:
+        // entries increase from the bottom, so the qualifying ones form a
+        // bottom part and the topmost of them answers
+        const int cnt = (int)(__ldcg(&a.s.top_cnt[rp]) & 0xffu);
+        const uint4* tk = reinterpret_cast<const uint4*>((const T*)a.s.top_key + (size_t)rp * kTopEntries);
+        const uint4* tp = reinterpret_cast<const uint4*>(a.s.top_pos + (size_t)rp * kTopEntries);
+        if constexpr (KB == 4) {
+            uint4 tw[kTopEntries / 4], pw[kTopEntries / 4];
+#pragma unroll
+            for (int k = 0; k < kTopEntries / 4; k++) {
+                tw[k] = __ldcg(&tk[k]);
+                pw[k] = __ldcg(&tp[k]);
+            }
+#pragma unroll
+            for (int k = 0; k < kTopEntries / 4; k++) {
+                const uint32_t wb[4] = {tw[k].x, tw[k].y, tw[k].z, tw[k].w};
+                const int pb[4] = {(int)pw[k].x, (int)pw[k].y, (int)pw[k].z, (int)pw[k].w};
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    if (4 * k + c < cnt && lt<INCL>(KeyTraits<T>::from_bits(wb[c]), q)) ans = pb[c];
+            }
+        } else {  // two 8-byte keys per 16-byte load
+            uint4 tw[kTopEntries / 2], pw[kTopEntries / 4];
+#pragma unroll
+            for (int k = 0; k < kTopEntries / 2; k++) tw[k] = __ldcg(&tk[k]);
+#pragma unroll
+            for (int k = 0; k < kTopEntries / 4; k++) pw[k] = __ldcg(&tp[k]);
+#pragma unroll
+            for (int k = 0; k < kTopEntries / 2; k++) {
+                const uint64_t kb2[2] = {((uint64_t)tw[k].y << 32) | tw[k].x, ((uint64_t)tw[k].w << 32) | tw[k].z};
+                const uint4 p4 = pw[k / 2];
+                const int pb2[2] = {(int)(k % 2 ? p4.z : p4.x), (int)(k % 2 ? p4.w : p4.y)};
+#pragma unroll
+                for (int c = 0; c < 2; c++)
+                    if (2 * k + c < cnt && lt<INCL>(KeyTraits<T>::from_bits(kb2[c]), q)) ans = pb2[c];
+            }
+        }
+    }
+    const bool miss = want && rp >= 0 && ans == -2;
+    if (__any_sync(FULL, miss)) {
+        const int lo = max(rp, 0) * a.tiles_per_range;
+        const int found =
+            find_in_tiles<T, B, INCL, MAPF, REV>(q, miss, lo, min(lo + a.tiles_per_range, a.num_tiles), d_in, a);
+        if (miss) ans = found;
+    }
+    return ans;
 }
 
 // ---------------------------------------------------------------------------
@@ -421,12 +585,14 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     constexpr int RPT = W * KB / 4;  // key TMA rows (128 bytes) per warp tile
     static_assert(KB == 4 || (KB == 8 && IPT == 8), "8-byte keys run with 8 keys per lane");
     constexpr int TPC = 32 / IPT;  // lanes per chunk
-    constexpr int K = kStackCap;
+    constexpr int K = kStackCapOf<KB>;
+    constexpr int kStages = kStagesOf<KB>;
+    constexpr int kDefCap = kDefCapOf<KB>;
     constexpr int MW = kMaxTileKeys / 32;  // flag-mask words per tile in global
     static_assert(IPT == 8 || IPT == 16, "IPT must be 8 or 16");
     auto ks = [](int e) { return kswz<KB>(e); };  // swizzled index of key e in V / sSM
     static_assert((K & (K - 1)) == 0, "the stack ring needs a power-of-two size");
-    static_assert(K % 32 == 0 && K <= WT, "a whole-tile push copies the tile's last K keys, 32 per step");
+    static_assert(K % 32 == 0 && kUpKeep <= K && kUpKeep <= WT, "a whole-tile push copies the tile's last keys, 32 per step");
     constexpr unsigned FULL = 0xffffffffu;
 
     extern __shared__ unsigned char smem_raw[];
@@ -446,7 +612,10 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     T* sDefV = (T*)(wsm + L::kDefV);
     int32_t* sCapP = (int32_t*)(wsm + L::kCapP);
     int32_t* sCapS = (int32_t*)(wsm + L::kCapS);
+    T* sPad = (T*)(wsm + L::kPad);
     uint64_t* bar = (uint64_t*)(wsm + L::kBar);
+    // 0, as a value the compiler does not know (grids are one-dimensional): see take_if_lt
+    const int zero = (int)gridDim.y - 1;
 
     const T* d_in = (const T*)a.d_in;
     T* tile_min_w = (T*)a.s.tile_min;
@@ -473,6 +642,27 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         else if constexpr (OUTM == OUT_SPAN) a.d_out[pos] = pos - v;
         else a.d_out[pos] = v;
     };
+    // the same for the four positions from pos on (a multiple of 4, in a tile that
+    // streams through TMA: 16-byte aligned), v >= 0
+    auto put4 = [&](int pos, int v) {
+        if constexpr (OUT64) {
+            const long long w = (long long)v + a.out_base;
+            longlong2* o = reinterpret_cast<longlong2*>(a.d_out64 + pos);
+            if (((uintptr_t)o & 15) == 0) {
+                o[0] = make_longlong2(w, w);
+                o[1] = make_longlong2(w, w);
+            } else {
+                for (int k = 0; k < 4; k++) a.d_out64[pos + k] = w;
+            }
+        } else if constexpr (REV) {
+            const int w = a.n - 1 - v;
+            *reinterpret_cast<int4*>(a.d_out + (a.n - 4 - pos)) = make_int4(w, w, w, w);
+        } else if constexpr (OUTM == OUT_SPAN) {
+            *reinterpret_cast<int4*>(a.d_out + pos) = make_int4(pos - v, pos + 1 - v, pos + 2 - v, pos + 3 - v);
+        } else {
+            *reinterpret_cast<int4*>(a.d_out + pos) = make_int4(v, v, v, v);
+        }
+    };
 
     // One claim per CTA: its warps take WPC consecutive range ids, in the order
     // the CTAs start (so every range a warp may wait on belongs to a started CTA).
@@ -484,6 +674,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     if (lane == 0) {
         epoch = ld_relaxed_u32(&a.s.ctr->epoch);
         for (int s = 0; s < kStages; s++) mbar_init(&bar[s], 1);
+        for (int k = 0; k < 4; k++) sPad[k] = KeyTraits<T>::pad();
         fence_mbarrier_init();
         fence_proxy_async_smem();
     }
@@ -617,7 +808,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 return bb ? tile_base + lane * IPT + 31 - __clz(bb) : lane_s;
             };
 
-            // ---- 1. in-thread answers: compare ladder over IPT keys in registers --------
+            // ---- 1. the lane's keys in registers ---------------------------------------
             T v[IPT];
             if constexpr (KB == 4) {
 #pragma unroll
@@ -774,12 +965,34 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 }
             };
 
+            // The four keys before the lane's first (lane 0: pads).
+            T h[4];
+            {
+                const T* hp = lane > 0 ? &V[ks(lane * IPT - 4)] : sPad;
+                if constexpr (KB == 4) {
+                    const uint4 rr = *reinterpret_cast<const uint4*>(hp);
+                    h[0] = KeyTraits<T>::from_bits(rr.x);
+                    h[1] = KeyTraits<T>::from_bits(rr.y);
+                    h[2] = KeyTraits<T>::from_bits(rr.z);
+                    h[3] = KeyTraits<T>::from_bits(rr.w);
+                } else {
+                    const T* hq = lane > 0 ? &V[ks(lane * IPT - 2)] : sPad + 2;
+                    const ulonglong2 r0 = *reinterpret_cast<const ulonglong2*>(hp);
+                    const ulonglong2 r1 = *reinterpret_cast<const ulonglong2*>(hq);
+                    h[0] = KeyTraits<T>::from_bits((uint64_t)r0.x);
+                    h[1] = KeyTraits<T>::from_bits((uint64_t)r0.y);
+                    h[2] = KeyTraits<T>::from_bits((uint64_t)r1.x);
+                    h[3] = KeyTraits<T>::from_bits((uint64_t)r1.y);
+                }
+            }
+            const T prev_last = h[3];
+
             // Monotone lanes: each key answers its neighbour (adj), or no key answers
             // any later one (none); across the lane boundary likewise (b_adj, b_none).
             // A few neighbour pairs first: on almost every tile of unordered keys some
             // lane is already neither increasing nor non-increasing there, and the
-            // full check (15 compares a lane) is skipped.
-            bool adj = false, none = false;
+            // full check (15 compares a lane) and the whole-tile paths are skipped.
+            bool adj = false, none = false, b_adj = false;
             unsigned mono = 0u;
             {
                 bool qa = true, qn = true;
@@ -799,10 +1012,9 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         none = none && !l;
                     }
                     mono = __ballot_sync(FULL, adj || none);
+                    b_adj = lane == 0 || lt<INCL>(prev_last, v[0]);
                 }
             }
-            const T prev_last = __shfl_up_sync(FULL, v[IPT - 1], 1);
-            const bool b_adj = lane == 0 || lt<INCL>(prev_last, v[0]);
 
             // ---- a whole tile below the range so far --------------------------------------
             // A tile that never increases (under the comparator, lane boundaries
@@ -811,10 +1023,74 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             // every stack entry (>= the range minimum >= the first key) is popped and
             // the tile's last key is its only strict suffix minimum.  (Single arrays,
             // also a single array behind a view head in the segmented kernel.)
-            if constexpr (EP) {
+            if (EP && mono == FULL && valid_keys == WT) {
                 const T first = __shfl_sync(FULL, v[0], 0);
-                if (mono == FULL && valid_keys == WT && __all_sync(FULL, none && (lane == 0 || !b_adj)) &&
-                    (!has_rmin || !lt<INCL>(rmin, first))) {
+                const bool never = __all_sync(FULL, none && (lane == 0 || !b_adj));
+                // No key of the tile answers another.  When the same entry of the stack's
+                // top 32 is the topmost one to qualify for the tile's first and for its
+                // last key, it answers every key between too (descending keys after a lower
+                // one: 671 low keys in 2^25 descending ones sent a quarter of the ranges
+                // through 16 rounds of stack queries a tile, 254 us against 51).
+                unsigned same = 0u;  // the window entries that qualify for every key
+                const int wlo = max(stk_lo, stk_hi - 32);
+                T wtop = KeyTraits<T>::pad();
+                if (never && has_rmin) {
+                    const bool in = wlo + lane < stk_hi;
+                    const T last = __shfl_sync(FULL, v[IPT - 1], 31);
+                    wtop = in ? sStkV[(wlo + lane) & (K - 1)] : KeyTraits<T>::pad();
+                    same = __ballot_sync(FULL, in && lt<INCL>(wtop, last));
+                    if (same != __ballot_sync(FULL, in && lt<INCL>(wtop, first))) same = 0u;
+                }
+                if (same) {
+                    const T tmin = __shfl_sync(FULL, v[IPT - 1], 31);
+                    const int top = 31 - __clz(same);
+                    const int tp = max(sStkP[(wlo + top) & (K - 1)] - (OUTM == OUT_I32 ? head : 0), -1);
+#pragma unroll
+                    for (int q4 = 0; q4 < IPT / 4; q4++)
+                        *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) = make_int4(tp, tp, tp, tp);
+                    if (((lane + 1) & (TPC - 1)) == 0) __stcg(&chunk_min_w[(size_t)t * W + lane / TPC], v[IPT - 1]);
+                    if (lane == 0) {
+                        __stcg(&a.s.tile_flag[t], 0u);
+                        __stcg(&tile_min_w[t], tmin);
+                    }
+                    if constexpr (OUTM != OUT_I32 || REV) {
+                        store_tile();
+                    } else {
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (full) {
+                            if (lane == 0) {
+                                tma_store_2d(&map_out, 0, t * W, O);
+                                bulk_commit();
+                            }
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < IPT; j++)
+                                if (!head || tile_base + j * 32 + lane >= head) a.d_out[tile_base + j * 32 + lane] = tp;
+                        }
+                    }
+                    __syncwarp();  // every lane has read the stack
+                    // the entries below the tile's minimum stay (the top one may equal it
+                    // under <=) and the tile's last key is pushed
+                    const int kp = wlo + top + (__shfl_sync(FULL, wtop, top) < tmin ? 1 : 0);
+                    if (lane == 31) {
+                        sStkV[kp & (K - 1)] = v[IPT - 1];
+                        sStkP[kp & (K - 1)] = tile_base + WT - 1;
+                    }
+                    stk_hi = kp + 1;
+                    if (stk_hi - K > stk_lo) {
+                        stk_lo = stk_hi - K;
+                        dropped = true;
+                    }
+                    rmin = KeyTraits<T>::vmin(rmin, tmin);
+                    __syncwarp();
+                    if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
+                        mbar_arrive_expect_tx(&bar[slot], (uint32_t)(WT * KB));
+                        tma_load_2d(V, &map_in, 0, tile_row(t + kStages), &bar[slot]);
+                    }
+                    continue;
+                }
+                if (never && (!has_rmin || !lt<INCL>(rmin, first))) {
                     const int4 m1 = make_int4(-1, -1, -1, -1);
 #pragma unroll
                     for (int q4 = 0; q4 < IPT / 4; q4++) *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) = m1;
@@ -866,11 +1142,10 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             // A strictly increasing tile whose first key is above the stack's top entry
             // (the range's last key): every key answers its predecessor under either
             // comparator, every key is a strict suffix minimum, and the ring keeps the
-            // tile's last K keys.
-            if constexpr (EP) {
+            // tile's last kUpKeep keys.
+            if (EP && mono == FULL && valid_keys == WT) {
                 const T first = __shfl_sync(FULL, v[0], 0);
-                bool up = mono == FULL && valid_keys == WT && __all_sync(FULL, adj && b_adj) && stk_hi > stk_lo &&
-                          sStkV[(stk_hi - 1) & (K - 1)] < first;
+                bool up = __all_sync(FULL, adj && b_adj) && stk_hi > stk_lo && sStkV[(stk_hi - 1) & (K - 1)] < first;
                 if constexpr (INCL) {
                     // adj means non-decreasing here: ties would not all be strict suffix
                     // minima, so check strict increase (only on such tiles)
@@ -915,14 +1190,14 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     }
                     const int base_idx = stk_hi;  // entry of tile key e: base_idx + e
 #pragma unroll
-                    for (int h = 0; h < K / 32; h++) {  // the tile's last K keys, one per lane and step
-                        const int e = WT - K + h * 32 + lane;
+                    for (int h = 0; h < kUpKeep / 32; h++) {  // the tile's last keys, one per lane and step
+                        const int e = WT - kUpKeep + h * 32 + lane;
                         sStkV[(base_idx + e) & (K - 1)] = V[ks(e)];
                         sStkP[(base_idx + e) & (K - 1)] = tile_base + e;
                     }
                     stk_hi = base_idx + WT;
-                    stk_lo = stk_hi - K;
-                    dropped = true;  // WT > K: the older entries are gone
+                    stk_lo = stk_hi - kUpKeep;
+                    dropped = true;  // the older entries are gone
                     rmin = KeyTraits<T>::vmin(rmin, first);
                     __syncwarp();
                     if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
@@ -933,12 +1208,11 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 }
             }
 
-            // Filled by the path below that handles the tile (steps 1-5, or a tile that never
-            // increases) and used by steps 6-9.
-            unsigned dm = 0u, cm = 0u;
-            T lmin = KeyTraits<T>::pad(), suf = KeyTraits<T>::pad(), tile_min_t = KeyTraits<T>::pad();
-            T wv = KeyTraits<T>::pad();
-            int win_lo = 0, dkeep = 0;
+            // Filled by the path below that handles the tile (steps 2-6, or a tile that never
+            // increases) and used by steps 7-9.
+            T tile_min_t = KeyTraits<T>::pad(), wv = KeyTraits<T>::pad();
+            int win_lo = 0, dkeep = 0, ppre = 0, ptot = 0, fcnt = 0;
+            unsigned fmask = 0;  // the lane's keys below every later key of the tile
             bool wvalid = false;
             // ---- a whole tile that never increases, above something earlier in the range -----
             // No key answers another, so every key's answer is the topmost qualifying entry
@@ -952,6 +1226,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             const bool dtile =
                 SEG && mono == FULL && valid_keys == WT && __all_sync(FULL, none && (lane == 0 || !b_adj));
             if (dtile) {
+                unsigned dm = 0u, cm = 0u;
                 const int dwin = max(stk_lo, stk_hi - 32);
                 const int wcnt = stk_hi - dwin;
                 const T dwv = dwin + lane < stk_hi ? sStkV[(dwin + lane) & (K - 1)] : KeyTraits<T>::pad();
@@ -1003,43 +1278,51 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 int kp = __shfl_sync(FULL, si, 31);
                 while (kp >= stk_lo && !(sStkV[kp & (K - 1)] < tile_min_t)) kp--;
                 dkeep = kp + 1;
+                flag_keys(dm, cm);
             } else {
-            unsigned umask = 0;     // keys without an in-thread answer
-            bool all_inc = false;   // the whole tile increases: every key answers its predecessor
+            // ---- 2. in-thread answers: compare ladder ---------------------------------------
+            // Key k of a lane against the lane's earlier keys, and its first keys also
+            // against the 4 - k nearest ones before the lane, so that every key has seen
+            // at least its four predecessors (10 compares a lane more; of 16 random keys
+            // 2.1 instead of 3.4 are left for the cross-lane queries).  The compares are
+            // what the ALU pipe does here; the selects go to the multiply-add pipe.
+            unsigned umask = 0;  // keys without an in-thread answer: bit IPT - 1 - k for key k
             {
                 int res[IPT];  // absolute answers, -1 = none in the thread
-                res[0] = -1;
-                // Monotone lanes need no ladder.
-                if (mono == FULL) {
+                if (mono == FULL) {  // monotone lanes need no ladder
+                    res[0] = lane > 0 && b_adj ? lb - 1 : -1;
 #pragma unroll
                     for (int k = 1; k < IPT; k++) res[k] = adj ? lb + k - 1 : -1;
-                    // every key answers its predecessor across lane boundaries too
-                    all_inc = __all_sync(FULL, adj && b_adj) && valid_keys == WT;
-                    if (all_inc && lane > 0) res[0] = lb - 1;
                 } else {
 #pragma unroll
-                    for (int k = 1; k < IPT; k++) {
-                        int rk = -1;
+                    for (int k = 0; k < IPT; k++) {
+                        int rk = -1 - lb;  // relative to lb
 #pragma unroll
-                        for (int j = 0; j < k; j++)
-                            if (lt<INCL>(v[j], v[k])) rk = lb + j;
-                        res[k] = rk;
+                        for (int j = k; j < 4; j++) take_if_lt<INCL>(rk, h[j], v[k], zero, j - 4);
+#pragma unroll
+                        for (int j = 0; j < k; j++) take_if_lt<INCL>(rk, v[j], v[k], zero, j);
+                        res[k] = rk + lb;
                     }
-                    // the first key answers the previous lane's last key when that qualifies
-                    if (lane > 0 && b_adj) res[0] = lb - 1;
+                    if constexpr (INCL) {  // lane 0's pads qualify for keys of the pad's value
+                        if (lane == 0)
+#pragma unroll
+                            for (int k = 0; k < 4; k++)
+                                if (res[k] < lb) res[k] = -1;
+                    }
                 }
 #pragma unroll
-                for (int k = 0; k < IPT; k++)
-                    if (res[k] < 0) umask |= 1u << k;
-                if (nvalid < IPT) umask &= (1u << nvalid) - 1u;  // (the tail tile's pads)
+                for (int k = 0; k < IPT; k++) umask = __funnelshift_l((unsigned)res[k], umask, 1);
+                if (nvalid < IPT) umask &= ~((1u << (IPT - nvalid)) - 1u);  // (the tail tile's pads)
                 // in-thread answers; every other key holds -1 until resolved below
 #pragma unroll
                 for (int q4 = 0; q4 < IPT / 4; q4++)
                     *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) =
                         make_int4(res[4 * q4], res[4 * q4 + 1], res[4 * q4 + 2], res[4 * q4 + 3]);
             }
-            {  // suffix minima of the lane's keys (for the key search of X keys)
-                T sfx[IPT];
+            // ---- 3. lane suffix minima, minima over lanes, the tile's strict suffix minima --
+            T lmin, tab[5];
+            {
+                T sfx[IPT];  // suffix minima of the lane's keys (for the key search of X keys)
                 sfx[IPT - 1] = v[IPT - 1];
 #pragma unroll
                 for (int k = IPT - 2; k >= 0; k--) sfx[k] = KeyTraits<T>::vmin(v[k], sfx[k + 1]);
@@ -1057,181 +1340,167 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                             make_ulonglong2((unsigned long long)KeyTraits<T>::bits(sfx[2 * q2]),
                                             (unsigned long long)KeyTraits<T>::bits(sfx[2 * q2 + 1]));
                 }
-            }
-            {
-                T cmn = lmin;
+                {
+                    T cmn = lmin;
 #pragma unroll
-                for (int o = 1; o < TPC; o <<= 1) cmn = KeyTraits<T>::vmin(cmn, __shfl_xor_sync(FULL, cmn, o));
-                if ((lane & (TPC - 1)) == 0) __stcg(&chunk_min_w[(size_t)t * W + lane / TPC], cmn);
-            }
-
-            // ---- 2. warp prefix minima over lane minima ---------------------------------
-            T pre = lmin;  // inclusive prefix / suffix minima over lanes, side by side
-            suf = lmin;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const T nb = __shfl_up_sync(FULL, pre, o);
-                const T na = __shfl_down_sync(FULL, suf, o);
-                if (lane >= o) pre = KeyTraits<T>::vmin(pre, nb);
-                if (lane + o < 32) suf = KeyTraits<T>::vmin(suf, na);
-            }
-            const T before = __shfl_up_sync(FULL, pre, 1);  // min of the lanes before (lane > 0)
-            tile_min_t = __shfl_sync(FULL, pre, 31);
-
-            // ---- 3. classify the keys without an in-thread answer ------------------------
-            // X: answered by an earlier lane of the tile; S: by an earlier tile of the
-            // range (the stack); D: by nothing in the range (deferred to phase 2).
-            unsigned gtb = 0, gtr = ~0u;
-#pragma unroll
-            for (int k = 0; k < IPT; k++) gtb |= (unsigned)lt<INCL>(before, v[k]) << k;
-            // Every key of a lane is >= the lane minimum: when the range minimum
-            // qualifies for every lane's minimum (most tiles after a range's first),
-            // it qualifies for every key and the per-key compares are skipped.
-            if (!__all_sync(FULL, lt<INCL>(rmin, lmin))) {
-                gtr = 0u;
-#pragma unroll
-                for (int k = 0; k < IPT; k++) gtr |= (unsigned)lt<INCL>(rmin, v[k]) << k;
-            }
-            const unsigned xm = lane > 0 ? (umask & gtb) : 0u;
-            const unsigned sm = has_rmin ? (umask & ~xm & gtr) : 0u;
-            dm = umask & ~xm & ~sm;
-            if constexpr (SEG) {
-                // Nothing in the range qualifies for a deferred key; if its segment
-                // starts inside the range, -1 is its final answer.  Only keys of the
-                // segment holding the range's first key stay deferred.
-                if (lb + IPT > first_end) dm &= lb >= first_end ? 0u : ((1u << (first_end - lb)) - 1u);
-            }
-            __syncwarp();  // the in-thread answers and suffix minima are in shared memory
-
-            // ---- 4. X keys: lane by binary lifting, then key by binary search ------------
-            const int cx = __popc(xm);
-            const int xtot = (int)__reduce_add_sync(FULL, (unsigned)cx);
-            if (xtot) {
-                // lane table: tab[k] = min of lane minima over lanes (lane - 2^k, lane]
-                T tab[5];
-                tab[0] = lmin;
-#pragma unroll
-                for (int k = 1; k < 5; k++) {
-                    const T u = __shfl_up_sync(FULL, tab[k - 1], 1 << (k - 1));
-                    tab[k] = lane >= (1 << (k - 1)) ? KeyTraits<T>::vmin(tab[k - 1], u) : tab[k - 1];
+                    for (int o = 1; o < TPC; o <<= 1) cmn = KeyTraits<T>::vmin(cmn, __shfl_xor_sync(FULL, cmn, o));
+                    if ((lane & (TPC - 1)) == 0) __stcg(&chunk_min_w[(size_t)t * W + lane / TPC], cmn);
                 }
-                // Up to NQ queries per lane and round.  A key e of lane ql = e / IPT is an X key
-                // only when some lane before ql qualifies, so the lifting below never
-                // passes lane 0: it ends on the nearest qualifying lane p (invariant: the
-                // answer lane is <= p and after each step p - answer < 2^k).  In lane p,
-                // the suffix minima qualify on a prefix [0, j] and key j is the answer.
-                constexpr int NQ = kXQueries;
-                auto resolve = [&](const int (&e)[NQ], const bool (&act)[NQ]) {
+                // Side by side: suffix minima over lanes, and the lane table of the X
+                // queries.  Slot s of the table stands for lane s - 1 (slot 0: a pad),
+                // tab[k] = the minimum of slots (s - 2^k, s].
+                T suf = lmin;
+                tab[0] = __shfl_up_sync(FULL, lmin, 1);
+                if (lane == 0) tab[0] = KeyTraits<T>::pad();
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    const T na = __shfl_down_sync(FULL, suf, 1 << k);
+                    if (lane + (1 << k) < 32) suf = KeyTraits<T>::vmin(suf, na);
+                    if (k < 4) {
+                        const T u = __shfl_up_sync(FULL, tab[k], 1 << k);
+                        tab[k + 1] = lane >= (1 << k) ? KeyTraits<T>::vmin(tab[k], u) : tab[k];
+                    }
+                }
+                tile_min_t = __shfl_sync(FULL, suf, 0);
+                const T after_w = __shfl_down_sync(FULL, suf, 1);  // min of the lanes after (lane < 31)
+                if (lane == 31 || lt<false>(lmin, after_w)) {      // else no key here beats every later key
+#pragma unroll
+                    for (int k = 0; k < IPT; k++)
+                        if ((k == IPT - 1 || sfx[k] < sfx[k + 1]) && (lane == 31 || sfx[k] < after_w)) fmask |= 1u << k;
+                }
+            }
+            // one prefix sum for both lists: keys to query, keys to push
+            fcnt = __popc(fmask);
+            ppre = warp_excl_sum(__popc(umask) | (fcnt << 16), ptot);
+            const int qtot = ptot & 0xffff;
+            win_lo = max(stk_lo, stk_hi - 32);  // the stack's top 32 entries, one per lane
+            const int widx = win_lo + lane;
+            wvalid = widx < stk_hi;
+            wv = wvalid ? sStkV[widx & (K - 1)] : KeyTraits<T>::pad();
+            const int wp = wvalid ? sStkP[widx & (K - 1)] : -1;
+
+            // ---- 4. keys without an in-thread answer: an earlier lane of the tile (X) -------
+            // Spread evenly over the lanes, up to NQ queries per lane and round: the lane by
+            // binary lifting over the table, then the key by binary search of that lane's
+            // suffix minima.  A query that ends on slot 0 or below has no answer in the tile;
+            // those keys (in order) are left in the front of the list.
+            int ns = 0, xtot = qtot;
+            auto list_keys = [&](unsigned m, int off) {  // the keys of mask m, from list entry off on
+                const int last_e = lane * IPT + IPT - 1;
+                while (m) {
+                    const int b = 31 - __clz(m);
+                    m ^= 1u << b;
+                    sList[off++] = (int16_t)(last_e - b);
+                }
+            };
+            unsigned smask = 0u;  // keys known to have no answer in the tile
+            int xoff = ppre & 0xffff;
+            constexpr int NQ = kXQueries;
+            T before = tab[4];  // the minimum of the lanes before
+            {
+                const T u = __shfl_up_sync(FULL, before, 16);
+                if (lane >= 16) before = KeyTraits<T>::vmin(before, u);
+            }
+            // A lane's listed keys do not increase: when no earlier lane qualifies for its
+            // first, none does for any.  No such key at all (ramps): nothing to query.
+            const T q1 = V[ks(lane * IPT + (IPT - 1 - (31 - __clz(umask | 1u))))];
+            if (!__any_sync(FULL, umask && lane > 0 && lt<INCL>(before, q1))) {
+                smask = umask;
+                xtot = xoff = 0;
+            } else if (qtot > 32 * NQ) {
+                // More than a round of keys: those no earlier lane qualifies for (most of
+                // them, when keys fall) need no query.
+#pragma unroll
+                for (int k = 0; k < IPT; k++) smask = (smask << 1) | (lane > 0 && lt<INCL>(before, V[ks(lane * IPT + k)]) ? 0u : 1u);
+                smask &= umask;
+                xoff = warp_excl_sum(__popc(umask ^ smask), xtot);
+            }
+            list_keys(umask ^ smask, xoff);
+            __syncwarp();  // in-thread answers, suffix minima and the list are in shared memory
+            {
+                for (int b0 = 0; b0 < xtot; b0 += 32 * NQ) {
+                    int e[NQ], pl[NQ];
+                    bool act[NQ];
                     T q[NQ];
-                    int p[NQ];
 #pragma unroll
                     for (int i2 = 0; i2 < NQ; i2++) {
-                        q[i2] = act[i2] ? V[ks(e[i2])] : KeyTraits<T>::pad();
-                        p[i2] = act[i2] ? e[i2] / IPT - 1 : 0;
+                        act[i2] = b0 + 32 * i2 + lane < xtot;
+                        e[i2] = act[i2] ? (int)sList[b0 + 32 * i2 + lane] : 0;
                     }
+#pragma unroll
+                    for (int i2 = 0; i2 < NQ; i2++) {
+                        q[i2] = V[ks(e[i2])];
+                        pl[i2] = e[i2] / IPT;  // slot of the lane before the key's
+                    }
+                    // invariant: the answer's slot is <= pl and after each step pl - slot < 2^k;
+                    // with no answer pl ends at 0 or below (a negative slot wraps to some
+                    // lane's words: whatever they hold, pl stays negative)
 #pragma unroll
                     for (int k = 4; k >= 0; k--) {
 #pragma unroll
                         for (int i2 = 0; i2 < NQ; i2++) {
-                            const T m = __shfl_sync(FULL, tab[k], p[i2]);  // p stays in [0, 31]
-                            if (act[i2] && !lt<INCL>(m, q[i2])) p[i2] -= 1 << k;
+                            const T m = __shfl_sync(FULL, tab[k], pl[i2]);
+                            if (!lt<INCL>(m, q[i2])) pl[i2] -= 1 << k;
                         }
                     }
-                    int j[NQ];
-#pragma unroll
-                    for (int i2 = 0; i2 < NQ; i2++) j[i2] = 0;
-#pragma unroll
-                    for (int i2 = 0; i2 < NQ; i2++)
-                        if (act[i2] && p[i2] < 0) {  // cannot happen (see the invariant); stay in bounds
-                            atomicOr(err, ERR_INTERNAL);
-                            p[i2] = 0;
-                        }
-                    // lane p's entries share one swizzle: word (p*IPT | j) ^ x
-                    int pb[NQ], px[NQ];
+                    // In lane pl - 1 the suffix minima qualify on a prefix [0, j] and key j is
+                    // the answer; the lane's entries share one swizzle: word (lane*IPT | j) ^ x
+                    int j[NQ], pb[NQ], px[NQ];
 #pragma unroll
                     for (int i2 = 0; i2 < NQ; i2++) {
-                        pb[i2] = p[i2] * IPT;
+                        j[i2] = 0;
+                        pb[i2] = max(pl[i2] - 1, 0) * IPT;
                         px[i2] = (pb[i2] >> 3) & (KB == 4 ? 0x1C : 0x0E);
                     }
 #pragma unroll
                     for (int s2 = IPT / 2; s2 > 0; s2 >>= 1) {
 #pragma unroll
                         for (int i2 = 0; i2 < NQ; i2++)
-                            if (act[i2] && lt<INCL>(sSM[(pb[i2] | (j[i2] + s2)) ^ px[i2]], q[i2])) j[i2] += s2;
+                            if (lt<INCL>(sSM[(pb[i2] | (j[i2] + s2)) ^ px[i2]], q[i2])) j[i2] += s2;
                     }
 #pragma unroll
-                    for (int i2 = 0; i2 < NQ; i2++)
-                        if (act[i2]) O[swz(e[i2])] = tile_base + p[i2] * IPT + j[i2];
-                };
-                const int xmax = (int)__reduce_max_sync(FULL, (unsigned)cx);
-                const int rounds = (xtot + 32 * NQ - 1) / (32 * NQ);
-                if (xmax > NQ * rounds + 1) {
-                    // spread the queries evenly: an ordered list of X keys
-                    int tot_unused;
-                    int off = warp_excl_sum(cx, tot_unused);
-                    unsigned m = xm;
-                    while (m) {
-                        const int k = __ffs(m) - 1;
-                        m &= m - 1;
-                        sList[off++] = (int16_t)(lane * IPT + k);
+                    for (int i2 = 0; i2 < NQ; i2++) {
+                        const bool out = act[i2] && pl[i2] <= 0;
+                        if (act[i2] && !out) O[swz(e[i2])] = tile_base + pb[i2] + j[i2];
+                        const unsigned om = __ballot_sync(FULL, out);
+                        if (out) sList[ns + __popc(om & ((1u << lane) - 1u))] = (int16_t)e[i2];
+                        ns += __popc(om);
                     }
                     __syncwarp();
-                    for (int b0 = 0; b0 < xtot; b0 += 32 * NQ) {
-                        int e[NQ];
-                        bool act[NQ];
-#pragma unroll
-                        for (int i2 = 0; i2 < NQ; i2++) {
-                            act[i2] = b0 + 32 * i2 + lane < xtot;
-                            e[i2] = act[i2] ? (int)sList[b0 + 32 * i2 + lane] : 0;
-                        }
-                        resolve(e, act);
-                    }
-                } else {
-                    unsigned m = xm;
-                    for (int rd = 0; rd < xmax; rd += NQ) {
-                        int e[NQ];
-                        bool act[NQ];
-#pragma unroll
-                        for (int i2 = 0; i2 < NQ; i2++) {
-                            act[i2] = m != 0;
-                            e[i2] = lane * IPT + (act[i2] ? __ffs(m) - 1 : 0);
-                            m &= m - 1;
-                        }
-                        resolve(e, act);
-                    }
                 }
             }
+            if (xtot < qtot) {
+                list_keys(smask, (ppre & 0xffff) - xoff);
+                ns = qtot - xtot;
+                __syncwarp();
+            }
 
-            // ---- 5. S keys: search of the range stack -------------------------------------
-            // Entries are strict suffix minima: values increase from bottom to top and
-            // the ones that qualify form a bottom part; the topmost of them answers.
-            // The top 32 entries sit one per lane (the window), so a query is one
-            // ballot.  With nothing ever dropped the bottom entry is the range minimum,
-            // which qualifies; otherwise a miss is "capped": the answer lies in the
-            // range below the kept entries and phase 2 finds it.
-            win_lo = max(stk_lo, stk_hi - 32);
-            const int widx = win_lo + lane;
-            wvalid = widx < stk_hi;
-            wv = wvalid ? sStkV[widx & (K - 1)] : KeyTraits<T>::pad();
-            cm = 0;
-            if (__any_sync(FULL, sm != 0)) {
-                const int wcnt = stk_hi - win_lo;  // window entries (uniform)
-                const int wp = wvalid ? sStkP[widx & (K - 1)] : -1;
-                // the answer of q: the topmost qualifying window entry (by a 6-step
-                // shuffle search), else a binary search below the window; -1 = miss
-                auto search = [&](T q, bool act) {
-                    int lo = -1;
+            // ---- 5. the rest: the range stack (S), else flagged: deferred or capped ---------
+            // Stack entries are strict suffix minima: values increase from bottom to top
+            // and the ones that qualify form a bottom part; the topmost of them answers.
+            // With nothing ever dropped the bottom entry is the range minimum; a key that
+            // the range minimum qualifies for but no kept entry is "capped" (phase 2 finds
+            // its answer in the range), any other is "deferred" (nothing in the range
+            // qualifies).  Flagged keys keep -1; they go to the lists of phase 2 and, for
+            // the lists' overflow, as a mask per tile to global memory.
+            int dtot = 0, ctot = 0;
+            for (int b0 = 0; b0 < ns; b0 += 32) {
+                const bool act = b0 + lane < ns;
+                const int e = act ? (int)sList[b0 + lane] : 0;
+                const T q = V[ks(e)];
+                int ans = -1;
+                if (__any_sync(FULL, act && has_rmin && lt<INCL>(rmin, q))) {
+                    int lo = -1;  // the topmost qualifying entry of the window
 #pragma unroll
                     for (int s2 = 32; s2 > 0; s2 >>= 1) {
                         const int cand = lo + s2;
                         const T wc = __shfl_sync(FULL, wv, cand & 31);
-                        if (act && cand < wcnt && lt<INCL>(wc, q)) lo = cand;
+                        if (cand < stk_hi - win_lo && lt<INCL>(wc, q)) lo = cand;
                     }
-                    const int ap = __shfl_sync(FULL, wp, lo & 31);
-                    int ans = -1;
-                    if (act) {
-                        ans = lo >= 0 ? ap : -1;
-                        if (lo < 0 && win_lo > stk_lo) {
+                    ans = __shfl_sync(FULL, wp, lo & 31);
+                    if (lo < 0) {
+                        ans = -1;
+                        if (act && win_lo > stk_lo) {  // below the window
                             int l2 = stk_lo, h2 = win_lo;
                             while (l2 < h2) {
                                 const int mid = (l2 + h2) >> 1;
@@ -1241,61 +1510,58 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                             if (l2 > stk_lo) ans = sStkP[(l2 - 1) & (K - 1)];
                         }
                     }
-                    return ans;
-                };
-                const int cs = __popc(sm);
-                int stot;
-                const int soff = warp_excl_sum(cs, stot);
-                const int smax = (int)__reduce_max_sync(FULL, (unsigned)cs);
-                if (smax > 1 && stot <= 32) {
-                    // The tile's S keys sit mostly in its first lanes: spread them, one per
-                    // lane, over a single round (the X list is consumed, its space is free).
-                    __syncwarp();
-                    {
-                        int o = soff;
-                        unsigned m = sm;
-                        while (m) {
-                            const int k = __ffs(m) - 1;
-                            m &= m - 1;
-                            sList[o++] = (int16_t)(lane * IPT + k);
+                }
+                if (act && ans >= 0) O[swz(e)] = ans;
+                const bool miss = act && ans < 0;
+                if (__any_sync(FULL, miss)) {
+                    const bool capd = miss && has_rmin && lt<INCL>(rmin, q);
+                    bool defd = miss && !capd;
+                    // Segmented: nothing in the range qualifies for a deferred key; if its
+                    // segment starts inside the range, -1 is its final answer.
+                    if constexpr (SEG) defd = defd && tile_base + e < first_end;
+                    const unsigned db = __ballot_sync(FULL, defd), cb = __ballot_sync(FULL, capd);
+                    if (db | cb) {
+                        uint32_t* fm = (uint32_t*)sSM;  // the suffix minima are no longer needed
+                        if (!(dtot | ctot)) {
+                            if (lane < W) fm[lane] = 0u;
+                            __syncwarp();
                         }
-                    }
-                    __syncwarp();
-                    const bool act = lane < stot;
-                    const int e = act ? (int)sList[lane] : 0;
-                    const int ans = search(act ? V[ks(e)] : KeyTraits<T>::pad(), act);
-                    if (act) O[swz(e)] = ans >= 0 ? ans : -2;  // -2: a miss, flagged by the key's lane
-                    if (__any_sync(FULL, act && ans < 0)) {      // (only once the stack has dropped entries)
-                        __syncwarp();
-                        unsigned m = sm;
-                        while (m) {
-                            const int k = __ffs(m) - 1;
-                            m &= m - 1;
-                            if (O[swz(lane * IPT + k)] == -2) {
-                                O[swz(lane * IPT + k)] = -1;
-                                cm |= 1u << k;
+                        if (defd || capd) atomicOr(&fm[e >> 5], 1u << (e & 31));
+                        const unsigned below = (1u << lane) - 1u;
+                        const int di = def_total + dtot + __popc(db & below);
+                        if (defd && di < kDefCap) {
+                            sDefP[di] = tile_base + e;
+                            sDefV[di] = q;
+                        }
+                        if (cb) {
+                            if (!dropped) atomicOr(err, ERR_INTERNAL);
+                            const int ci = cap_total + ctot + __popc(cb & below);
+                            int sstart = 0;
+                            if constexpr (SEG) {  // the start of the key's segment, from its lane
+                                const unsigned bw = __shfl_sync(FULL, bword, e / IPT) & ((2u << (e % IPT)) - 1u);
+                                sstart = __shfl_sync(FULL, lane_s, e / IPT);
+                                if (bw) sstart = tile_base + e / IPT * IPT + 31 - __clz(bw);
+                            }
+                            if (capd && ci < kCapCap) {
+                                sCapP[ci] = tile_base + e;
+                                if constexpr (SEG) sCapS[ci] = sstart;
                             }
                         }
-                    }
-                } else {
-                    unsigned m = sm;
-                    for (int rd = 0; rd < smax; rd++) {
-                        const bool act = m != 0;
-                        const int k = act ? __ffs(m) - 1 : 0;
-                        m &= m - 1;
-                        const int ans = search(act ? V[ks(lane * IPT + k)] : KeyTraits<T>::pad(), act);
-                        if (act) {
-                            if (ans >= 0) O[swz(lane * IPT + k)] = ans;
-                            else cm |= 1u << k;
-                        }
+                        dtot += __popc(db);
+                        ctot += __popc(cb);
                     }
                 }
-                if (cm && !dropped) atomicOr(err, ERR_INTERNAL);
             }
-            }  // steps 1-5
 
-            // ---- 6. flagged keys: deferred (D) and capped (C) -----------------------------
-            flag_keys(dm, cm);
+            // ---- 6. flagged keys: the tile's mask and flag word -----------------------------
+            if (dtot | ctot) {
+                __syncwarp();
+                if (lane < W) __stcg(&a.s.tile_mask[(size_t)t * MW + lane], ((const uint32_t*)sSM)[lane]);
+                def_total += dtot;
+                cap_total += ctot;
+            }
+            if (lane == 0) __stcg(&a.s.tile_flag[t], (uint32_t)(dtot + ctot) | (ctot ? 0x80000000u : 0u));
+            }  // steps 2-6
 
             // ---- 7. output: the whole tile, flagged keys as -1 ----------------------------
             store_tile();
@@ -1313,22 +1579,6 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     dropped = true;
                 }
             } else {
-                const T after_w = __shfl_down_sync(FULL, suf, 1);  // min of the lanes after (lane < 31)
-                unsigned fmask = 0;
-                const bool has_aft = lane < 31;
-                if (!has_aft || lt<false>(lmin, after_w)) {  // else no key here beats every later key
-                    bool has_run = has_aft;
-                    T run = after_w;
-#pragma unroll
-                    for (int k = IPT - 1; k >= 0; k--) {
-                        if (!has_run || v[k] < run) fmask |= 1u << k;  // strict suffix minimum
-                        run = has_run ? KeyTraits<T>::vmin(run, v[k]) : v[k];
-                        has_run = true;
-                    }
-                }
-                const int fcnt = __popc(fmask);
-                int total;
-                const int fpre = warp_excl_sum(fcnt, total);
                 // Entries below the tile minimum survive: a bottom part of the stack.
                 const unsigned below = __ballot_sync(FULL, wvalid && wv < tile_min_t);
                 int keep;
@@ -1346,20 +1596,18 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     keep = lo;
                 }
                 __syncwarp();  // every lane has read the old stack
-                const int newtop = keep + total;
-                {
-                    int idx = keep + fpre;
-                    unsigned m = fmask;
-                    if (idx + fcnt <= newtop - K) m = 0;  // all of this lane's entries drop at once
-                    while (m) {
-                        const int k = __ffs(m) - 1;
-                        m &= m - 1;
-                        if (idx >= newtop - K) {
-                            sStkV[idx & (K - 1)] = V[ks(lane * IPT + k)];
-                            sStkP[idx & (K - 1)] = lb + k;
-                        }
-                        idx++;
+                const int newtop = keep + (ptot >> 16);
+                int idx = keep + (ppre >> 16);
+                unsigned m = fmask;
+                if (idx + fcnt <= newtop - K) m = 0;  // all of this lane's entries drop at once
+                while (m) {
+                    const int k = __ffs(m) - 1;
+                    m &= m - 1;
+                    if (idx >= newtop - K) {
+                        sStkV[idx & (K - 1)] = V[ks(lane * IPT + k)];
+                        sStkP[idx & (K - 1)] = lb + k;
                     }
+                    idx++;
                 }
                 stk_hi = newtop;
                 if (newtop - K > stk_lo) {
@@ -1403,106 +1651,100 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         __syncwarp();  // lane 0's acquire and wait before every lane's reads and writes
 
         // ======================= phase 2: flagged keys ===============================
-        const T* tile_min_r = (const T*)a.s.tile_min;
-        const T* chunk_min_r = (const T*)a.s.chunk_min;
         const int range_begin = t0 * WT;
-        auto range_end = [&](int rr) { return min(min((rr + 1) * a.tiles_per_range, a.num_tiles) * WT, a.n); };
+        T* sg = sV;  // the TMA ring is idle now: running minima of the earlier groups
+        bool staged = false;
+        T wpm = win;  // running minima of the window, from the nearest range on
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const T nb = __shfl_up_sync(FULL, wpm, o);
+            if (lane >= o) wpm = KeyTraits<T>::vmin(wpm, nb);
+        }
 
         // A. deferred keys: the range's prefix minima, non-increasing, so the ones P
-        //    qualifies form a prefix of the list and the rest keep -1.  Each answer is
-        //    in the nearest earlier range whose minimum qualifies, at the top of its
-        //    published stack (lane-parallel searches), else found by find_left.
+        //    qualifies form a prefix of them and the rest keep -1.  Answers of
+        //    non-increasing queries only move left, so while the last answer's key
+        //    (the cursor) still qualifies it is the answer; else answer_before,
+        //    one key per lane.
         bool a_done = !has_p;
+        int cur = -1;
+        T cv = KeyTraits<T>::pad();
+        // up to 32 deferred keys in order, one per lane (uniform call)
+        auto deferred32 = [&](const bool in, const T q, const int pos) {
+            const bool want = in && lt<INCL>(P, q);  // (segmented: all of the range's first segment)
+            if (__ballot_sync(FULL, want) != __ballot_sync(FULL, in)) a_done = true;
+            const bool ok = want && cur >= 0 && lt<INCL>(cv, q);
+            if (ok && (!head || pos >= head)) put(pos, SEG ? seg_rel(cur, first_start) : cur);
+            const bool rest = want && !ok;
+            const unsigned rm = __ballot_sync(FULL, rest);
+            if (!rm) return;
+            const int ans = answer_before<T, WT, INCL, MAPF, REV>(q, rest, r, wpm, sg, staged, d_in, a);
+            if (rest) {
+                if (ans < 0) atomicOr(err, ERR_INTERNAL);
+                else if (!head || pos >= head) put(pos, SEG ? seg_rel(ans, first_start) : ans);
+            }
+            cur = __shfl_sync(FULL, ans, 31 - __clz(rm));
+            if (cur < 0) {
+                a_done = true;
+            } else if (SEG && cur < first_start) {
+                a_done = true;  // before the segment: so are the answers of the lower keys (-1 already)
+            } else if (!a_done) {
+                cv = key_at<T, MAPF, REV>(d_in, a.n, cur);
+            }
+        };
         const int nlist = min(def_total, kDefCap);
         for (int b0 = 0; b0 < nlist && !a_done; b0 += 32) {
             const int j = b0 + lane;
             const bool in = j < nlist;
-            const T q = in ? sDefV[j] : KeyTraits<T>::pad();
-            const int pos = in ? sDefP[j] : 0;
-            const bool want = in && lt<INCL>(P, q);  // (segmented: all of the range's first segment)
-            if (__ballot_sync(FULL, want) != __ballot_sync(FULL, in)) a_done = true;
-            if (!__any_sync(FULL, want)) break;
-            int rp = -1;
-#pragma unroll 4
-            for (int i2 = 0; i2 < 32; i2++) {
-                const T m = __shfl_sync(FULL, win, i2);
-                if (want && rp < 0 && r - 1 - i2 >= 0 && lt<INCL>(m, q)) rp = r - 1 - i2;
-            }
-            {  // no range of the window qualifies: the nearest one below it, key by key
-                unsigned nw = __ballot_sync(FULL, want && rp < 0);
-                while (nw) {
-                    const int f = __ffs(nw) - 1;
-                    nw &= nw - 1;
-                    const int found = nearest_range<T, INCL>(__shfl_sync(FULL, q, f), r - 33, a);
-                    if (lane == f) rp = found;
-                }
-            }
-            int ans = -2;  // -2: not found yet
-            if (want && rp >= 0) {
-                // rp's published stack top, keys and positions in one round of loads:
-                // entries increase from the bottom, so the qualifying ones form a
-                // bottom part and the topmost of them answers
-                const int cnt = (int)(__ldcg(&a.s.top_cnt[rp]) & 0xffu);
-                const uint4* tk = reinterpret_cast<const uint4*>((const T*)a.s.top_key + (size_t)rp * kTopEntries);
-                const uint4* tp = reinterpret_cast<const uint4*>(a.s.top_pos + (size_t)rp * kTopEntries);
-                if constexpr (KB == 4) {
-                    uint4 tw[kTopEntries / 4], pw[kTopEntries / 4];
-#pragma unroll
-                    for (int k = 0; k < kTopEntries / 4; k++) {
-                        tw[k] = __ldcg(&tk[k]);
-                        pw[k] = __ldcg(&tp[k]);
-                    }
-#pragma unroll
-                    for (int k = 0; k < kTopEntries / 4; k++) {
-                        const uint32_t wb[4] = {tw[k].x, tw[k].y, tw[k].z, tw[k].w};
-                        const int pb[4] = {(int)pw[k].x, (int)pw[k].y, (int)pw[k].z, (int)pw[k].w};
-#pragma unroll
-                        for (int c = 0; c < 4; c++)
-                            if (4 * k + c < cnt && lt<INCL>(KeyTraits<T>::from_bits(wb[c]), q)) ans = pb[c];
-                    }
-                } else {  // two 8-byte keys per 16-byte load
-                    uint4 tw[kTopEntries / 2], pw[kTopEntries / 4];
-#pragma unroll
-                    for (int k = 0; k < kTopEntries / 2; k++) tw[k] = __ldcg(&tk[k]);
-#pragma unroll
-                    for (int k = 0; k < kTopEntries / 4; k++) pw[k] = __ldcg(&tp[k]);
-#pragma unroll
-                    for (int k = 0; k < kTopEntries / 2; k++) {
-                        const uint64_t kb2[2] = {((uint64_t)tw[k].y << 32) | tw[k].x, ((uint64_t)tw[k].w << 32) | tw[k].z};
-                        const uint4 p4 = pw[k / 2];
-                        const int pb2[2] = {(int)(k % 2 ? p4.z : p4.x), (int)(k % 2 ? p4.w : p4.y)};
-#pragma unroll
-                        for (int c = 0; c < 2; c++)
-                            if (2 * k + c < cnt && lt<INCL>(KeyTraits<T>::from_bits(kb2[c]), q)) ans = pb2[c];
-                    }
-                }
-            }
-            unsigned fb = __ballot_sync(FULL, want && ans == -2);
-            while (fb) {
-                const int f = __ffs(fb) - 1;
-                fb &= fb - 1;
-                const T qf = __shfl_sync(FULL, q, f);
-                const int rpf = __shfl_sync(FULL, rp, f);
-                const int lim = rpf >= 0 ? range_end(rpf) : range_begin;
-                const int found = find_left<T, WT, INCL, MAPF, REV>(qf, lim, d_in, tile_min_r, chunk_min_r, a);
-                if (lane == f) ans = found;
-            }
-            if (want) {
-                if (ans < 0) atomicOr(err, ERR_INTERNAL);
-                else if (!head || pos >= head) put(pos, SEG ? seg_rel(ans, first_start) : ans);
-            }
+            deferred32(in, in ? sDefV[j] : KeyTraits<T>::pad(), in ? sDefP[j] : 0);
         }
+        // The flagged keys at or after `from` of tile t, 32 per step (uniform call).  A
+        // mixed tile's keys look in the earlier tiles of the range first (capped keys
+        // are answered there, deferred ones are not); with_deferred: keys without an
+        // answer there go to deferred32.
+        auto flagged_tile = [&](const int t, const bool mixed, const int from, const bool with_deferred) {
+            uint32_t mw = lane < W ? __ldcg(&a.s.tile_mask[(size_t)t * MW + lane]) : 0u;
+            if (lane < W) {
+                const int p0 = t * WT + 32 * lane, lim = max(from, head);
+                if (p0 < lim) mw &= lim - p0 >= 32 ? 0u : (0xffffffffu << (lim - p0));
+            }
+            int tot;
+            int off = warp_excl_sum(__popc(mw), tot);
+            __syncwarp();
+            while (mw) {
+                const int k = __ffs(mw) - 1;
+                mw &= mw - 1;
+                sList[off++] = (int16_t)(32 * lane + k);
+            }
+            __syncwarp();
+            for (int b0 = 0; b0 < tot; b0 += 32) {
+                bool in = b0 + lane < tot;
+                const int pos = t * WT + (in ? (int)sList[b0 + lane] : 0);
+                const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
+                if (mixed) {
+                    const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, t, d_in, a);
+                    if constexpr (SEG) {  // the keys' own segments, one after another
+                        for (unsigned m = __ballot_sync(FULL, in && found >= 0); m; m &= m - 1) {
+                            const int f = __ffs(m) - 1;
+                            const int sf = (int)seg_off(seg_idx(__shfl_sync(FULL, pos, f) - head)) + head;
+                            if (lane == f) put(pos, seg_rel(found, sf));
+                        }
+                    } else if (in && found >= 0) {
+                        put(pos, found);
+                    }
+                    // (segmented: flagged keys without an answer in the range are of its first segment)
+                    in = in && found < 0;
+                }
+                if (with_deferred && !a_done) deferred32(in, q, pos);
+            }
+            __syncwarp();
+        };
         if (!a_done && def_total > kDefCap) {
             // A'. the list overflowed and P qualified every listed key: continue over
-            //     the tile flags after the last listed key, with a monotone cursor
-            //     (answers of non-increasing queries only move left).
-            //     Flag words 32 tiles per load (lane i: tile tb + i), a tile's mask
-            //     words in one load (lane w: word w): the scan pays one L2 round
-            //     trip per 32 tiles and one per flagged tile, not one per tile and word.
+            //     the tile flags after the last listed key, 32 tiles per load.
             const int from = sDefP[kDefCap - 1] + 1;
-            int cur = -1;
-            T cv = KeyTraits<T>::pad();
-            static_assert(W <= 16, "two tiles' mask words per load");
+            constexpr int TPL = 32 / W;  // tiles per load of mask words
+            const T* tile_min_r = (const T*)a.s.tile_min;
             for (int tb = from / WT; tb < t1 && !a_done; tb += 32) {
               const bool tin = tb + lane < t1;
               const uint32_t tfl = tin ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
@@ -1512,161 +1754,71 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 // Flagged tiles whose pending keys all take the cursor: not mixed, and
                 // P and the cursor's key both qualify for the tile's minimum (<= every
                 // pending key).  Pending keys do not increase, so these form a prefix
-                // of the flagged tiles; their keys are not read, and the mask words of
-                // two tiles come in one load (lanes 0-15 and 16-31).
+                // of the flagged tiles; their keys are not read.  A tile that is all
+                // pending takes the cursor in 16-byte stores without its masks; of
+                // the others the masks of 32/W tiles come in one load.
                 const unsigned fast = __ballot_sync(
                     FULL, ((fl >> lane) & 1u) && (tfl >> 31) == 0 && cur >= 0 && lt<INCL>(P, tmn) && lt<INCL>(cv, tmn));
                 const unsigned slow = fl & ~fast;
                 unsigned take = slow ? fl & ((slow & (0u - slow)) - 1u) : fl;
                 fl &= ~take;
-                while (take) {
-                    const int ta = __ffs(take) - 1;
-                    take &= take - 1;
-                    const int tb2 = take ? __ffs(take) - 1 : -1;
-                    if (take) take &= take - 1;
-                    const int mine = lane < 16 ? ta : tb2;
-                    const uint32_t mw2 =
-                        mine >= 0 && (lane & 15) < W ? __ldcg(&a.s.tile_mask[(size_t)(tb + mine) * MW + (lane & 15)]) : 0u;
+                unsigned whole = __ballot_sync(FULL, ((take >> lane) & 1u) && (tfl & 0x3fffffffu) == (uint32_t)WT &&
+                                                         (tb + lane) * WT >= from && tile_full(tb + lane));
+                take &= ~whole;
+                while (whole) {
+                    const int t = tb + __ffs(whole) - 1;
+                    whole &= whole - 1;
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const int tt = h ? tb2 : ta;
-                        if (tt < 0) break;
+                    for (int j = 0; j < WT / 128; j++) put4(t * WT + 128 * j + 4 * lane, SEG ? seg_rel(cur, first_start) : cur);
+                }
+                while (take) {
+                    int tt[TPL], mine = -1;
+#pragma unroll
+                    for (int h = 0; h < TPL; h++) {
+                        tt[h] = take ? __ffs(take) - 1 : -1;
+                        if (take) take &= take - 1;
+                        if (lane / W == h) mine = tt[h];
+                    }
+                    const uint32_t mw2 = mine >= 0 ? __ldcg(&a.s.tile_mask[(size_t)(tb + mine) * MW + (lane % W)]) : 0u;
+#pragma unroll
+                    for (int h = 0; h < TPL; h++) {
+                        if (tt[h] < 0) break;
 #pragma unroll
                         for (int w = 0; w < W; w++) {
-                            const uint32_t mw = __shfl_sync(FULL, mw2, 16 * h + w);
-                            const int pos = (tb + tt) * WT + w * 32 + lane;
+                            const uint32_t mw = __shfl_sync(FULL, mw2, W * h + w);
+                            const int pos = (tb + tt[h]) * WT + w * 32 + lane;
                             if (((mw >> lane) & 1u) && pos >= from && (!head || pos >= head))
                                 put(pos, SEG ? seg_rel(cur, first_start) : cur);
                         }
                     }
                 }
                 if (!fl) break;
-                // the first other flagged tile, key by key
-                const int fsrc = __ffs(fl) - 1;
+                const int fsrc = __ffs(fl) - 1;  // the first other flagged tile, key by key
                 fl &= fl - 1;
-                const int t = tb + fsrc;
-                const bool mixed = (__shfl_sync(FULL, tfl, fsrc) >> 31) != 0;
-                const uint32_t mwl = lane < W ? __ldcg(&a.s.tile_mask[(size_t)t * MW + lane]) : 0u;
-                // The tile's pending keys, every word's loads in flight together, staged
-                // in the idle TMA ring (each lane reads back only its own slots).
-#pragma unroll
-                for (int w = 0; w < W; w++) {
-                    const uint32_t mw = __shfl_sync(FULL, mwl, w);
-                    const int pos = t * WT + w * 32 + lane;
-                    const bool pk = ((mw >> lane) & 1u) && pos >= from && (!head || pos >= head);
-                    sV[w * 32 + lane] = pk ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
-                }
-                for (int w = 0; w < W && !a_done; w++) {
-                    const uint32_t mw = __shfl_sync(FULL, mwl, w);
-                    const int pos = t * WT + w * 32 + lane;
-                    unsigned pend = __ballot_sync(FULL, ((mw >> lane) & 1u) && pos >= from && (!head || pos >= head));
-                    if (!pend) continue;
-                    const T q = ((pend >> lane) & 1u) ? sV[w * 32 + lane] : KeyTraits<T>::pad();
-                    if (mixed) {  // deferred and capped keys: a full search each
-                        while (pend) {
-                            const int f = __ffs(pend) - 1;
-                            pend &= pend - 1;
-                            const int pf = t * WT + w * 32 + f;
-                            const int found = find_left<T, WT, INCL, MAPF, REV>(__shfl_sync(FULL, q, f), pf, d_in, tile_min_r,
-                                                                     chunk_min_r, a);
-                            int sf = 0;
-                            if constexpr (SEG) sf = (int)seg_off(seg_idx(pf - head)) + head;
-                            if (lane == f) {
-                                if (found < -1) atomicOr(err, ERR_INTERNAL);
-                                else put(pos, SEG ? seg_rel(found, sf) : found);
-                            }
-                        }
-                        continue;
-                    }
-                    const unsigned wq = __ballot_sync(FULL, ((pend >> lane) & 1u) && lt<INCL>(P, q));
-                    if (wq != pend) {
-                        a_done = true;
-                        pend = wq;
-                    }
-                    while (pend) {
-                        // the pending keys, in order, up to the first one the cursor's
-                        // key does not qualify for, take the cursor
-                        const unsigned ok = __ballot_sync(FULL, ((pend >> lane) & 1u) && cur >= 0 && lt<INCL>(cv, q));
-                        const unsigned fail = pend & ~ok;
-                        const unsigned tk = fail ? (pend & ((fail & (0u - fail)) - 1u)) : pend;
-                        if ((tk >> lane) & 1u) put(pos, SEG ? seg_rel(cur, first_start) : cur);
-                        pend &= ~tk;
-                        if (!pend) break;
-                        const int f = __ffs(pend) - 1;
-                        const T qf = __shfl_sync(FULL, q, f);
-                        // qf's answer lies before the range: in the nearest earlier range
-                        // whose minimum qualifies (the window, else the group minima), at
-                        // the topmost qualifying entry of that range's final stack (every
-                        // key after it there is >= qf); find_left when the published top
-                        // part does not reach it
-                        int found = -2;
-                        {
-                            const unsigned wm = __ballot_sync(FULL, r - 1 - lane >= 0 && lt<INCL>(win, qf));
-                            const int rpf = wm ? r - 1 - (__ffs(wm) - 1) : nearest_range<T, INCL>(qf, r - 33, a);
-                            if (rpf >= 0) {
-                                const int cnt = (int)(__ldcg(&a.s.top_cnt[rpf]) & 0xffu);
-                                const T tkey = lane < cnt ? __ldcg(&((const T*)a.s.top_key)[(size_t)rpf * kTopEntries + lane])
-                                                          : KeyTraits<T>::pad();
-                                const unsigned m = __ballot_sync(FULL, lane < cnt && lt<INCL>(tkey, qf));
-                                found = m ? __ldcg(&a.s.top_pos[(size_t)rpf * kTopEntries + 31 - __clz(m)])
-                                          : find_left<T, WT, INCL, MAPF, REV>(qf, range_end(rpf), d_in, tile_min_r, chunk_min_r, a);
-                            }
-                        }
-                        if (found < 0) {
-                            if (lane == 0) atomicOr(err, ERR_INTERNAL);
-                            pend = 0;
-                            a_done = true;
-                        } else {
-                            cur = found;
-                            cv = key_at<T, MAPF, REV>(d_in, a.n, cur);
-                        }
-                    }
-                }
+                flagged_tile(tb + fsrc, (__shfl_sync(FULL, tfl, fsrc) >> 31) != 0, from, true);
               }
             }
         }
 
         // B. capped keys: the answer is in the range, below the stack's kept part.
         const int ncap = min(cap_total, kCapCap);
-        for (int j = 0; j < ncap; j++) {
-            const int pos = sCapP[j];
-            const int found = find_left<T, WT, INCL, MAPF, REV>(key_at<T, MAPF, REV>(d_in, a.n, pos), pos, d_in, tile_min_r,
-                                                           chunk_min_r, a);
-            if (lane == 0) {
+        for (int b0 = 0; b0 < ncap; b0 += 32) {
+            const bool in = b0 + lane < ncap;
+            const int pos = in ? sCapP[b0 + lane] : range_begin;
+            const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
+            const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, pos / WT, d_in, a);
+            if (in) {
                 if (found < 0) atomicOr(err, ERR_INTERNAL);
-                else if (!head || pos >= head) put(pos, SEG ? seg_rel(found, sCapS[j]) : found);
+                else if (!head || pos >= head) put(pos, SEG ? seg_rel(found, sCapS[b0 + lane]) : found);
             }
         }
         if (cap_total > kCapCap) {
             // B'. the capped list overflowed: every flagged key of the mixed tiles after it
-            //     (flag and mask words loaded 32 at a time, as in A')
             const int from = sCapP[kCapCap - 1] + 1;
             for (int tb = from / WT; tb < t1; tb += 32) {
-              const uint32_t tfl = tb + lane < t1 ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
-              unsigned fl = __ballot_sync(FULL, (tfl >> 31) != 0);
-              while (fl) {
-                const int t = tb + __ffs(fl) - 1;
-                fl &= fl - 1;
-                const uint32_t mwl = lane < W ? __ldcg(&a.s.tile_mask[(size_t)t * MW + lane]) : 0u;
-                for (int w = 0; w < W; w++) {
-                    const uint32_t mw = __shfl_sync(FULL, mwl, w);
-                    const int pos = t * WT + w * 32 + lane;
-                    unsigned pend = __ballot_sync(FULL, ((mw >> lane) & 1u) && pos >= from && (!head || pos >= head));
-                    while (pend) {
-                        const int f = __ffs(pend) - 1;
-                        pend &= pend - 1;
-                        const int pf = t * WT + w * 32 + f;
-                        const int found =
-                            find_left<T, WT, INCL, MAPF, REV>(key_at<T, MAPF, REV>(d_in, a.n, pf), pf, d_in, tile_min_r, chunk_min_r, a);
-                        int sf = 0;
-                        if constexpr (SEG) sf = (int)seg_off(seg_idx(pf - head)) + head;
-                        if (lane == f) {
-                            if (found < -1) atomicOr(err, ERR_INTERNAL);
-                            else put(pf, SEG ? seg_rel(found, sf) : found);
-                        }
-                    }
-                }
-              }
+                const uint32_t tfl = tb + lane < t1 ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
+                for (unsigned fl = __ballot_sync(FULL, (tfl >> 31) != 0); fl; fl &= fl - 1)
+                    flagged_tile(tb + __ffs(fl) - 1, true, from, false);
             }
         }
     }
