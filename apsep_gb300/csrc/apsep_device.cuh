@@ -210,6 +210,13 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // Completed bulk (async-proxy) writes to global -> ordered before later generic accesses.
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
+// Asynchronous copy of 16 bytes from global to shared memory, through L2 only
+// (both addresses 16-byte aligned), and the wait for all of the thread's copies.
+__device__ __forceinline__ void copy_async16(void* smem_dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
 }

@@ -88,10 +88,12 @@ struct WLayout {
     static constexpr size_t kCapS = kCapP + (size_t)kCapCap * 4;      // int32[kCapCap]: segment starts
     static constexpr size_t kPad = (kCapS + (size_t)kCapCap * 4 + 15) / 16 * 16;  // T[4]: pads (lane 0's earlier keys)
     static constexpr size_t kBar = kPad + 4 * KB;  // uint64[S]
-    static constexpr size_t kEnd = kBar + (size_t)kStagesOf<KB> * 8;
+    static constexpr size_t kFlag = kBar + (size_t)kStagesOf<KB> * 8;  // int32: phase 2's group minima are staged
+    static constexpr size_t kEnd = kFlag + 8;
     static constexpr size_t kBytes = (kEnd + 1023) / 1024 * 1024;     // keeps every warp 1024-aligned
     static_assert(kO % 1024 == 0 && kSM % 1024 == 0 && (WT * KB) % 1024 == 0,
                   "swizzled buffers need 1024-byte alignment");
+    static_assert(kList - kV >= (size_t)KB * (kMaxRanges / 32 + 8 * 32) + 4 * 8 * 32, "room for phase 2's staging");
     static_assert(kStkV % 8 == 0 && kDefV % 8 == 0, "8-byte keys need 8-byte aligned arrays");
 };
 
@@ -127,9 +129,15 @@ __device__ __forceinline__ T range_min(const RangeArgs& a, int i) {
 template <typename T>
 __device__ __forceinline__ T group_min_of(const RangeArgs& a, int g) {
     if constexpr (sizeof(T) == 8) {
+        const ulonglong2* w = reinterpret_cast<const ulonglong2*>(&a.s.range_key[32 * g]);
+        ulonglong2 u[16];  // every range of the group is there: it lies before some published range's group
+#pragma unroll
+        for (int i = 0; i < 16; i++) u[i] = __ldcg(w + i);
         T m = KeyTraits<T>::pad();
 #pragma unroll
-        for (int i = 0; i < 32; i++) m = KeyTraits<T>::vmin(m, range_min<T>(a, min(32 * g + i, a.num_ranges - 1)));
+        for (int i = 0; i < 16; i++)
+            m = KeyTraits<T>::vmin(m, KeyTraits<T>::vmin(KeyTraits<T>::from_bits((uint64_t)u[i].x),
+                                                         KeyTraits<T>::from_bits((uint64_t)u[i].y)));
         return m;
     } else {
         return group_key<T>(&a.s.group_min[g]);
@@ -179,6 +187,33 @@ __device__ __forceinline__ T key_at(const T* d_in, int n, int pos) {
     return load_key<T, KMAP>(d_in + (REV ? n - 1 - pos : pos));
 }
 
+// N consecutive keys or minima through L2, 16 bytes per load where they are aligned.
+template <typename T, int N>
+__device__ __forceinline__ void load_run(const T* p, T (&m)[32]) {
+    constexpr int PER = 16 / (int)sizeof(T);
+    static_assert(N <= 32 && N % PER == 0, "whole 16-byte loads");
+    if (((uintptr_t)p & 15) == 0) {
+        uint4 w[N / PER];
+#pragma unroll
+        for (int k = 0; k < N / PER; k++) w[k] = __ldcg(reinterpret_cast<const uint4*>(p) + k);
+#pragma unroll
+        for (int k = 0; k < N / PER; k++) {
+            if constexpr (sizeof(T) == 4) {
+                m[4 * k] = KeyTraits<T>::from_bits(w[k].x);
+                m[4 * k + 1] = KeyTraits<T>::from_bits(w[k].y);
+                m[4 * k + 2] = KeyTraits<T>::from_bits(w[k].z);
+                m[4 * k + 3] = KeyTraits<T>::from_bits(w[k].w);
+            } else {
+                m[2 * k] = KeyTraits<T>::from_bits(((uint64_t)w[k].y << 32) | w[k].x);
+                m[2 * k + 1] = KeyTraits<T>::from_bits(((uint64_t)w[k].w << 32) | w[k].z);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < N; k++) m[k] = __ldcg(p + k);
+    }
+}
+
 // Phase 2's searches take up to kFew queries one by one, the warp's lanes side by
 // side on 32 entries of a level (one load and a ballot a step), and more of them
 // one per lane (a round of independent loads a step for all): a lone query is
@@ -225,27 +260,29 @@ __device__ __noinline__ int find_in_tiles(T q, bool need, int lo, int hi, const 
     for (int t = hi - 1; need && s < 0 && t >= lo; t -= 16) {
         T m[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) m[k] = __ldcg(&tile_min[max(t - k, lo)]);
+        for (int k = 0; k < 16; k++) m[k] = t - k >= lo ? __ldcg(&tile_min[t - k]) : KeyTraits<T>::pad();
 #pragma unroll
         for (int k = 0; k < 16; k++)
             if (s < 0 && t - k >= lo && lt<INCL>(m[k], q)) s = t - k;
     }
     int p = -2;
     if (need && s >= 0) {
+        T m[32];
+        load_run<T, W>(chunk_min + (size_t)s * W, m);
         int c = 0;
 #pragma unroll
         for (int k = 0; k < W; k++)
-            if (lt<INCL>(__ldcg(&chunk_min[(size_t)s * W + k]), q)) c = k;
-        const int row = s * B + c * 32;
-#pragma unroll 1
-        for (int h = 16; h >= 0 && p < 0; h -= 16) {
-            T m[16];
+            if (lt<INCL>(m[k], q)) c = k;
+        const int row = s * B + c * 32;  // (whole tiles lie below hi: the row ends inside the array)
+        if (row >= a.head) {
+            load_run<T, 32>(d_in + (REV ? a.n - 32 - row : row), m);
+        } else {  // the view's virtual keys are not read
 #pragma unroll
-            for (int k = 0; k < 16; k++) m[k] = key_at<T, MAPF, REV>(d_in, a.n, min(max(row + h + k, a.head), a.n - 1));
-#pragma unroll
-            for (int k = 0; k < 16; k++)
-                if (row + h + k >= a.head && row + h + k < a.n && lt<INCL>(m[k], q)) p = row + h + k;
+            for (int k = 0; k < 32; k++) m[k] = __ldcg(&d_in[max(row + k, a.head)]);
         }
+#pragma unroll
+        for (int k = 0; k < 32; k++)
+            if (row + k >= a.head && lt<INCL>(map_key<T, MAPF>(m[REV ? 31 - k : k]), q)) p = row + k;
     }
     __syncwarp();
     return p;
@@ -260,7 +297,7 @@ __device__ __noinline__ int find_in_tiles(T q, bool need, int lo, int hi, const 
 // range's published stack, else its tiles.  -2: the published minima contradict
 // each other.
 template <typename T, int B, bool INCL, int MAPF = KMAP_NONE, bool REV = false>
-__device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, bool& staged,
+__device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, int* staged,
                                           const T* __restrict__ d_in, const RangeArgs& a) {
     constexpr unsigned FULL = 0xffffffffu;
     constexpr int KB = (int)sizeof(T);
@@ -316,7 +353,7 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, b
     }
     {
         int lo = -1;  // the nearest lo + 1 ranges do not qualify
-#pragma unroll
+#pragma unroll 1
         for (int s = 16; s > 0; s >>= 1)
             if (!lt<INCL>(__shfl_sync(FULL, wpm, lo + s), q)) lo += s;
         if (lt<INCL>(__shfl_sync(FULL, wpm, lo + 1), q)) rp = max(r - 2 - lo, -1);
@@ -324,14 +361,22 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, b
     if (__any_sync(FULL, want && rp < 0)) {
         const int ng = r >= 33 ? ((r - 33) >> 5) + 1 : 0;  // groups of earlier ranges (the window's part does not qualify)
         static_assert(kMaxRanges / 32 == 128, "four groups per lane");
-        if (!staged) {
+        if (!*staged) {
+            __syncwarp();
+#pragma unroll 1
+            for (int g = lane; g < kMaxRanges / 32; g += 32) {
+                T m = KeyTraits<T>::pad();
+                if (g < ng) m = group_min_of<T>(a, g);
+                sg[g] = m;
+            }
+            __syncwarp();
             T m[4];
 #pragma unroll
-            for (int j = 0; j < 4; j++) m[j] = 4 * lane + j < ng ? group_min_of<T>(a, 4 * lane + j) : KeyTraits<T>::pad();
+            for (int j = 0; j < 4; j++) m[j] = sg[4 * lane + j];
 #pragma unroll
             for (int j = 2; j >= 0; j--) m[j] = KeyTraits<T>::vmin(m[j], m[j + 1]);
             T x = m[0];
-#pragma unroll
+#pragma unroll 1
             for (int o = 1; o < 32; o <<= 1) {
                 const T y = __shfl_down_sync(FULL, x, o);
                 if (lane + o < 32) x = KeyTraits<T>::vmin(x, y);
@@ -340,67 +385,70 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, b
             __syncwarp();
 #pragma unroll
             for (int j = 0; j < 4; j++) sg[4 * lane + j] = lane < 31 ? KeyTraits<T>::vmin(m[j], after) : m[j];
+            if (lane == 0) *staged = 1;
             __syncwarp();
-            staged = true;
         }
         if (want && rp < 0 && ng > 0) {
             int g = 0;
-#pragma unroll
+#pragma unroll 1
             for (int s = 64; s > 0; s >>= 1)
                 if (g + s < ng && lt<INCL>(sg[g + s], q)) g += s;
-#pragma unroll 1
-            for (int h = 16; h >= 0 && rp < 0; h -= 16) {
-                T m[16];
+            // its 32 range minima, two words a load (8-byte keys: their key words)
+            const uint4* w = reinterpret_cast<const uint4*>(KB == 8 ? &a.s.range_key[32 * g] : &a.s.range_state[32 * g]);
+            uint4 u[16];
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int i = 32 * g + h + k;
-                    if constexpr (KB == 8) m[k] = range_min<T>(a, i);
-                    else m[k] = KeyTraits<T>::from_bits(__ldcg((const uint32_t*)&a.s.range_state[i]));
+            for (int k = 0; k < 16; k++) u[k] = __ldcg(w + k);
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                T m0, m1;
+                if constexpr (KB == 8) {
+                    m0 = KeyTraits<T>::from_bits(((uint64_t)u[k].y << 32) | u[k].x);
+                    m1 = KeyTraits<T>::from_bits(((uint64_t)u[k].w << 32) | u[k].z);
+                } else {
+                    m0 = KeyTraits<T>::from_bits(u[k].x);
+                    m1 = KeyTraits<T>::from_bits(u[k].z);
                 }
-#pragma unroll
-                for (int k = 0; k < 16; k++)
-                    if (lt<INCL>(m[k], q)) rp = 32 * g + h + k;
+                if (lt<INCL>(m0, q)) rp = 32 * g + 2 * k;
+                if (lt<INCL>(m1, q)) rp = 32 * g + 2 * k + 1;
             }
         }
     }
+    // The published stack tops of the ranges that lanes ask for, up to kSlots of them
+    // copied to shared memory at a time (all copies in flight together), then searched
+    // by the lanes side by side: entries increase from the bottom, so the qualifying
+    // ones form a bottom part and the topmost of them answers.
+    constexpr int kSlots = 8;
+    T* sk = sg + kMaxRanges / 32;               // T[kSlots][32]
+    int32_t* sp = (int32_t*)(sk + kSlots * 32);  // int32[kSlots][32]
     int ans = -2;
-    if (want && rp >= 0) {
-        // rp's published stack top, keys and positions in one round of loads:
-        // entries increase from the bottom, so the qualifying ones form a
-        // bottom part and the topmost of them answers
-        const int cnt = (int)(__ldcg(&a.s.top_cnt[rp]) & 0xffu);
-        const uint4* tk = reinterpret_cast<const uint4*>((const T*)a.s.top_key + (size_t)rp * kTopEntries);
-        const uint4* tp = reinterpret_cast<const uint4*>(a.s.top_pos + (size_t)rp * kTopEntries);
-        if constexpr (KB == 4) {
-            uint4 tw[kTopEntries / 4], pw[kTopEntries / 4];
-#pragma unroll
-            for (int k = 0; k < kTopEntries / 4; k++) {
-                tw[k] = __ldcg(&tk[k]);
-                pw[k] = __ldcg(&tp[k]);
-            }
-#pragma unroll
-            for (int k = 0; k < kTopEntries / 4; k++) {
-                const uint32_t wb[4] = {tw[k].x, tw[k].y, tw[k].z, tw[k].w};
-                const int pb[4] = {(int)pw[k].x, (int)pw[k].y, (int)pw[k].z, (int)pw[k].w};
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-                    if (4 * k + c < cnt && lt<INCL>(KeyTraits<T>::from_bits(wb[c]), q)) ans = pb[c];
-            }
-        } else {  // two 8-byte keys per 16-byte load
-            uint4 tw[kTopEntries / 2], pw[kTopEntries / 4];
-#pragma unroll
-            for (int k = 0; k < kTopEntries / 2; k++) tw[k] = __ldcg(&tk[k]);
-#pragma unroll
-            for (int k = 0; k < kTopEntries / 4; k++) pw[k] = __ldcg(&tp[k]);
-#pragma unroll
-            for (int k = 0; k < kTopEntries / 2; k++) {
-                const uint64_t kb2[2] = {((uint64_t)tw[k].y << 32) | tw[k].x, ((uint64_t)tw[k].w << 32) | tw[k].z};
-                const uint4 p4 = pw[k / 2];
-                const int pb2[2] = {(int)(k % 2 ? p4.z : p4.x), (int)(k % 2 ? p4.w : p4.y)};
-#pragma unroll
-                for (int c = 0; c < 2; c++)
-                    if (2 * k + c < cnt && lt<INCL>(KeyTraits<T>::from_bits(kb2[c]), q)) ans = pb2[c];
-            }
+    const int rq = want ? rp : -1;
+    unsigned todo = __ballot_sync(FULL, rq >= 0);
+    while (todo) {
+        int slot = -1, cnt = 0, ns = 0;
+        __syncwarp();
+#pragma unroll 1
+        for (; todo && ns < kSlots; ns++) {
+            const int rc = __shfl_sync(FULL, rq, __ffs(todo) - 1);
+            const unsigned same = __ballot_sync(FULL, rq == rc);
+            todo &= ~same;
+            if (rq == rc) slot = ns;
+            if (lane == ns) cnt = (int)(__ldcg(&a.s.top_cnt[rc]) & 0xffu);
+            static_assert(kTopEntries == 32, "2 KB lanes copy the keys of a stack top, 8 its positions");
+            if (lane < 2 * KB)
+                copy_async16((char*)(sk + ns * 32) + 16 * lane,
+                             (const char*)((const T*)a.s.top_key + (size_t)rc * kTopEntries) + 16 * lane);
+            else if (lane < 2 * KB + 8)
+                copy_async16(sp + ns * 32 + 4 * (lane - 2 * KB), a.s.top_pos + (size_t)rc * kTopEntries + 4 * (lane - 2 * KB));
+        }
+        copy_async_wait();
+        __syncwarp();
+        cnt = __shfl_sync(FULL, cnt, slot & 31);
+        if (slot >= 0) {
+            int lo = -1;
+#pragma unroll 1
+            for (int s = 32; s > 0; s >>= 1)
+                if (lo + s < cnt && lt<INCL>(sk[slot * 32 + lo + s], q)) lo += s;
+            if (lo >= 0) ans = sp[slot * 32 + lo];
         }
     }
     const bool miss = want && rp >= 0 && ans == -2;
@@ -558,6 +606,291 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, T& p, bo
     }
 }
 
+// ---------------------------------------------------------------------------
+// Phase 2 of range r: its flagged keys, whose answers need the other ranges'
+// publications.  A function of its own: its registers (up to 32 loads in flight a
+// lane) then cost phase 1 none (inlined, the 8-byte kernels spilled there: 125 ->
+// 142 us at 2^24 int64 keys).
+// ---------------------------------------------------------------------------
+template <typename T, int IPT, bool INCL, bool SEG, int MAPF, int OUTM, bool REV>
+__device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, const int r, const int t0, const int t1,
+                                    const int def_total, const int cap_total, const int first_start, const T P,
+                                    const bool has_p, const T win) {
+    constexpr int KB = (int)sizeof(T);
+    using L = WLayout<IPT, KB>;
+    constexpr int WT = L::WT, W = WT / 32, RPT = W * KB / 4, MW = kMaxTileKeys / 32, kDefCap = kDefCapOf<KB>;
+    constexpr unsigned FULL = 0xffffffffu;
+    constexpr bool OUT64 = OUTM == OUT_I64;
+    const int lane = threadIdx.x & 31;
+    T* sV = (T*)(wsm + L::kV);
+    int16_t* sList = (int16_t*)(wsm + L::kList);
+    const int32_t* sDefP = (const int32_t*)(wsm + L::kDefP);
+    const T* sDefV = (const T*)(wsm + L::kDefV);
+    const int32_t* sCapP = (const int32_t*)(wsm + L::kCapP);
+    const int32_t* sCapS = (const int32_t*)(wsm + L::kCapS);
+    const T* d_in = (const T*)a.d_in;
+    uint32_t* err = &a.s.ctr->err;
+    const int head = SEG ? a.head : 0;
+    auto seg_off = [&](int i) -> int64_t {
+        return a.offsets ? (int64_t)__ldg(&a.offsets[i]) : (i == 0 ? (int64_t)0 : (int64_t)(a.n - head));
+    };
+    auto seg_idx = [&](int pos) { return a.offsets ? seg_find(a.offsets, a.nseg, pos, err) : 0; };
+    auto tile_full = [&](int t) { return a.tma_rows > 0 && (t + 1) * RPT <= a.tma_rows && (t > 0 || head == 0); };
+    // a final answer v of position pos (phase 2); int64 answers: out_base + v, and
+    // UNRESOLVED64 for none (the key is left to the int64-position path); spans:
+    // pos - v
+    auto put = [&](int pos, int v) {
+        if constexpr (OUT64) a.d_out64[pos] = v >= 0 ? (int64_t)v + a.out_base : UNRESOLVED64;
+        else if constexpr (REV) a.d_out[a.n - 1 - pos] = v >= 0 ? a.n - 1 - v : -1;
+        else if constexpr (OUTM == OUT_SPAN) a.d_out[pos] = pos - v;
+        else a.d_out[pos] = v;
+    };
+    // the same for the four positions from pos on (a multiple of 4, in a tile that
+    // streams through TMA: 16-byte aligned), v >= 0
+    auto put4 = [&](int pos, int v) {
+        if constexpr (OUT64) {
+            const long long w = (long long)v + a.out_base;
+            longlong2* o = reinterpret_cast<longlong2*>(a.d_out64 + pos);
+            if (((uintptr_t)o & 15) == 0) {
+                o[0] = make_longlong2(w, w);
+                o[1] = make_longlong2(w, w);
+            } else {
+                for (int k = 0; k < 4; k++) a.d_out64[pos + k] = w;
+            }
+        } else if constexpr (REV) {
+            const int w = a.n - 1 - v;
+            *reinterpret_cast<int4*>(a.d_out + (a.n - 4 - pos)) = make_int4(w, w, w, w);
+        } else if constexpr (OUTM == OUT_SPAN) {
+            *reinterpret_cast<int4*>(a.d_out + pos) = make_int4(pos - v, pos + 1 - v, pos + 2 - v, pos + 3 - v);
+        } else {
+            *reinterpret_cast<int4*>(a.d_out + pos) = make_int4(v, v, v, v);
+        }
+    };
+
+    // ======================= phase 2: flagged keys ===============================
+    const int range_begin = t0 * WT;
+    T* sg = sV;  // the TMA ring is idle now: running minima of the earlier groups
+    int* staged = (int*)(wsm + L::kFlag);
+    if (lane == 0) *staged = 0;
+    __syncwarp();
+    T wpm = win;  // running minima of the window, from the nearest range on
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const T nb = __shfl_up_sync(FULL, wpm, o);
+        if (lane >= o) wpm = KeyTraits<T>::vmin(wpm, nb);
+    }
+
+    // A. deferred keys: the range's prefix minima, non-increasing, so the ones P
+    //    qualifies form a prefix of them and the rest keep -1.  Answers of
+    //    non-increasing queries only move left, so while the last answer's key
+    //    (the cursor) still qualifies it is the answer; else answer_before,
+    //    one key per lane.
+    bool a_done = !has_p;
+    int cur = -1;
+    T cv = KeyTraits<T>::pad();
+    // up to 32 deferred keys in order, one per lane (uniform call)
+    auto deferred32 = [&](const bool in, const T q, const int pos) {
+        const bool want = in && lt<INCL>(P, q);  // (segmented: all of the range's first segment)
+        if (__ballot_sync(FULL, want) != __ballot_sync(FULL, in)) a_done = true;
+        const bool ok = want && cur >= 0 && lt<INCL>(cv, q);
+        if (ok && (!head || pos >= head)) put(pos, SEG ? seg_rel(cur, first_start) : cur);
+        const bool rest = want && !ok;
+        const unsigned rm = __ballot_sync(FULL, rest);
+        if (!rm) return;
+        const int ans = answer_before<T, WT, INCL, MAPF, REV>(q, rest, r, wpm, sg, staged, d_in, a);
+        if (rest) {
+            if (ans < 0) atomicOr(err, ERR_INTERNAL);
+            else if (!head || pos >= head) put(pos, SEG ? seg_rel(ans, first_start) : ans);
+        }
+        cur = __shfl_sync(FULL, ans, 31 - __clz(rm));
+        if (cur < 0) {
+            a_done = true;
+        } else if (SEG && cur < first_start) {
+            a_done = true;  // before the segment: so are the answers of the lower keys (-1 already)
+        } else if (!a_done) {
+            cv = key_at<T, MAPF, REV>(d_in, a.n, cur);
+        }
+    };
+    const int nlist = min(def_total, kDefCap);
+    for (int b0 = 0; b0 < nlist && !a_done; b0 += 32) {
+        const int j = b0 + lane;
+        const bool in = j < nlist;
+        deferred32(in, in ? sDefV[j] : KeyTraits<T>::pad(), in ? sDefP[j] : 0);
+    }
+    // The flagged keys at or after `from` of tile t, 32 per step (uniform call).  A
+    // mixed tile's keys look in the earlier tiles of the range first (capped keys
+    // are answered there, deferred ones are not); with_deferred: keys without an
+    // answer there go to deferred32.
+    auto flagged_tile = [&](const int t, const bool mixed, const int from, const bool with_deferred) {
+        uint32_t mw = lane < W ? __ldcg(&a.s.tile_mask[(size_t)t * MW + lane]) : 0u;
+        if (lane < W) {
+            const int p0 = t * WT + 32 * lane, lim = max(from, head);
+            if (p0 < lim) mw &= lim - p0 >= 32 ? 0u : (0xffffffffu << (lim - p0));
+        }
+        int tot;
+        int off = warp_excl_sum(__popc(mw), tot);
+        __syncwarp();
+        while (mw) {
+            const int k = __ffs(mw) - 1;
+            mw &= mw - 1;
+            sList[off++] = (int16_t)(32 * lane + k);
+        }
+        __syncwarp();
+        for (int b0 = 0; b0 < tot; b0 += 32) {
+            bool in = b0 + lane < tot;
+            const int pos = t * WT + (in ? (int)sList[b0 + lane] : 0);
+            const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
+            if (mixed) {
+                const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, t, d_in, a);
+                if constexpr (SEG) {  // the keys' own segments, one after another
+                    for (unsigned m = __ballot_sync(FULL, in && found >= 0); m; m &= m - 1) {
+                        const int f = __ffs(m) - 1;
+                        const int sf = (int)seg_off(seg_idx(__shfl_sync(FULL, pos, f) - head)) + head;
+                        if (lane == f) put(pos, seg_rel(found, sf));
+                    }
+                } else if (in && found >= 0) {
+                    put(pos, found);
+                }
+                // (segmented: flagged keys without an answer in the range are of its first segment)
+                in = in && found < 0;
+            }
+            if (with_deferred && !a_done) deferred32(in, q, pos);
+        }
+        __syncwarp();
+    };
+    if (!a_done && def_total > kDefCap) {
+        // A'. the list overflowed and P qualified every listed key: continue over
+        //     the tile flags after the last listed key, 32 tiles per load.
+        const int from = sDefP[kDefCap - 1] + 1;
+        constexpr int TPL = 32 / W;  // tiles per load of mask words
+        const T* tile_min_r = (const T*)a.s.tile_min;
+        for (int tb = from / WT; tb < t1 && !a_done; tb += 32) {
+          const bool tin = tb + lane < t1;
+          const uint32_t tfl = tin ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
+          const T tmn = tin ? __ldcg(&tile_min_r[tb + lane]) : KeyTraits<T>::pad();
+          unsigned fl = __ballot_sync(FULL, (tfl & 0x7fffffffu) != 0);
+          while (fl && !a_done) {
+            // Flagged tiles whose pending keys all take the cursor: not mixed, and
+            // P and the cursor's key both qualify for the tile's minimum (<= every
+            // pending key).  Pending keys do not increase, so these form a prefix
+            // of the flagged tiles; their keys are not read.  A tile that is all
+            // pending takes the cursor in 16-byte stores without its masks; of
+            // the others the masks of 32/W tiles come in one load.
+            const unsigned fast = __ballot_sync(
+                FULL, ((fl >> lane) & 1u) && (tfl >> 31) == 0 && cur >= 0 && lt<INCL>(P, tmn) && lt<INCL>(cv, tmn));
+            const unsigned slow = fl & ~fast;
+            unsigned take = slow ? fl & ((slow & (0u - slow)) - 1u) : fl;
+            fl &= ~take;
+            unsigned whole = __ballot_sync(FULL, ((take >> lane) & 1u) && (tfl & 0x3fffffffu) == (uint32_t)WT &&
+                                                     (tb + lane) * WT >= from && tile_full(tb + lane));
+            take &= ~whole;
+            while (whole) {
+                const int t = tb + __ffs(whole) - 1;
+                whole &= whole - 1;
+#pragma unroll
+                for (int j = 0; j < WT / 128; j++) put4(t * WT + 128 * j + 4 * lane, SEG ? seg_rel(cur, first_start) : cur);
+            }
+            while (take) {
+                int tt[TPL], mine = -1;
+#pragma unroll
+                for (int h = 0; h < TPL; h++) {
+                    tt[h] = take ? __ffs(take) - 1 : -1;
+                    if (take) take &= take - 1;
+                    if (lane / W == h) mine = tt[h];
+                }
+                const uint32_t mw2 = mine >= 0 ? __ldcg(&a.s.tile_mask[(size_t)(tb + mine) * MW + (lane % W)]) : 0u;
+#pragma unroll
+                for (int h = 0; h < TPL; h++) {
+                    if (tt[h] < 0) break;
+#pragma unroll
+                    for (int w = 0; w < W; w++) {
+                        const uint32_t mw = __shfl_sync(FULL, mw2, W * h + w);
+                        const int pos = (tb + tt[h]) * WT + w * 32 + lane;
+                        if (((mw >> lane) & 1u) && pos >= from && (!head || pos >= head))
+                            put(pos, SEG ? seg_rel(cur, first_start) : cur);
+                    }
+                }
+            }
+            if (!fl) break;
+            // The first other flagged tile: alone when it is mixed or all pending, else
+            // with the tiles after it that are neither, up to a list of WT keys.
+            const int fsrc = __ffs(fl) - 1;
+            const int cnt = ((fl >> lane) & 1u) ? (int)(tfl & 0x3fffffffu) : 0;
+            const bool alone = cnt == WT || (cnt && (tfl >> 31));
+            int dummy;
+            const int before = warp_excl_sum(min(cnt, WT), dummy);
+            const unsigned stop = __ballot_sync(FULL, alone || before + cnt > WT);
+            unsigned tk = stop ? fl & ((stop & (0u - stop)) - 1u) : fl;
+            if ((stop >> fsrc) & 1u) {
+                fl &= fl - 1;
+                flagged_tile(tb + fsrc, (__shfl_sync(FULL, tfl, fsrc) >> 31) != 0, from, true);
+                continue;
+            }
+            fl &= ~tk;
+            int tot = 0;
+            while (tk) {  // lists the keys: 4 * TPL tiles' masks in flight
+                uint32_t mw[4];
+                int mt[4];
+#pragma unroll
+                for (int p2 = 0; p2 < 4; p2++) {
+                    mt[p2] = -1;
+#pragma unroll
+                    for (int h = 0; h < TPL; h++) {
+                        if (lane / W == h && tk) mt[p2] = __ffs(tk) - 1;
+                        tk &= tk - 1;
+                    }
+                    mw[p2] = mt[p2] >= 0 ? __ldcg(&a.s.tile_mask[(size_t)(tb + mt[p2]) * MW + (lane % W)]) : 0u;
+                }
+#pragma unroll
+                for (int p2 = 0; p2 < 4; p2++) {
+                    const int w0 = mt[p2] * WT + 32 * (lane % W);  // relative to tile tb
+                    const int lim = max(from, head) - tb * WT;
+                    if (w0 < lim) mw[p2] &= lim - w0 >= 32 ? 0u : (0xffffffffu << (lim - w0));
+                    int n2;
+                    int off = tot + warp_excl_sum(__popc(mw[p2]), n2);
+                    for (uint32_t m = mw[p2]; m; m &= m - 1) sList[off++] = (int16_t)(w0 + __ffs(m) - 1);
+                    tot += n2;
+                }
+            }
+            __syncwarp();
+            auto key_of = [&](const int j) {
+                return j < tot ? key_at<T, MAPF, REV>(d_in, a.n, tb * WT + (int)sList[j]) : KeyTraits<T>::pad();
+            };
+            T qn = key_of(lane);
+            for (int b0 = 0; b0 < tot && !a_done; b0 += 32) {
+                const T q = qn;
+                qn = key_of(b0 + 32 + lane);
+                const bool in = b0 + lane < tot;
+                deferred32(in, q, in ? tb * WT + (int)sList[b0 + lane] : 0);
+            }
+            __syncwarp();
+          }
+        }
+    }
+
+    // B. capped keys: the answer is in the range, below the stack's kept part.
+    const int ncap = min(cap_total, kCapCap);
+    for (int b0 = 0; b0 < ncap; b0 += 32) {
+        const bool in = b0 + lane < ncap;
+        const int pos = in ? sCapP[b0 + lane] : range_begin;
+        const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
+        const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, pos / WT, d_in, a);
+        if (in) {
+            if (found < 0) atomicOr(err, ERR_INTERNAL);
+            else if (!head || pos >= head) put(pos, SEG ? seg_rel(found, sCapS[b0 + lane]) : found);
+        }
+    }
+    if (cap_total > kCapCap) {
+        // B'. the capped list overflowed: every flagged key of the mixed tiles after it
+        const int from = sCapP[kCapCap - 1] + 1;
+        for (int tb = from / WT; tb < t1; tb += 32) {
+            const uint32_t tfl = tb + lane < t1 ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
+            for (unsigned fl = __ballot_sync(FULL, (tfl >> 31) != 0); fl; fl &= fl - 1)
+                flagged_tile(tb + __ffs(fl) - 1, true, from, false);
+        }
+    }
+}
+
 // MAPF: the key map (KMAP_*): keys pass through it as they enter shared memory
 // or registers -- float64 bit patterns in int64 slots compared through
 // f64_order, or the order-reversing flip for previous-greater queries.
@@ -633,37 +966,6 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     static_assert(OUTM == OUT_I32 || (!SEG && EP), "int64 and span answers: single arrays only");
     static_assert(!REV || (!SEG && EP && OUTM == OUT_I32 && KB == 4), "reversed runs: single arrays of 4-byte keys");
     constexpr bool OUT64 = OUTM == OUT_I64;
-    // a final answer v of position pos (phase 2); int64 answers: out_base + v, and
-    // UNRESOLVED64 for none (the key is left to the int64-position path); spans:
-    // pos - v
-    auto put = [&](int pos, int v) {
-        if constexpr (OUT64) a.d_out64[pos] = v >= 0 ? (int64_t)v + a.out_base : UNRESOLVED64;
-        else if constexpr (REV) a.d_out[a.n - 1 - pos] = v >= 0 ? a.n - 1 - v : -1;
-        else if constexpr (OUTM == OUT_SPAN) a.d_out[pos] = pos - v;
-        else a.d_out[pos] = v;
-    };
-    // the same for the four positions from pos on (a multiple of 4, in a tile that
-    // streams through TMA: 16-byte aligned), v >= 0
-    auto put4 = [&](int pos, int v) {
-        if constexpr (OUT64) {
-            const long long w = (long long)v + a.out_base;
-            longlong2* o = reinterpret_cast<longlong2*>(a.d_out64 + pos);
-            if (((uintptr_t)o & 15) == 0) {
-                o[0] = make_longlong2(w, w);
-                o[1] = make_longlong2(w, w);
-            } else {
-                for (int k = 0; k < 4; k++) a.d_out64[pos + k] = w;
-            }
-        } else if constexpr (REV) {
-            const int w = a.n - 1 - v;
-            *reinterpret_cast<int4*>(a.d_out + (a.n - 4 - pos)) = make_int4(w, w, w, w);
-        } else if constexpr (OUTM == OUT_SPAN) {
-            *reinterpret_cast<int4*>(a.d_out + pos) = make_int4(pos - v, pos + 1 - v, pos + 2 - v, pos + 3 - v);
-        } else {
-            *reinterpret_cast<int4*>(a.d_out + pos) = make_int4(v, v, v, v);
-        }
-    };
-
     // One claim per CTA: its warps take WPC consecutive range ids, in the order
     // the CTAs start (so every range a warp may wait on belongs to a started CTA).
     if (threadIdx.x == 0) {
@@ -1650,177 +1952,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         }
         __syncwarp();  // lane 0's acquire and wait before every lane's reads and writes
 
-        // ======================= phase 2: flagged keys ===============================
-        const int range_begin = t0 * WT;
-        T* sg = sV;  // the TMA ring is idle now: running minima of the earlier groups
-        bool staged = false;
-        T wpm = win;  // running minima of the window, from the nearest range on
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const T nb = __shfl_up_sync(FULL, wpm, o);
-            if (lane >= o) wpm = KeyTraits<T>::vmin(wpm, nb);
-        }
-
-        // A. deferred keys: the range's prefix minima, non-increasing, so the ones P
-        //    qualifies form a prefix of them and the rest keep -1.  Answers of
-        //    non-increasing queries only move left, so while the last answer's key
-        //    (the cursor) still qualifies it is the answer; else answer_before,
-        //    one key per lane.
-        bool a_done = !has_p;
-        int cur = -1;
-        T cv = KeyTraits<T>::pad();
-        // up to 32 deferred keys in order, one per lane (uniform call)
-        auto deferred32 = [&](const bool in, const T q, const int pos) {
-            const bool want = in && lt<INCL>(P, q);  // (segmented: all of the range's first segment)
-            if (__ballot_sync(FULL, want) != __ballot_sync(FULL, in)) a_done = true;
-            const bool ok = want && cur >= 0 && lt<INCL>(cv, q);
-            if (ok && (!head || pos >= head)) put(pos, SEG ? seg_rel(cur, first_start) : cur);
-            const bool rest = want && !ok;
-            const unsigned rm = __ballot_sync(FULL, rest);
-            if (!rm) return;
-            const int ans = answer_before<T, WT, INCL, MAPF, REV>(q, rest, r, wpm, sg, staged, d_in, a);
-            if (rest) {
-                if (ans < 0) atomicOr(err, ERR_INTERNAL);
-                else if (!head || pos >= head) put(pos, SEG ? seg_rel(ans, first_start) : ans);
-            }
-            cur = __shfl_sync(FULL, ans, 31 - __clz(rm));
-            if (cur < 0) {
-                a_done = true;
-            } else if (SEG && cur < first_start) {
-                a_done = true;  // before the segment: so are the answers of the lower keys (-1 already)
-            } else if (!a_done) {
-                cv = key_at<T, MAPF, REV>(d_in, a.n, cur);
-            }
-        };
-        const int nlist = min(def_total, kDefCap);
-        for (int b0 = 0; b0 < nlist && !a_done; b0 += 32) {
-            const int j = b0 + lane;
-            const bool in = j < nlist;
-            deferred32(in, in ? sDefV[j] : KeyTraits<T>::pad(), in ? sDefP[j] : 0);
-        }
-        // The flagged keys at or after `from` of tile t, 32 per step (uniform call).  A
-        // mixed tile's keys look in the earlier tiles of the range first (capped keys
-        // are answered there, deferred ones are not); with_deferred: keys without an
-        // answer there go to deferred32.
-        auto flagged_tile = [&](const int t, const bool mixed, const int from, const bool with_deferred) {
-            uint32_t mw = lane < W ? __ldcg(&a.s.tile_mask[(size_t)t * MW + lane]) : 0u;
-            if (lane < W) {
-                const int p0 = t * WT + 32 * lane, lim = max(from, head);
-                if (p0 < lim) mw &= lim - p0 >= 32 ? 0u : (0xffffffffu << (lim - p0));
-            }
-            int tot;
-            int off = warp_excl_sum(__popc(mw), tot);
-            __syncwarp();
-            while (mw) {
-                const int k = __ffs(mw) - 1;
-                mw &= mw - 1;
-                sList[off++] = (int16_t)(32 * lane + k);
-            }
-            __syncwarp();
-            for (int b0 = 0; b0 < tot; b0 += 32) {
-                bool in = b0 + lane < tot;
-                const int pos = t * WT + (in ? (int)sList[b0 + lane] : 0);
-                const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
-                if (mixed) {
-                    const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, t, d_in, a);
-                    if constexpr (SEG) {  // the keys' own segments, one after another
-                        for (unsigned m = __ballot_sync(FULL, in && found >= 0); m; m &= m - 1) {
-                            const int f = __ffs(m) - 1;
-                            const int sf = (int)seg_off(seg_idx(__shfl_sync(FULL, pos, f) - head)) + head;
-                            if (lane == f) put(pos, seg_rel(found, sf));
-                        }
-                    } else if (in && found >= 0) {
-                        put(pos, found);
-                    }
-                    // (segmented: flagged keys without an answer in the range are of its first segment)
-                    in = in && found < 0;
-                }
-                if (with_deferred && !a_done) deferred32(in, q, pos);
-            }
-            __syncwarp();
-        };
-        if (!a_done && def_total > kDefCap) {
-            // A'. the list overflowed and P qualified every listed key: continue over
-            //     the tile flags after the last listed key, 32 tiles per load.
-            const int from = sDefP[kDefCap - 1] + 1;
-            constexpr int TPL = 32 / W;  // tiles per load of mask words
-            const T* tile_min_r = (const T*)a.s.tile_min;
-            for (int tb = from / WT; tb < t1 && !a_done; tb += 32) {
-              const bool tin = tb + lane < t1;
-              const uint32_t tfl = tin ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
-              const T tmn = tin ? __ldcg(&tile_min_r[tb + lane]) : KeyTraits<T>::pad();
-              unsigned fl = __ballot_sync(FULL, (tfl & 0x7fffffffu) != 0);
-              while (fl && !a_done) {
-                // Flagged tiles whose pending keys all take the cursor: not mixed, and
-                // P and the cursor's key both qualify for the tile's minimum (<= every
-                // pending key).  Pending keys do not increase, so these form a prefix
-                // of the flagged tiles; their keys are not read.  A tile that is all
-                // pending takes the cursor in 16-byte stores without its masks; of
-                // the others the masks of 32/W tiles come in one load.
-                const unsigned fast = __ballot_sync(
-                    FULL, ((fl >> lane) & 1u) && (tfl >> 31) == 0 && cur >= 0 && lt<INCL>(P, tmn) && lt<INCL>(cv, tmn));
-                const unsigned slow = fl & ~fast;
-                unsigned take = slow ? fl & ((slow & (0u - slow)) - 1u) : fl;
-                fl &= ~take;
-                unsigned whole = __ballot_sync(FULL, ((take >> lane) & 1u) && (tfl & 0x3fffffffu) == (uint32_t)WT &&
-                                                         (tb + lane) * WT >= from && tile_full(tb + lane));
-                take &= ~whole;
-                while (whole) {
-                    const int t = tb + __ffs(whole) - 1;
-                    whole &= whole - 1;
-#pragma unroll
-                    for (int j = 0; j < WT / 128; j++) put4(t * WT + 128 * j + 4 * lane, SEG ? seg_rel(cur, first_start) : cur);
-                }
-                while (take) {
-                    int tt[TPL], mine = -1;
-#pragma unroll
-                    for (int h = 0; h < TPL; h++) {
-                        tt[h] = take ? __ffs(take) - 1 : -1;
-                        if (take) take &= take - 1;
-                        if (lane / W == h) mine = tt[h];
-                    }
-                    const uint32_t mw2 = mine >= 0 ? __ldcg(&a.s.tile_mask[(size_t)(tb + mine) * MW + (lane % W)]) : 0u;
-#pragma unroll
-                    for (int h = 0; h < TPL; h++) {
-                        if (tt[h] < 0) break;
-#pragma unroll
-                        for (int w = 0; w < W; w++) {
-                            const uint32_t mw = __shfl_sync(FULL, mw2, W * h + w);
-                            const int pos = (tb + tt[h]) * WT + w * 32 + lane;
-                            if (((mw >> lane) & 1u) && pos >= from && (!head || pos >= head))
-                                put(pos, SEG ? seg_rel(cur, first_start) : cur);
-                        }
-                    }
-                }
-                if (!fl) break;
-                const int fsrc = __ffs(fl) - 1;  // the first other flagged tile, key by key
-                fl &= fl - 1;
-                flagged_tile(tb + fsrc, (__shfl_sync(FULL, tfl, fsrc) >> 31) != 0, from, true);
-              }
-            }
-        }
-
-        // B. capped keys: the answer is in the range, below the stack's kept part.
-        const int ncap = min(cap_total, kCapCap);
-        for (int b0 = 0; b0 < ncap; b0 += 32) {
-            const bool in = b0 + lane < ncap;
-            const int pos = in ? sCapP[b0 + lane] : range_begin;
-            const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
-            const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, pos / WT, d_in, a);
-            if (in) {
-                if (found < 0) atomicOr(err, ERR_INTERNAL);
-                else if (!head || pos >= head) put(pos, SEG ? seg_rel(found, sCapS[b0 + lane]) : found);
-            }
-        }
-        if (cap_total > kCapCap) {
-            // B'. the capped list overflowed: every flagged key of the mixed tiles after it
-            const int from = sCapP[kCapCap - 1] + 1;
-            for (int tb = from / WT; tb < t1; tb += 32) {
-                const uint32_t tfl = tb + lane < t1 ? __ldcg(&a.s.tile_flag[tb + lane]) : 0u;
-                for (unsigned fl = __ballot_sync(FULL, (tfl >> 31) != 0); fl; fl &= fl - 1)
-                    flagged_tile(tb + __ffs(fl) - 1, true, from, false);
-            }
-        }
+        phase2<T, IPT, INCL, SEG, MAPF, OUTM, REV>(a, wsm, r, t0, t1, def_total, cap_total, first_start, P, has_p, win);
     }
 
     // ---- run bookkeeping: the last warp resets the control block --------------------------
