@@ -1070,6 +1070,10 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             // ---- 0. segmented runs: where segments start among the tile's keys ----------
             unsigned bword = 0;  // segment starts among this lane's keys (bit k: key k)
             int lane_s = 0;      // start of the segment holding this lane's first key
+            // No segment starts inside the tile (most tiles): its answers are made relative
+            // to the one start as they are found, with no pass over them before the store.
+            bool one_seg = false;
+            int rel = 0;  // that start (0 when answers are converted at the store)
             if constexpr (SEG) {
                 const int tile_end = tile_base + WT;
                 const int in_start = cur_start;
@@ -1102,6 +1106,8 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     lane_s = max(in_start, lane > 0 ? before_b : -1);
                 } else {
                     lane_s = in_start;
+                    one_seg = in_start <= tile_base;  // (not so in the view's first tile)
+                    rel = one_seg ? in_start : 0;
                 }
             }
             // start of the segment holding key k of this lane
@@ -1238,8 +1244,8 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         *po = o;
                     }
                 }
-                if constexpr (SEG) {  // answers relative to their segment's start
-                    __syncwarp();     // every lane's answers are in O
+                if (SEG && !one_seg) {  // answers relative to their segment's start
+                    __syncwarp();       // every lane's answers are in O
     #pragma unroll
                     for (int q4 = 0; q4 < IPT / 4; q4++) {
                         int4* po = reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]);
@@ -1532,6 +1538,22 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 const int dwin = max(stk_lo, stk_hi - 32);
                 const int wcnt = stk_hi - dwin;
                 const T dwv = dwin + lane < stk_hi ? sStkV[(dwin + lane) & (K - 1)] : KeyTraits<T>::pad();
+                const T first = __shfl_sync(FULL, v[0], 0), last = __shfl_sync(FULL, v[IPT - 1], 31);
+                const unsigned bl = __ballot_sync(FULL, lane < wcnt && lt<INCL>(dwv, last));
+                const unsigned bf = __ballot_sync(FULL, lane < wcnt && lt<INCL>(dwv, first));
+                int si;  // stack index of the current answer
+                if (bl == bf && (bl || !(has_rmin && lt<INCL>(rmin, first)))) {
+                    // the same window entry, or nothing in the range, answers every key (a tile
+                    // inside one descending run; with the loop below per key a batch of such runs took
+                    // 417 us instead of 314)
+                    si = bl ? dwin + 31 - __clz(bl) : stk_lo - 1;
+                    int rk = -1;
+                    if (bl) rk = one_seg ? seg_rel(sStkP[si & (K - 1)], rel) : sStkP[si & (K - 1)];
+                    else dm = IPT == 32 ? ~0u : (1u << IPT) - 1u;
+#pragma unroll
+                    for (int q4 = 0; q4 < IPT / 4; q4++)
+                        *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) = make_int4(rk, rk, rk, rk);
+                } else {
                 int lo = -1;  // topmost qualifying window entry for the lane's first key
 #pragma unroll
                 for (int s2 = 32; s2 > 0; s2 >>= 1) {
@@ -1539,7 +1561,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     const T wc = __shfl_sync(FULL, dwv, cand & 31);
                     if (cand < wcnt && lt<INCL>(wc, v[0])) lo = cand;
                 }
-                int si = lo >= 0 ? dwin + lo : stk_lo - 1;  // stack index of the current answer
+                si = lo >= 0 ? dwin + lo : stk_lo - 1;
                 if (lo < 0 && dwin > stk_lo) {  // below the window (values increase upwards)
                     int l2 = stk_lo, h2 = dwin;
                     while (l2 < h2) {
@@ -1562,12 +1584,13 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         while (si >= stk_lo && !lt<INCL>(sStkV[si & (K - 1)], vk)) si--;
                     int rk = -1;
                     if (si >= stk_lo) {
-                        rk = sStkP[si & (K - 1)];
+                        rk = one_seg ? seg_rel(sStkP[si & (K - 1)], rel) : sStkP[si & (K - 1)];
                     } else {
                         if (has_rmin && lt<INCL>(rmin, vk)) cm |= 1u << k;  // below the kept entries
                         else dm |= 1u << k;
                     }
                     O[swz(lane * IPT + k)] = rk;
+                }
                 }
                 if constexpr (SEG) {  // deferred keys outside the range's first segment are final (-1)
                     if (lb + IPT > first_end) dm &= lb >= first_end ? 0u : ((1u << (first_end - lb)) - 1u);
@@ -1591,25 +1614,26 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             unsigned umask = 0;  // keys without an in-thread answer: bit IPT - 1 - k for key k
             {
                 int res[IPT];  // absolute answers, -1 = none in the thread
+                const int lbo = lb - rel;
                 if (mono == FULL) {  // monotone lanes need no ladder
-                    res[0] = lane > 0 && b_adj ? lb - 1 : -1;
+                    res[0] = lane > 0 && b_adj ? lbo - 1 : -1;
 #pragma unroll
-                    for (int k = 1; k < IPT; k++) res[k] = adj ? lb + k - 1 : -1;
+                    for (int k = 1; k < IPT; k++) res[k] = adj ? lbo + k - 1 : -1;
                 } else {
 #pragma unroll
                     for (int k = 0; k < IPT; k++) {
-                        int rk = -1 - lb;  // relative to lb
+                        int rk = -1 - lbo;  // relative to lbo
 #pragma unroll
                         for (int j = k; j < 4; j++) take_if_lt<INCL>(rk, h[j], v[k], zero, j - 4);
 #pragma unroll
                         for (int j = 0; j < k; j++) take_if_lt<INCL>(rk, v[j], v[k], zero, j);
-                        res[k] = rk + lb;
+                        res[k] = rk + lbo;
                     }
                     if constexpr (INCL) {  // lane 0's pads qualify for keys of the pad's value
                         if (lane == 0)
 #pragma unroll
                             for (int k = 0; k < 4; k++)
-                                if (res[k] < lb) res[k] = -1;
+                                if (res[k] < lbo) res[k] = -1;
                     }
                 }
 #pragma unroll
@@ -1763,7 +1787,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
 #pragma unroll
                     for (int i2 = 0; i2 < NQ; i2++) {
                         const bool out = act[i2] && pl[i2] <= 0;
-                        if (act[i2] && !out) O[swz(e[i2])] = tile_base + pb[i2] + j[i2];
+                        if (act[i2] && !out) O[swz(e[i2])] = tile_base - rel + pb[i2] + j[i2];
                         const unsigned om = __ballot_sync(FULL, out);
                         if (out) sList[ns + __popc(om & ((1u << lane) - 1u))] = (int16_t)e[i2];
                         ns += __popc(om);
@@ -1813,7 +1837,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         }
                     }
                 }
-                if (act && ans >= 0) O[swz(e)] = ans;
+                if (act && ans >= 0) O[swz(e)] = SEG && one_seg ? seg_rel(ans, rel) : ans;
                 const bool miss = act && ans < 0;
                 if (__any_sync(FULL, miss)) {
                     const bool capd = miss && has_rmin && lt<INCL>(rmin, q);
@@ -1901,6 +1925,20 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 const int newtop = keep + (ptot >> 16);
                 int idx = keep + (ppre >> 16);
                 unsigned m = fmask;
+                // Mostly the tile's last keys, all of them (a ramp): copied in key order, one
+                // per lane, instead of up to IPT steps with every lane on its own keys.
+                const int tot = ptot >> 16;
+                if (tot >= 64) {
+                    const int k0 = WT - tot - lane * IPT;  // the lane's first key to push
+                    const unsigned all = (2u << (IPT - 1)) - 1u;
+                    if (__all_sync(FULL, fmask == (k0 <= 0 ? all : k0 >= IPT ? 0u : all & (all << k0)))) {
+                        for (int i2 = max(0, tot - K) + lane; i2 < tot; i2 += 32) {
+                            sStkV[(keep + i2) & (K - 1)] = V[ks(WT - tot + i2)];
+                            sStkP[(keep + i2) & (K - 1)] = tile_base + WT - tot + i2;
+                        }
+                        m = 0;
+                    }
+                }
                 if (idx + fcnt <= newtop - K) m = 0;  // all of this lane's entries drop at once
                 while (m) {
                     const int k = __ffs(m) - 1;

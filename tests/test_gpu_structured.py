@@ -21,6 +21,10 @@ def keys(shape: str, n: int, seed: int) -> np.ndarray:
         return np.cumsum(rng.integers(-1000, 801, n))
     if shape == "ramps":
         return i % 257
+    if shape == "falling_runs":  # descending runs of up to 4096 keys from random starts
+        ends = np.cumsum(rng.integers(1, 4097, n // 1024 + 2))
+        run = np.searchsorted(ends, i, side="right")
+        return rng.integers(4096, 1 << 30, ends.size + 1)[run] - (i - np.concatenate([[0], ends])[run])
     if shape == "noisy_down":
         return 8 * (n - i) + rng.integers(0, 64, n)
     x = i.copy() if shape == "up_few" else n - 1 - i
@@ -29,7 +33,7 @@ def keys(shape: str, n: int, seed: int) -> np.ndarray:
     return x
 
 
-SHAPES = ("walk", "walk_down", "ramps", "noisy_down", "down_few", "up_few")
+SHAPES = ("walk", "walk_down", "ramps", "falling_runs", "noisy_down", "down_few", "up_few")
 
 
 def ranked(a: np.ndarray) -> np.ndarray:
@@ -73,7 +77,7 @@ def test_every_configuration(shape):
 def test_batch(dtype, le):
     from apsep_gb300 import Plan
     rng = np.random.default_rng(11)
-    lens = [1, 3, 700, 33, 200_000, 0, 5, 41_003, 512, 300_000, 31, 90_001, 123_456]
+    lens = [1, 3, 700, 33, 200_000, 0, 5, 41_003, 512, 300_000, 31, 90_001, 123_456, 64, 150_000, 77, 99_999]
     parts = [keys(SHAPES[k % len(SHAPES)], m, k) if m else np.zeros(0, np.int64) for k, m in enumerate(lens)]
     a = np.concatenate(parts) + rng.integers(0, 2)
     offs = np.concatenate([[0], np.cumsum(lens)]).astype(np.int64)
