@@ -93,7 +93,6 @@ struct WLayout {
     static constexpr size_t kBytes = (kEnd + 1023) / 1024 * 1024;     // keeps every warp 1024-aligned
     static_assert(kO % 1024 == 0 && kSM % 1024 == 0 && (WT * KB) % 1024 == 0,
                   "swizzled buffers need 1024-byte alignment");
-    static_assert(kList - kV >= (size_t)KB * (kMaxRanges / 32 + 8 * 32) + 4 * 8 * 32, "room for phase 2's staging");
     static_assert(kStkV % 8 == 0 && kDefV % 8 == 0, "8-byte keys need 8-byte aligned arrays");
 };
 
@@ -230,9 +229,10 @@ __device__ __forceinline__ int last_of(int lo, int hi, T q, Load load) {
 
 // Search inside one range: each lane with `need` finds the rightmost key that
 // qualifies for its q in its tiles [lo, hi) -- the nearest tile by tile minima,
-// its chunk, its key.  -2 when no tile's minimum qualifies.
+// its chunk, its key.  -2 when no tile's minimum qualifies; exact = false: some
+// tile's minimum is known to qualify.
 template <typename T, int B, bool INCL, int MAPF = KMAP_NONE, bool REV = false>
-__device__ __noinline__ int find_in_tiles(T q, bool need, int lo, int hi, const T* __restrict__ d_in,
+__device__ __noinline__ int find_in_tiles(T q, bool need, int lo, int hi, bool exact, const T* __restrict__ d_in,
                                           const RangeArgs& a) {
     constexpr int W = B / 32;
     const T* tile_min = (const T*)a.s.tile_min;
@@ -256,7 +256,7 @@ __device__ __noinline__ int find_in_tiles(T q, bool need, int lo, int hi, const 
         }
         return p;
     }
-    int s = -1;
+    int s = hi - lo == 1 && !exact ? lo : -1;  // (a range of one tile whose minimum is known to qualify)
     for (int t = hi - 1; need && s < 0 && t >= lo; t -= 16) {
         T m[16];
 #pragma unroll
@@ -303,15 +303,19 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
     constexpr int KB = (int)sizeof(T);
     const int lane = threadIdx.x & 31;
     int rp = -1;
-    const unsigned wm = __ballot_sync(FULL, want);
-    if (__popc(wm) <= kFew) {
-        int ans = -2;
-        bool miss = false;
-        for (unsigned m = wm; m; m &= m - 1) {
-            const int f = __ffs(m) - 1;
+    {
+        int lo = -1;  // the nearest lo + 1 ranges do not qualify
+#pragma unroll 1
+        for (int s = 16; s > 0; s >>= 1)
+            if (!lt<INCL>(__shfl_sync(FULL, wpm, lo + s), q)) lo += s;
+        if (lt<INCL>(__shfl_sync(FULL, wpm, lo + 1), q)) rp = max(r - 2 - lo, -1);
+    }
+    unsigned far = __ballot_sync(FULL, want && rp < 0);  // answers before the window
+    if (__popc(far) <= kFew) {
+        for (; far; far &= far - 1) {
+            const int f = __ffs(far) - 1;
             const T qf = __shfl_sync(FULL, q, f);
-            const unsigned w = __ballot_sync(FULL, lt<INCL>(wpm, qf));
-            int rf = w ? r - __ffs(w) : -1;
+            int rf = -1;
             if constexpr (KB == 8) {  // no group words: the range minima, 8 groups a step
                 for (int hi = r - 33; hi >= 0 && rf < 0; hi -= 256) {
                     T u[8];
@@ -324,41 +328,14 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
                     }
                 }
             } else {
-                int g = rf >= 0 || r < 33 ? -1 : (r - 33) >> 5, gf = -1;
-                for (; g >= 0 && gf < 0; g -= 32)
+                int gf = -1;
+                for (int g = r < 33 ? -1 : (r - 33) >> 5; g >= 0 && gf < 0; g -= 32)
                     gf = last_of<T, INCL>(max(g - 31, 0), g, qf, [&](int i) { return group_min_of<T>(a, i); });
                 if (gf >= 0) rf = last_of<T, INCL>(32 * gf, 32 * gf + 31, qf, [&](int i) { return range_min<T>(a, i); });
             }
-            int af = -2;
-            if (rf >= 0) {  // the range's published stack top
-                const int cnt = (int)(__ldcg(&a.s.top_cnt[rf]) & 0xffu);
-                const T tk = __ldcg((const T*)a.s.top_key + (size_t)rf * kTopEntries + lane);
-                const int tp = __ldcg(&a.s.top_pos[(size_t)rf * kTopEntries + lane]);
-                const unsigned b = __ballot_sync(FULL, lane < cnt && lt<INCL>(tk, qf));
-                if (b) af = __shfl_sync(FULL, tp, 31 - __clz(b));
-            }
-            if (lane == f) {
-                ans = af;
-                rp = rf;
-                miss = rf >= 0 && af == -2;
-            }
+            if (lane == f) rp = rf;
         }
-        if (__any_sync(FULL, miss)) {
-            const int lo = max(rp, 0) * a.tiles_per_range;
-            const int found =
-                find_in_tiles<T, B, INCL, MAPF, REV>(q, miss, lo, min(lo + a.tiles_per_range, a.num_tiles), d_in, a);
-            if (miss) ans = found;
-        }
-        return ans;
-    }
-    {
-        int lo = -1;  // the nearest lo + 1 ranges do not qualify
-#pragma unroll 1
-        for (int s = 16; s > 0; s >>= 1)
-            if (!lt<INCL>(__shfl_sync(FULL, wpm, lo + s), q)) lo += s;
-        if (lt<INCL>(__shfl_sync(FULL, wpm, lo + 1), q)) rp = max(r - 2 - lo, -1);
-    }
-    if (__any_sync(FULL, want && rp < 0)) {
+    } else {
         const int ng = r >= 33 ? ((r - 33) >> 5) + 1 : 0;  // groups of earlier ranges (the window's part does not qualify)
         static_assert(kMaxRanges / 32 == 128, "four groups per lane");
         if (!*staged) {
@@ -414,36 +391,39 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
         }
     }
     // The published stack tops of the ranges that lanes ask for, up to kSlots of them
-    // copied to shared memory at a time (all copies in flight together), then searched
-    // by the lanes side by side: entries increase from the bottom, so the qualifying
-    // ones form a bottom part and the topmost of them answers.
-    constexpr int kSlots = 8;
+    // copied to shared memory at a time, each by the first lane that asks for it (all
+    // copies in flight together), then searched by the lanes side by side: entries
+    // increase from the bottom, so the qualifying ones form a bottom part and the
+    // topmost of them answers.
+    using L = WLayout<B / 32, KB>;
+    constexpr int kRoom = (int)((L::kList - L::kV - KB * (kMaxRanges / 32)) / (32 * (KB + 4)));
+    constexpr int kSlots = kRoom < 16 ? kRoom : 16;
+    static_assert(kSlots >= 8, "room for phase 2's staging");
+    static_assert(kTopEntries == 32, "a lane copies 2 KB + 8 times 16 bytes");
     T* sk = sg + kMaxRanges / 32;               // T[kSlots][32]
     int32_t* sp = (int32_t*)(sk + kSlots * 32);  // int32[kSlots][32]
     int ans = -2;
     const int rq = want ? rp : -1;
-    unsigned todo = __ballot_sync(FULL, rq >= 0);
-    while (todo) {
-        int slot = -1, cnt = 0, ns = 0;
+    const int first = __ffs(__match_any_sync(FULL, rq)) - 1;  // the first lane with this lane's range
+    const unsigned firsts = __ballot_sync(FULL, rq >= 0 && first == lane);
+    const int nth = __popc(firsts & ((1u << first) - 1u));
+    for (int s0 = 0; s0 < __popc(firsts); s0 += kSlots) {
+        const int slot = rq >= 0 ? nth - s0 : -1;
+        int cnt = 0;
         __syncwarp();
-#pragma unroll 1
-        for (; todo && ns < kSlots; ns++) {
-            const int rc = __shfl_sync(FULL, rq, __ffs(todo) - 1);
-            const unsigned same = __ballot_sync(FULL, rq == rc);
-            todo &= ~same;
-            if (rq == rc) slot = ns;
-            if (lane == ns) cnt = (int)(__ldcg(&a.s.top_cnt[rc]) & 0xffu);
-            static_assert(kTopEntries == 32, "2 KB lanes copy the keys of a stack top, 8 its positions");
-            if (lane < 2 * KB)
-                copy_async16((char*)(sk + ns * 32) + 16 * lane,
-                             (const char*)((const T*)a.s.top_key + (size_t)rc * kTopEntries) + 16 * lane);
-            else if (lane < 2 * KB + 8)
-                copy_async16(sp + ns * 32 + 4 * (lane - 2 * KB), a.s.top_pos + (size_t)rc * kTopEntries + 4 * (lane - 2 * KB));
+        if (slot >= 0 && slot < kSlots && first == lane) {
+            cnt = (int)(__ldcg(&a.s.top_cnt[rq]) & 0xffu);
+            const char* tk = (const char*)((const T*)a.s.top_key + (size_t)rq * kTopEntries);
+            const char* tp = (const char*)(a.s.top_pos + (size_t)rq * kTopEntries);
+#pragma unroll
+            for (int k = 0; k < 2 * KB; k++) copy_async16((char*)(sk + slot * 32) + 16 * k, tk + 16 * k);
+#pragma unroll
+            for (int k = 0; k < 8; k++) copy_async16((char*)(sp + slot * 32) + 16 * k, tp + 16 * k);
         }
         copy_async_wait();
         __syncwarp();
-        cnt = __shfl_sync(FULL, cnt, slot & 31);
-        if (slot >= 0) {
+        cnt = __shfl_sync(FULL, cnt, first);
+        if (slot >= 0 && slot < kSlots) {
             int lo = -1;
 #pragma unroll 1
             for (int s = 32; s > 0; s >>= 1)
@@ -455,7 +435,7 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
     if (__any_sync(FULL, miss)) {
         const int lo = max(rp, 0) * a.tiles_per_range;
         const int found =
-            find_in_tiles<T, B, INCL, MAPF, REV>(q, miss, lo, min(lo + a.tiles_per_range, a.num_tiles), d_in, a);
+            find_in_tiles<T, B, INCL, MAPF, REV>(q, miss, lo, min(lo + a.tiles_per_range, a.num_tiles), false, d_in, a);
         if (miss) ans = found;
     }
     return ans;
@@ -741,7 +721,7 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
             const int pos = t * WT + (in ? (int)sList[b0 + lane] : 0);
             const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
             if (mixed) {
-                const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, t, d_in, a);
+                const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, t, true, d_in, a);
                 if constexpr (SEG) {  // the keys' own segments, one after another
                     for (unsigned m = __ballot_sync(FULL, in && found >= 0); m; m &= m - 1) {
                         const int f = __ffs(m) - 1;
@@ -874,7 +854,7 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
         const bool in = b0 + lane < ncap;
         const int pos = in ? sCapP[b0 + lane] : range_begin;
         const T q = in ? key_at<T, MAPF, REV>(d_in, a.n, pos) : KeyTraits<T>::pad();
-        const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, pos / WT, d_in, a);
+        const int found = find_in_tiles<T, WT, INCL, MAPF, REV>(q, in, t0, pos / WT, true, d_in, a);
         if (in) {
             if (found < 0) atomicOr(err, ERR_INTERNAL);
             else if (!head || pos >= head) put(pos, SEG ? seg_rel(found, sCapS[b0 + lane]) : found);
