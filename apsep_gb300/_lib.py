@@ -6,6 +6,7 @@ point.  If the library is missing, build it with
 """
 from __future__ import annotations
 
+import array
 import ctypes
 import os
 import threading
@@ -106,7 +107,6 @@ def copy_spans(srcs, dsts, nbytes, stream_handle: int) -> None:
     n = len(srcs)
     if n == 0:
         return
-    a = (ctypes.c_void_p * n)(*srcs)
-    b = (ctypes.c_void_p * n)(*dsts)
-    c = (ctypes.c_int64 * n)(*nbytes)
-    check(load().apsep_copy_spans(a, b, c, n, ctypes.c_void_p(stream_handle)), "apsep_copy_spans")
+    a, b, c = array.array("Q", srcs), array.array("Q", dsts), array.array("q", nbytes)
+    check(load().apsep_copy_spans(a.buffer_info()[0], b.buffer_info()[0], c.buffer_info()[0], n,
+                                  ctypes.c_void_p(stream_handle)), "apsep_copy_spans")

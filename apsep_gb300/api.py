@@ -27,9 +27,18 @@ _DTYPES = {torch.int32: _lib.INT32, torch.float32: _lib.FLOAT32, torch.int64: _l
 _WIDE = (torch.int64, torch.float64)  # 8-byte keys: single arrays, one configuration
 
 
+# The current stream's handle without building a Stream object (2 us a call on
+# the GPU host, as much as a short array's launch); the public call where this
+# PyTorch has no such function.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def _stream_handle(device: torch.device, stream=None) -> int:
-    s = stream if stream is not None else torch.cuda.current_stream(device)
-    return int(s.cuda_stream)
+    if stream is not None:
+        return int(stream.cuda_stream)
+    if _raw_stream is not None and device.index is not None:
+        return _raw_stream(device.index)
+    return int(torch.cuda.current_stream(device).cuda_stream)
 
 
 class Plan:
@@ -56,6 +65,7 @@ class Plan:
             from . import autotune
             tuning = autotune.load()
         self._tuning = tuning
+        self._cfg_of = {}  # the table's configuration per size class (n.bit_length()), as they come up
         with torch.cuda.device(self.device):
             _lib.check(self._lib.apsep_plan_create(ctypes.byref(self._h), _DTYPES[dtype],
                                                    _lib.LE if inclusive else _lib.LT, self.capacity),
@@ -80,7 +90,10 @@ class Plan:
     def _tune_for(self, n: int) -> None:
         if self._tuning is None:
             return
-        cfg = self._tuning.config_for(n, self.dtype)
+        b = n.bit_length()
+        if b not in self._cfg_of:
+            self._cfg_of[b] = self._tuning.config_for(n, self.dtype)
+        cfg = self._cfg_of[b]
         if cfg is not None and cfg != self._cfg:
             _lib.check(self._lib.apsep_plan_set_config(self._h, int(cfg)), "apsep_plan_set_config")
             self._cfg = cfg
@@ -90,19 +103,20 @@ class Plan:
         """Enqueue out[:n] = APSE(x[:n]) on the current (or given) stream."""
         if not x.is_cuda or x.dtype != self.dtype or not x.is_contiguous():
             raise ValueError("x must be a contiguous CUDA %s tensor" % self.dtype)
-        n = x.numel() if n is None else int(n)
+        total = x.numel()
+        n = total if n is None else int(n)
         if out is None:
             out = torch.empty(max(n, 0), dtype=torch.int32, device=x.device)
         if out.dtype != torch.int32 or not out.is_cuda or not out.is_contiguous():
             raise ValueError("out must be a contiguous CUDA int32 tensor")
-        if n > x.numel() or n > out.numel():
+        if n > total or n > out.numel():
             raise ValueError("n exceeds the buffers")
         incl = self.inclusive if inclusive is None else bool(inclusive)
         self._tune_for(n)
-        st = self._lib.apsep_run_cmp(self._h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-                                     n, _lib.LE if incl else _lib.LT,
-                                     ctypes.c_void_p(_stream_handle(x.device, stream)))
-        _lib.check(st, "apsep_run")
+        st = self._lib.apsep_run_cmp(self._h, x.data_ptr(), out.data_ptr(), n, _lib.LE if incl else _lib.LT,
+                                     _stream_handle(x.device, stream))
+        if st:
+            _lib.check(st, "apsep_run")
         return out
 
     def run_segmented(self, x: torch.Tensor, offsets: torch.Tensor, out: torch.Tensor | None = None,
@@ -121,10 +135,10 @@ class Plan:
         if out.dtype != torch.int32 or not out.is_cuda or not out.is_contiguous() or out.numel() < n:
             raise ValueError("out must be a contiguous CUDA int32 tensor of x.numel() entries")
         self._tune_for(n)
-        st = self._lib.apsep_run_segmented(self._h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-                                           n, ctypes.c_void_p(offsets.data_ptr()), offsets.numel() - 1,
-                                           ctypes.c_void_p(_stream_handle(x.device, stream)))
-        _lib.check(st, "apsep_run_segmented")
+        st = self._lib.apsep_run_segmented(self._h, x.data_ptr(), out.data_ptr(), n, offsets.data_ptr(),
+                                           offsets.numel() - 1, _stream_handle(x.device, stream))
+        if st:
+            _lib.check(st, "apsep_run_segmented")
         return out
 
     def workspace64_bytes(self, n: int) -> int:

@@ -124,22 +124,23 @@ class RingPool:
         size = self.span_size(n)
         if size > self.capacity:
             return None
+        head = self.head
         if not self._spans:
             start = 0
         else:
             tail = self._spans[0][0]
-            if self.head == tail:  # head caught up with the tail: full
+            if head == tail:  # head caught up with the tail: full
                 return None
-            if self.head > tail:  # free: [head, capacity) and [0, tail)
-                if self.head + size <= self.capacity:
-                    start = self.head
+            if head > tail:  # free: [head, capacity) and [0, tail)
+                if head + size <= self.capacity:
+                    start = head
                 elif size <= tail:
                     start = 0
                 else:
                     return None
             else:  # wrapped; free: [head, tail)
-                if self.head + size <= tail:
-                    start = self.head
+                if head + size <= tail:
+                    start = head
                 else:
                     return None
         e = [start, size, False]
@@ -165,6 +166,7 @@ class _Lane:
         self.event = torch.cuda.Event()
         self.offs = torch.empty(max_segments + 1, dtype=torch.int64, device=device)
         self.offs_host = torch.empty(max_segments + 1, dtype=torch.int64).pin_memory()
+        self.offs_np = self.offs_host.numpy()  # the same memory
         self.err_host = torch.zeros(1, dtype=torch.int32).pin_memory()
         self.batch: list = []
 
@@ -264,21 +266,23 @@ class PoolServer:
         ln.batch = batch
         ln.stream.wait_event(copied)
         with torch.cuda.stream(ln.stream):
-            ln.offs_host[:ns + 1] = torch.tensor(offs, dtype=torch.int64)
-            ln.offs[:ns + 1].copy_(ln.offs_host[:ns + 1], non_blocking=True)
-            ln.plan.run_segmented(keys_ring[base:base + total], ln.offs[:ns + 1],
-                                  out=ans_ring[base:base + total], stream=ln.stream)
+            ln.offs_np[:ns + 1] = offs
+            d_offs = ln.offs[:ns + 1]
+            d_offs.copy_(ln.offs_host[:ns + 1], non_blocking=True)
+            ln.plan.run_segmented(keys_ring[base:base + total], d_offs, out=ans_ring[base:base + total],
+                                  stream=ln.stream)
             srcs, dsts, nb = [], [], []
             a0 = ans_ring.data_ptr()
             for r in batch:
-                if r.out is None or r.n == 0:
+                n = r._n
+                if r.out is None or n == 0:
                     continue
-                if r.out.is_cuda:  # device answers: one gathered copy for the batch
+                if r._out_ptr is not None:  # device answers: one gathered copy for the batch
                     srcs.append(a0 + 4 * r.slot)
-                    dsts.append(r.out.data_ptr())
-                    nb.append(4 * r.n)
+                    dsts.append(r._out_ptr)
+                    nb.append(4 * n)
                 else:
-                    r.out[:r.n].copy_(ans_ring[r.slot:r.slot + r.n], non_blocking=True)
+                    r.out[:n].copy_(ans_ring[r.slot:r.slot + n], non_blocking=True)
             _lib.copy_spans(srcs, dsts, nb, ln.stream.cuda_stream)
         self._finish_launch(ln)
 
@@ -291,13 +295,14 @@ class PoolServer:
             for r in ln.batch:
                 r.failed = True
         ans_ring = self.rings[kind][1]
+        free = self._pools[kind].free
         for r in ln.batch:
             r.t_done = now
             if on_done is not None:
                 # the answers in the pool (or r.out), valid during the call
                 on_done(r, ans_ring[r.slot:r.slot + r.n] if r.slot is not None else r.out[:r.n])
             if r.slot is not None:
-                self._pools[kind].free(r.slot)
+                free(r.slot)
         ln.batch = []
 
     def _admit_chunk(self, k, waiting, admitted, ahead) -> bool:
@@ -383,29 +388,35 @@ class PoolServer:
         called when it completes, with a device view that stays valid only
         during the call (its pool span is released right after);
         keep_answers gives such requests a pinned host out instead."""
-        for r in requests:
-            if r.kind not in self.lanes:
-                raise ValueError("no pool for keys of %s (inclusive=%s)" % r.kind)
-            if r.n > min(self.max_batch_keys, self.ring_keys) and not self._direct(r):
-                raise ValueError("request %d (%d keys) exceeds a batch (%d keys)" % (r.rid, r.n,
-                                 min(self.max_batch_keys, self.ring_keys)))
-            if not r.keys.is_contiguous() or (r.out is not None and (not r.out.is_contiguous()
-                                                                   or r.out.dtype != torch.int32
-                                                                   or r.out.numel() < r.n)):
+        pools = {k: RingPool(self.ring_keys) for k in self.kinds}
+        limit = min(self.max_batch_keys, self.ring_keys)
+        never_direct = self.direct_min_keys is None
+        for r in requests:  # what the loop below needs of a request is looked up once, here
+            keys, out = r.keys, r.out
+            n = keys.numel()
+            kind = (keys.dtype, bool(r.inclusive))
+            if kind not in self.lanes:
+                raise ValueError("no pool for keys of %s (inclusive=%s)" % kind)
+            direct = False if never_direct else self._direct(r)
+            if n > limit and not direct:
+                raise ValueError("request %d (%d keys) exceeds a batch (%d keys)" % (r.rid, n, limit))
+            if not keys.is_contiguous() or (out is not None and (not out.is_contiguous() or out.dtype != torch.int32
+                                                                 or out.numel() < n)):
                 raise ValueError("request %d: keys and out must be contiguous, out int32 of n entries" % r.rid)
-            if keep_answers and r.out is None:
-                r.out = torch.empty(r.n, dtype=torch.int32).pin_memory()
+            if keep_answers and out is None:
+                r.out = out = torch.empty(n, dtype=torch.int32).pin_memory()
+                direct = False if never_direct else self._direct(r)
             r.failed = False
             r.slot = None
             r.t_done = None
-        self._pools = {k: RingPool(self.ring_keys) for k in self.kinds}
-        for r in requests:  # looked up once: the loop below runs per request
-            r._n = r.n
-            r._kind = r.kind
-            r._span = self._pools[r._kind].span_size(r._n)
-            r._dev = r.keys.is_cuda
-            r._ptr = r.keys.data_ptr()
-            r._direct = self._direct(r)
+            r._n = n
+            r._kind = kind
+            r._span = pools[kind].span_size(n)
+            r._dev = keys.is_cuda
+            r._ptr = keys.data_ptr()
+            r._out_ptr = out.data_ptr() if out is not None and out.is_cuda else None
+            r._direct = direct
+        self._pools = pools
         order = sorted(requests, key=lambda r: r.arrival if realtime else 0.0)
         waiting = {k: collections.deque() for k in self.kinds}
         admitted = {k: collections.deque() for k in self.kinds}  # in the ring, not yet launched
@@ -444,7 +455,7 @@ class PoolServer:
             for r in order:
                 r.answers = r.out[:r.n].cpu().numpy() if r.out.is_cuda else r.out[:r.n].numpy().copy()
         lat = [1e3 * (r.t_done - (r.arrival if realtime else 0.0)) for r in order]
-        return ServeStats(len(order), sum(r.n for r in order), t_end, lat, self._nbatches, self.device_bytes)
+        return ServeStats(len(order), sum(r._n for r in order), t_end, lat, self._nbatches, self.device_bytes)
 
 
 def device_loop(requests: list, realtime: bool = True, device=None) -> ServeStats:
