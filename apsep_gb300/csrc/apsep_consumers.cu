@@ -72,12 +72,14 @@ Work carve(void* d_work, int64_t n, int dtype) {
 
 template <typename T>
 __global__ void flip_keys(const T* __restrict__ in, T* __restrict__ out, int64_t n) {
+    apsep::grid_dependency_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = flip(in[i]);
 }
 
 template <typename T>
 __global__ void reverse_keys(const T* __restrict__ in, T* __restrict__ out, int64_t n) {
+    apsep::grid_dependency_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = in[n - 1 - i];
 }
@@ -94,11 +96,13 @@ __device__ __forceinline__ int64_t next_of(const int32_t* __restrict__ R, bool d
 }
 
 __global__ void mirror_answers(const int32_t* __restrict__ ar, int32_t* __restrict__ out, int64_t n) {
+    apsep::grid_dependency_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         out[i] = (int32_t)next_from_reversed(ar, n, i);
 }
 
 __global__ void span_from_previous(int32_t* __restrict__ a, int64_t n) {
+    apsep::grid_dependency_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         a[i] = (int32_t)(i - a[i]);
 }
@@ -109,6 +113,7 @@ __global__ void span_from_previous(int32_t* __restrict__ a, int64_t n) {
 __global__ void rect_area(const int32_t* __restrict__ h, const int32_t* __restrict__ L,
                           const int32_t* __restrict__ ar, bool direct, int64_t n, unsigned long long* __restrict__ best) {
     __shared__ long long warp_best[kThreads / 32];
+    apsep::grid_dependency_wait();
     long long m = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = next_of(ar, direct, n, i);
@@ -136,6 +141,7 @@ __global__ void rect_area(const int32_t* __restrict__ h, const int32_t* __restri
 template <typename T>
 __global__ void cartesian_parent(const T* __restrict__ a, const int32_t* __restrict__ L,
                                  const int32_t* __restrict__ ar, bool direct, int32_t* __restrict__ out, int64_t n) {
+    apsep::grid_dependency_wait();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t l = L[i], r = next_of(ar, direct, n, i);
         int64_t p;
@@ -168,7 +174,11 @@ apsep_status check_args(apsep_plan* plan, const void* d_in, const void* d_out, s
     return APSEP_OK;
 }
 
-apsep_status launched() { return cudaGetLastError() == cudaSuccess ? APSEP_OK : APSEP_ECUDA; }
+// Launches a grid-stride kernel over n elements.
+template <typename K, typename... A>
+apsep_status launched(K kernel, int64_t n, cudaStream_t st, const A&... args) {
+    return apsep::launch_pdl(kernel, grid_for(n), kThreads, 0, st, args...) == cudaSuccess ? APSEP_OK : APSEP_ECUDA;
+}
 
 }  // namespace
 
@@ -190,9 +200,9 @@ apsep_status apsep_run_prev_greater(apsep_plan* plan, const void* d_in, int32_t*
     const cudaStream_t st = (cudaStream_t)stream;
     for_key_type(dtype, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        flip_keys<T><<<grid_for(n), kThreads, 0, st>>>((const T*)d_in, (T*)d_work, n);
+        s = launched(flip_keys<T>, n, st, (const T*)d_in, (T*)d_work, n);
     });
-    if ((s = launched()) != APSEP_OK) return s;
+    if (s != APSEP_OK) return s;
     return apsep_run_cmp(plan, d_work, d_out, n, cmp, stream);
 }
 
@@ -208,12 +218,12 @@ apsep_status apsep_run_next_smaller(apsep_plan* plan, const void* d_in, int32_t*
     const Work w = carve(d_work, n, dtype);
     for_key_type(dtype, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        reverse_keys<T><<<grid_for(n), kThreads, 0, st>>>((const T*)d_in, (T*)w.keys, n);
+        s = launched(reverse_keys<T>, n, st, (const T*)d_in, (T*)w.keys, n);
     });
-    if ((s = launched()) != APSEP_OK) return s;
+    if (s != APSEP_OK) return s;
     if ((s = apsep_run_cmp(plan, w.keys, w.a, n, cmp, stream)) != APSEP_OK) return s;
-    mirror_answers<<<grid_for(n), kThreads, 0, st>>>(w.a, d_out, n);
-    return launched();
+    s = launched(mirror_answers, n, st, w.a, d_out, n);
+    return s;
 }
 
 apsep_status apsep_stock_span(apsep_plan* plan, const void* d_in, int32_t* d_out, int64_t n, void* d_work,
@@ -226,8 +236,8 @@ apsep_status apsep_stock_span(apsep_plan* plan, const void* d_in, int32_t* d_out
     if ((s = plan_run_flipped(plan, d_in, d_out, n, APSEP_LT, 1, stream)) != APSEP_ENOTSUP) return s;
     s = apsep_run_prev_greater(plan, d_in, d_out, n, APSEP_LT, d_work, stream);
     if (s != APSEP_OK || n == 0) return s;
-    span_from_previous<<<grid_for(n), kThreads, 0, (cudaStream_t)stream>>>(d_out, n);
-    return launched();
+    s = launched(span_from_previous, n, (cudaStream_t)stream, d_out, n);
+    return s;
 }
 
 apsep_status apsep_largest_rectangle(apsep_plan* plan, const int32_t* d_heights, int64_t n, int64_t* d_area,
@@ -247,13 +257,13 @@ apsep_status apsep_largest_rectangle(apsep_plan* plan, const int32_t* d_heights,
     bool direct = true;
     if ((s = plan_run_reversed(plan, d_heights, w.a, n, APSEP_LT, stream)) == APSEP_ENOTSUP) {
         direct = false;
-        reverse_keys<int32_t><<<grid_for(n), kThreads, 0, st>>>(d_heights, (int32_t*)w.keys, n);
-        if ((s = launched()) != APSEP_OK) return s;
+        s = launched(reverse_keys<int32_t>, n, st, d_heights, (int32_t*)w.keys, n);
+        if (s != APSEP_OK) return s;
         s = apsep_run_cmp(plan, w.keys, w.a, n, APSEP_LT, stream);
     }
     if (s != APSEP_OK) return s;
-    rect_area<<<grid_for(n), kThreads, 0, st>>>(d_heights, w.b, w.a, direct, n, (unsigned long long*)d_area);
-    return launched();
+    s = launched(rect_area, n, st, d_heights, w.b, w.a, direct, n, (unsigned long long*)d_area);
+    return s;
 }
 
 apsep_status apsep_cartesian_parents(apsep_plan* plan, const void* d_in, int32_t* d_out, int64_t n, void* d_work,
@@ -269,17 +279,17 @@ apsep_status apsep_cartesian_parents(apsep_plan* plan, const void* d_in, int32_t
         direct = false;
         for_key_type(dtype, [&](auto tag) {
             using T = std::remove_pointer_t<decltype(tag)>;
-            reverse_keys<T><<<grid_for(n), kThreads, 0, st>>>((const T*)d_in, (T*)w.keys, n);
+            s = launched(reverse_keys<T>, n, st, (const T*)d_in, (T*)w.keys, n);
         });
-        if ((s = launched()) != APSEP_OK) return s;
+        if (s != APSEP_OK) return s;
         s = apsep_run_cmp(plan, w.keys, w.a, n, APSEP_LT, stream);
     }
     if (s != APSEP_OK) return s;
     for_key_type(dtype, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        cartesian_parent<T><<<grid_for(n), kThreads, 0, st>>>((const T*)d_in, w.b, w.a, direct, d_out, n);
+        s = launched(cartesian_parent<T>, n, st, (const T*)d_in, w.b, w.a, direct, d_out, n);
     });
-    return launched();
+    return s;
 }
 
 }  // extern "C"

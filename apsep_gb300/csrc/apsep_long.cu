@@ -103,6 +103,7 @@ __device__ __forceinline__ K entry(const K* keys, const Levels<K>& lv, int lev, 
 template <typename K>
 __global__ void __launch_bounds__(kThreads) level_kernel(const K* __restrict__ src, int64_t src_size,
                                                          K* __restrict__ dst, int64_t e_lo, int64_t e_hi) {
+    grid_dependency_wait();
     const int lane = threadIdx.x & 31;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t e = e_lo + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); e < e_hi; e += nw) {
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(kPrologue)
     prologue_kernel(const K* __restrict__ keys, Levels<K> lv, int64_t b0, bool look_before, RangeScratch rs,
                     int num_ranges, K* __restrict__ rpre, Frontier<K>* fr) {
     __shared__ K wsum[kPrologue / 32];
+    grid_dependency_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (warp == 0 && look_before) {
         int64_t idx = b0;
@@ -224,6 +226,7 @@ __global__ void __launch_bounds__(kThreads)
     __shared__ K su[kLevels];
     __shared__ K spm;  // the minimum of everything before b0
     __shared__ uint32_t shas;
+    grid_dependency_wait();
     if (threadIdx.x < kLevels) su[threadIdx.x] = look_before ? fr->u[threadIdx.x] : KeyTraits<K>::pad();
     if (threadIdx.x == 0) {
         const uint32_t h = look_before ? fr->has : 0u;
@@ -368,13 +371,15 @@ apsep_status run_long(apsep_plan* plan, const K* keys, int64_t* out, int64_t n, 
         apsep_status s = plan_run_out64(plan, keys + b0, out + b0, b1 - b0, b0, cmp, cdst, st, &ra);
         if (s != APSEP_OK) return s;
         const bool look = b0 > 0;
-        prologue_kernel<K, MAPF><<<1, kPrologue, 0, st>>>(keys, lv, b0, look, ra.s, ra.num_ranges, rpre, fr);
+        if (launch_pdl(prologue_kernel<K, MAPF>, 1, kPrologue, 0, st, keys, lv, b0, look, ra.s, ra.num_ranges, rpre, fr) !=
+            cudaSuccess)
+            return APSEP_ECUDA;
         const int groups = (ra.num_tiles + 31) / 32;  // 32 tiles per warp and step
         const int grid = (int)std::min<int64_t>(std::max<int64_t>(ceil_div(groups, kThreads / 32), 1),
                                                 (int64_t)sms * std::max(per_sm, 1));
-        fix<<<grid, kThreads, 0, st>>>(keys, out, b0, b1, lv, fr, look, rpre, ra.s, (const K*)ra.s.chunk_min,
-                                       ra.num_tiles, ra.tiles_per_range, &ra.s.ctr->err);
-        if (cudaGetLastError() != cudaSuccess) return APSEP_ECUDA;
+        if (launch_pdl(fix, grid, kThreads, 0, st, keys, out, b0, b1, lv, fr, look, rpre, ra.s,
+                       (const K*)ra.s.chunk_min, ra.num_tiles, ra.tiles_per_range, &ra.s.ctr->err) != cudaSuccess)
+            return APSEP_ECUDA;
         if (!pieces || b1 == n) continue;
         // level entries that complete inside this piece (level 1 came with the run)
         int64_t span = 32;
@@ -383,10 +388,11 @@ apsep_status run_long(apsep_plan* plan, const K* keys, int64_t* out, int64_t n, 
             const int64_t e_lo = b0 / span, e_hi = b1 / span;
             if (e_hi > e_lo) {
                 const int g = (int)std::min<int64_t>(ceil_div(e_hi - e_lo, kThreads / 32), (int64_t)sms * 8);
-                level_kernel<K><<<g, kThreads, 0, st>>>(lv.p[l - 1], lv.size[l - 1], lv.p[l], e_lo, e_hi);
+                if (launch_pdl(level_kernel<K>, g, kThreads, 0, st, lv.p[l - 1], lv.size[l - 1], lv.p[l], e_lo, e_hi) !=
+                    cudaSuccess)
+                    return APSEP_ECUDA;
             }
         }
-        if (cudaGetLastError() != cudaSuccess) return APSEP_ECUDA;
     }
     return APSEP_OK;
 }

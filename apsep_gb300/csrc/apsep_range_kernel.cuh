@@ -946,20 +946,21 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     static_assert(OUTM == OUT_I32 || (!SEG && EP), "int64 and span answers: single arrays only");
     static_assert(!REV || (!SEG && EP && OUTM == OUT_I32 && KB == 4), "reversed runs: single arrays of 4-byte keys");
     constexpr bool OUT64 = OUTM == OUT_I64;
+    uint32_t epoch = 0;
+    if (lane == 0) {
+        for (int s = 0; s < kStages; s++) mbar_init(&bar[s], 1);
+        for (int k = 0; k < 4; k++) sPad[k] = KeyTraits<T>::pad();
+        fence_mbarrier_init();
+        fence_proxy_async_smem();
+    }
+    grid_dependency_wait();
     // One claim per CTA: its warps take WPC consecutive range ids, in the order
     // the CTAs start (so every range a warp may wait on belongs to a started CTA).
     if (threadIdx.x == 0) {
         sCta[0] = (int)atomicAdd(&a.s.ctr->range_counter, (unsigned)WPC);
         sCta[1] = 0;
     }
-    uint32_t epoch = 0;
-    if (lane == 0) {
-        epoch = ld_relaxed_u32(&a.s.ctr->epoch);
-        for (int s = 0; s < kStages; s++) mbar_init(&bar[s], 1);
-        for (int k = 0; k < 4; k++) sPad[k] = KeyTraits<T>::pad();
-        fence_mbarrier_init();
-        fence_proxy_async_smem();
-    }
+    if (lane == 0) epoch = ld_relaxed_u32(&a.s.ctr->epoch);
     __syncthreads();  // the CTA's claim is in shared memory
     const int r = sCta[0] + warp;
     epoch = __shfl_sync(FULL, epoch, 0);
@@ -2009,8 +2010,7 @@ inline cudaError_t launch_t(RangeArgs& a, const CUtensorMap& mi, const CUtensorM
     a.tiles_per_range = tpr;
     a.num_ranges = (a.num_tiles + tpr - 1) / tpr;
     const int ctas = (a.num_ranges + WPC - 1) / WPC;
-    apse_warp_kernel<T, IPT, WPC, INCL, SEG, EP, MAPF, OUTM, REV><<<ctas, WPC * 32, smem, st>>>(mi, mo, a);
-    return cudaGetLastError();
+    return launch_pdl(apse_warp_kernel<T, IPT, WPC, INCL, SEG, EP, MAPF, OUTM, REV>, ctas, WPC * 32, smem, st, mi, mo, a);
 }
 
 template <typename T, int IPT, int WPC, bool INCL, bool SEG, bool EP, int MAPF = KMAP_NONE, int OUTM = OUT_I32,

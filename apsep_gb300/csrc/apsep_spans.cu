@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "apsep.h"
+#include "apsep_internal.h"
 
 namespace {
 
@@ -46,6 +47,7 @@ constexpr int kDepth = (int)(kPiece / 16 / kThreads);  // 16-byte copies per thr
 
 __global__ void __launch_bounds__(kThreads, 16) copy_spans_kernel(const __grid_constant__ SpanBatch b) {
     __shared__ __align__(16) uint4 stage[kThreads * kDepth];  // one piece (16 KB)
+    apsep::grid_dependency_wait();
     const int64_t total = b.piece_start[b.n];
     for (int64_t pc = blockIdx.x; pc < total; pc += gridDim.x) {
         // the span holding piece pc: the last s with piece_start[s] <= pc (empty spans are skipped)
@@ -131,8 +133,8 @@ extern "C" apsep_status apsep_copy_spans(const void* const* src, void* const* ds
         const int64_t pieces = b.piece_start[m];
         if (pieces == 0) continue;
         const int grid = (int)(pieces < ctas ? pieces : ctas);
-        copy_spans_kernel<<<grid, kThreads, 0, (cudaStream_t)stream>>>(b);
-        if (cudaGetLastError() != cudaSuccess) return APSEP_ECUDA;
+        if (apsep::launch_pdl(copy_spans_kernel, grid, kThreads, 0, (cudaStream_t)stream, b) != cudaSuccess)
+            return APSEP_ECUDA;
     }
     return APSEP_OK;
 }
