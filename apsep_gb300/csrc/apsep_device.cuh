@@ -247,6 +247,13 @@ __device__ __forceinline__ uint32_t atom_add_acq_rel_u32(uint32_t* p, uint32_t v
 __device__ __forceinline__ void red_min_u64(uint64_t* p, uint64_t v) {
     asm volatile("red.relaxed.gpu.global.min.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
+// Fire-and-forget atomic add (relaxed, gpu scope).
+__device__ __forceinline__ void red_add_u32(uint32_t* p, uint32_t v) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+// Orders this thread's earlier accesses (and what it observed) before its later
+// ones at gpu scope; __threadfence() is the sequentially consistent form.
+__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ uint32_t ld_relaxed_u32(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

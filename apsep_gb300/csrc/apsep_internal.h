@@ -40,7 +40,6 @@ struct RangeScratch {
     Counters* ctr;
     uint64_t* group_min;    // [max_ranges/32] atomic min of (EPOCH_LIMIT - epoch) << 32 | ordered key
                             //   over each group of 32 ranges; all-ones when created
-    uint32_t* cta_ready;    // [kMaxCtas * kReadyStride] epoch in which every range has published, one line per CTA
     uint64_t* range_state;  // [max_ranges] tag<<32 | key bits: min of a finished range
     uint64_t* range_key;    // [max_ranges] 8-byte keys: the range minimum (range_state holds the tag)
     void* top_key;          // [max_ranges * kTopEntries] key: top of each range's final stack, bottom first
@@ -57,13 +56,11 @@ struct RangeScratch {
 constexpr int kMinTileKeys = 256;   // smallest tile of any configuration (one warp's)
 constexpr int kMaxTileKeys = 512;   // largest tile of any configuration
 constexpr int kMaxRanges = 4096;    // persistent warps per run, upper bound
-constexpr int kMaxCtas = kMaxRanges / 4;  // every configuration runs >= 4 warps per CTA
-constexpr int kReadyStride = 16;          // words between two CTAs' ready flags (64 bytes)
 constexpr int kTopEntries = 32;           // stack entries each range publishes for later ranges
 
 // Byte offsets of the scratch arrays for `capacity` keys (256-byte aligned).
 struct ScratchOffsets {
-    size_t gmin, ready, state, rkey, topk, topp, topc, tmin, cmin, flag, mask, total;
+    size_t gmin, state, rkey, topk, topp, topc, tmin, cmin, flag, mask, total;
     int64_t cap_tiles;
 };
 constexpr size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -74,8 +71,7 @@ constexpr ScratchOffsets scratch_offsets(int64_t capacity, int kb = 4) {
     o.cap_tiles = (cap + kMinTileKeys - 1) / kMinTileKeys + 1;
     const size_t cap_chunks = (size_t)(cap + 31) / 32 + kMaxTileKeys / 32;
     o.gmin = align256(sizeof(Counters));
-    o.ready = align256(o.gmin + (size_t)(kMaxRanges / 32) * 8);
-    o.state = align256(o.ready + (size_t)kMaxCtas * kReadyStride * 4);
+    o.state = align256(o.gmin + (size_t)(kMaxRanges / 32) * 8);
     o.rkey = align256(o.state + (size_t)kMaxRanges * 8);
     o.topk = align256(o.rkey + (size_t)kMaxRanges * 8);
     o.topp = align256(o.topk + (size_t)kMaxRanges * kTopEntries * kb);

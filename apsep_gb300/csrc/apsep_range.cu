@@ -21,7 +21,6 @@ size_t carve_scratch(void* base, int64_t capacity, RangeScratch* s, int kb) {
         char* b = (char*)base;
         s->ctr = (Counters*)b;
         s->group_min = (uint64_t*)(b + o.gmin);
-        s->cta_ready = (uint32_t*)(b + o.ready);
         s->range_state = (uint64_t*)(b + o.state);
         s->range_key = (uint64_t*)(b + o.rkey);
         s->top_key = b + o.topk;

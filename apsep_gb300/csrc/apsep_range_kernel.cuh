@@ -69,7 +69,7 @@ constexpr int kUpKeep = 64;     // entries a wholly increasing tile leaves on th
 constexpr int kXQueries = 3;    // cross-lane queries per lane and round (32 * 3 keys per round)
 // Deferred keys listed in shared memory per range (a random walk's prefix
 // minima, ~sqrt(range) of them, fit; 8-byte keys: what shared memory leaves).
-template <int KB> constexpr int kDefCapOf = KB == 8 ? 128 : 256;
+template <int KB> constexpr int kDefCapOf = KB == 8 ? 128 : 192;
 constexpr int kCapCap = 32;     // capped keys listed in shared memory per range
 
 // Shared memory of one warp (KB: bytes per key).
@@ -446,11 +446,14 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
 //
 // Publishing range r (lane 0): an atomic minimum into its group's word
 // (groups of 32 ranges), a fence, the range's tagged minimum (range_state),
-// and one relaxed increment of the count of published ranges.  The range
-// that completes the count raises one ready flag per CTA.  Range r then
-// needs the minima of the earlier ranges of its group plus those of the
-// earlier groups: one round of loads, no hot spot, and no step of the last
-// range's path waits on another range's loads.
+// and one fire-and-forget increment of the count of published ranges.  One
+// warp per CTA polls that count (152 pollers), the others a word in shared
+// memory.  Range r then needs the minima of the earlier ranges of its group
+// plus those of the earlier groups: one round of loads, and no step of the last
+// range's path waits on another range's loads.  (With the last range raising a
+// flag per CTA, two more fences and a store and a load through L2, a run took
+// 0.6-1.4 us longer: 2^18 uniform keys 14.2 -> 12.9 us.  One warp loading the
+// minima for its whole CTA took 1 us longer again.)
 //
 // Group words: atomic minima of (EPOCH_LIMIT - epoch) << 32 | ordered key.
 // The current run's tag is below every older run's, so its first minimum
@@ -458,8 +461,8 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
 // start all-ones and are cleared again when the epoch wraps).
 //
 // Every range of a launch is resident when the launch fits the device (the
-// grid is sized from occupancy), so the ready flag always comes.  When it
-// does not come within a bound (the launch shares the device and some warps
+// grid is sized from occupancy), so the count always completes.  When it does
+// not within a bound (the launch shares the device and some warps
 // have not started), range r falls back to waiting on the tagged minima of
 // the ranges before it, all of which already run (ids are handed out in
 // start order), so no wait depends on a warp that may not start.  Every wait
@@ -472,36 +475,25 @@ constexpr int kDirectRanges = 256;
 
 template <typename T>
 __device__ void range_publish(int r, uint32_t epoch, T rmin, const RangeArgs& a) {
-    constexpr unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     const uint32_t tag = (epoch << 2) | FLAG_AGG;
-    const bool direct = a.num_ranges <= kDirectRanges;
-    int last = 0;
-    if (lane == 0 && r != a.skip_publish_range) {
+    if ((threadIdx.x & 31) == 0 && r != a.skip_publish_range) {
         if constexpr (sizeof(T) == 8)
             __stcg((unsigned long long*)&a.s.range_key[r], (unsigned long long)KeyTraits<T>::bits(rmin));
         else
             red_min_u64(&a.s.group_min[r >> 5], ((uint64_t)(EPOCH_LIMIT - epoch) << 32) | KeyTraits<T>::ord(rmin));
         // release: this range's words (every lane's, ordered by the caller's
         // __syncwarp) and the group minimum before the range minimum and the count
-        __threadfence();
+        fence_acq_rel();
         __stcg((unsigned long long*)&a.s.range_state[r],
                ((uint64_t)tag << 32) | (sizeof(T) == 8 ? 0u : (uint32_t)KeyTraits<T>::bits(rmin)));
-        if (!direct) {
-            last = atomicAdd(&a.s.ctr->finished, 1u) == (uint32_t)(a.num_ranges - 1);
-            if (last) __threadfence();  // acquire: every range's publication
-        }
+        if (a.num_ranges > kDirectRanges) red_add_u32(&a.s.ctr->finished, 1u);
     }
-    if (!__shfl_sync(FULL, last, 0)) return;
-    __syncwarp();
-    __threadfence();  // release to the flags' readers
-    for (int c = lane; c < (int)gridDim.x; c += 32) a.s.cta_ready[(size_t)c * kReadyStride] = epoch;
 }
 
 // p: the minimum over ranges [0, r); win (lane i): the minimum of range r-1-i
 // (pad below range 0), the window phase 2 searches first.
 template <typename T>
-__device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, T& p, bool& has_p, T& win) {
+__device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, int* sReady, T& p, bool& has_p, T& win) {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int g = r >> 5;
@@ -510,7 +502,8 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, T& p, bo
     win = KeyTraits<T>::pad();
     has_p = r > 0;
     if (r == 0) return;
-    const uint32_t* flag = &a.s.cta_ready[(size_t)blockIdx.x * kReadyStride];
+    const uint32_t* count = &a.s.ctr->finished;
+    const uint32_t all = (uint32_t)a.num_ranges;
     // every range has published: the window (it holds the group's earlier
     // ranges) and the earlier groups, in one round of loads
     auto from_ready = [&]() {
@@ -537,18 +530,30 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, T& p, bo
         for (int o = 16; o > 0; o >>= 1) m = KeyTraits<T>::vmin(m, __shfl_xor_sync(FULL, m, o));
         p = m;
     };
-    // 1. the ready flag of this CTA (one line, polled by one lane per warp); a
-    //    launch of few ranges raises none: its ranges wait on their predecessors
+    // 1. the count of published ranges, polled by the first warp of the CTA that gets
+    //    here; the others watch its word in shared memory (0: waiting, 1: every
+    //    range has published, 2: gave up).  A launch of few ranges has no count: its
+    //    ranges wait on their predecessors.
     int ready = 0;
     if (lane == 0 && a.num_ranges > kDirectRanges) {
         const uint32_t bound = min(a.spin_limit, 1u << 16);
-        for (uint32_t s = 0;; s++) {
-            if (ld_acquire_u32(flag) == epoch) {
-                ready = 1;
-                break;
+        volatile int* word = sReady;
+        if (atomicExch(sReady + 1, 1) == 0) {
+            for (uint32_t s = 0;; s++) {
+                if (ld_acquire_u32(count) == all) {
+                    ready = 1;
+                    break;
+                }
+                if (s >= bound) break;
+                if (s >= 64) __nanosleep(64);
             }
-            if (s >= bound) break;
-            __nanosleep(s < 8 ? 64 : 256);
+            __threadfence_block();
+            *word = ready ? 1 : 2;
+        } else {
+            int w;
+            for (uint32_t s = 0; (w = *word) == 0 && s < 16 * bound; s++) __nanosleep(32);
+            __threadfence_block();
+            ready = w == 1;
         }
     }
     __syncwarp();  // lane 0's acquire before the other lanes' loads
@@ -556,7 +561,7 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, T& p, bo
         from_ready();
         return;
     }
-    // 2. fallback: wait for the tagged minima of the earlier ranges (or the flag)
+    // 2. fallback: wait for the tagged minima of the earlier ranges (or the count)
     for (uint32_t spins = 0;; spins++) {
         bool ok = true;
         T m = KeyTraits<T>::pad();
@@ -573,7 +578,7 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, T& p, bo
             win = wi >= 0 ? range_min<T>(a, wi) : KeyTraits<T>::pad();
             return;
         }
-        if (__shfl_sync(FULL, lane == 0 ? (int)(ld_acquire_u32(flag) == epoch) : 0, 0)) {
+        if (__shfl_sync(FULL, lane == 0 && a.num_ranges > kDirectRanges ? (int)(ld_acquire_u32(count) == all) : 0, 0)) {
             __syncwarp();
             from_ready();
             return;
@@ -886,9 +891,12 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
 // land -- and writes each answer mirrored back, n - 1 - answer (-1 for none)
 // at element n - 1 - position: the next smaller key, in one run.
 
+// 16 warps per SM in every configuration: without the bound the 4-warp CTAs took
+// 205 registers a thread and 8 warps fitted; with it, and a deferred list that
+// lets four of their CTAs share an SM, 2^20 random-walk keys 34.7 -> 28.5 us.
 template <typename T, int IPT, int WPC, bool INCL, bool SEG, bool EP, int MAPF = KMAP_NONE, int OUTM = OUT_I32,
           bool REV = false>
-__global__ void __launch_bounds__(WPC * 32, (WPC >= 16 && sizeof(T) == 4 ? 1 : 2))
+__global__ void __launch_bounds__(WPC * 32, 16 / WPC)
 apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_out,
                  const RangeArgs a) {
     constexpr int KB = (int)sizeof(T);  // bytes per key
@@ -913,7 +921,8 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     const int warp = threadIdx.x >> 5;
     unsigned char* cta_sm = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* wsm = cta_sm + (size_t)warp * L::kBytes;
-    // CTA words: [0] the CTA's first range, [1] warps of the CTA finished
+    // CTA words: [0] the CTA's first range, [1] warps of the CTA finished, [2] and [3]
+    // see range_prefix
     int* sCta = (int*)(cta_sm + (size_t)WPC * L::kBytes);
     T* sV = (T*)(wsm + L::kV);
     int32_t* O = (int32_t*)(wsm + L::kO);
@@ -958,7 +967,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     // the CTAs start (so every range a warp may wait on belongs to a started CTA).
     if (threadIdx.x == 0) {
         sCta[0] = (int)atomicAdd(&a.s.ctr->range_counter, (unsigned)WPC);
-        sCta[1] = 0;
+        sCta[1] = sCta[2] = sCta[3] = 0;
     }
     if (lane == 0) epoch = ld_relaxed_u32(&a.s.ctr->epoch);
     __syncthreads();  // the CTA's claim is in shared memory
@@ -1962,13 +1971,13 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         }
         __syncwarp();  // every lane's words before lane 0's release in range_publish
         range_publish<T>(r, epoch, rmin, a);
-        T P, win;
-        bool has_p;
-        range_prefix<T>(r, epoch, a, P, has_p, win);
-        if (lane == 0) {
+        if (lane == 0) {  // (beside the wait for the other ranges)
             bulk_wait0();       // this range's tile stores have landed ...
             fence_proxy_async();  // ... before phase 2 overwrites flagged keys
         }
+        T P, win;
+        bool has_p;
+        range_prefix<T>(r, epoch, a, sCta + 2, P, has_p, win);
         __syncwarp();  // lane 0's acquire and wait before every lane's reads and writes
 
         phase2<T, IPT, INCL, SEG, MAPF, OUTM, REV>(a, wsm, r, t0, t1, def_total, cap_total, first_start, P, has_p, win);
@@ -1993,7 +2002,6 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     if (last && epoch >= EPOCH_LIMIT) {  // once per 2^30 runs: stale words could alias
         for (int i = lane; i < a.s.max_ranges; i += 32) a.s.range_state[i] = 0;
         for (int i = lane; i < a.s.max_ranges / 32; i += 32) a.s.group_min[i] = ~0ull;
-        for (int i = lane; i < kMaxCtas; i += 32) a.s.cta_ready[(size_t)i * kReadyStride] = 0;
     }
 }
 
