@@ -14,7 +14,8 @@
 // reversals itself (apsep_mapped.cu): previous greater and the stock span are
 // one run each with the keys flipped as they load (and position - answer as
 // the answers leave), next smaller one run over the reversed array with its
-// answers mirrored as they leave (n a multiple of 32), and the histogram and
+// answers mirrored as they leave (the last n % 32 keys apart: a pass over the answers
+// completes them from those), and the histogram and
 // Cartesian tree take that run for their next-smaller half.  Otherwise each is
 // a few memory-bound passes (flip / reverse / mirror / epilogue, grid-stride,
 // coalesced) around one or two engine runs.  All run on the caller's plan and
@@ -89,10 +90,53 @@ __device__ __forceinline__ int64_t next_from_reversed(const int32_t* __restrict_
     const int32_t a = ar[n - 1 - i];
     return a >= 0 ? n - 1 - a : -1;
 }
-// next[i] from R: the next-smaller answers themselves (direct, a reversed run
-// of the engine), or the reversed array's previous-smaller answers.
-__device__ __forceinline__ int64_t next_of(const int32_t* __restrict__ R, bool direct, int64_t n, int64_t i) {
-    return direct ? (int64_t)R[i] : next_from_reversed(R, n, i);
+// The keys after the last multiple of 32 (the engine's reversed run takes whole
+// 32-key rows): at most 31 of them, in shared memory, with their minimum.
+template <typename T>
+struct Tail {
+    const T* v;
+    T least;
+    int count;
+    int64_t base;  // position of the first (n when there is none)
+};
+// Called by every thread of the block; v: 32 keys of its shared memory.
+template <typename T>
+__device__ __forceinline__ Tail<T> load_tail(const T* __restrict__ a, int64_t n, int64_t base, T* v) {
+    const int count = (int)(n - base);
+    if ((int)threadIdx.x < count) v[threadIdx.x] = a[base + threadIdx.x];
+    __syncthreads();
+    T least = count > 0 ? v[0] : T(0);
+    for (int j = 1; j < count; j++) least = v[j] < least ? v[j] : least;
+    return {v, least, count, base};
+}
+// The first tail key at or after position i that is smaller (or equal) than q, or -1.
+template <bool LE, typename T>
+__device__ __forceinline__ int64_t next_in_tail(const Tail<T>& t, T q, int64_t i) {
+    if (t.count == 0 || !(LE ? t.least <= q : t.least < q)) return -1;
+    for (int j = i > t.base ? (int)(i - t.base) : 0; j < t.count; j++)
+        if (LE ? t.v[j] <= q : t.v[j] < q) return t.base + j;
+    return -1;
+}
+// next[i] from R: the next-smaller answers themselves over the keys before the
+// tail (direct, a reversed run of the engine), or the reversed array's
+// previous-smaller answers (no tail).
+template <typename T>
+__device__ __forceinline__ int64_t next_of(const T* __restrict__ a, const int32_t* __restrict__ R, bool direct,
+                                           const Tail<T>& t, int64_t n, int64_t i) {
+    if (!direct) return next_from_reversed(R, n, i);
+    const int64_t r = i < t.base ? (int64_t)R[i] : -1;
+    return r >= 0 || t.count == 0 ? r : next_in_tail<false>(t, a[i], i + 1);
+}
+
+// Completes next-smaller answers of a reversed run over the keys before the tail:
+// its unanswered keys and the tail's own.
+template <typename T, bool LE>
+__global__ void next_with_tail(const T* __restrict__ a, int32_t* __restrict__ out, int64_t n, int64_t base) {
+    __shared__ T tail_keys[32];
+    apsep::grid_dependency_wait();
+    const Tail<T> t = load_tail(a, n, base, tail_keys);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        if (i >= base || out[i] < 0) out[i] = (int32_t)next_in_tail<LE>(t, a[i], i + 1);
 }
 
 __global__ void mirror_answers(const int32_t* __restrict__ ar, int32_t* __restrict__ out, int64_t n) {
@@ -111,12 +155,15 @@ __global__ void span_from_previous(int32_t* __restrict__ a, int64_t n) {
 // next strictly smaller (n: none).  Only positive areas compete (heights are
 // non-negative by contract; a negative height contributes nothing).
 __global__ void rect_area(const int32_t* __restrict__ h, const int32_t* __restrict__ L,
-                          const int32_t* __restrict__ ar, bool direct, int64_t n, unsigned long long* __restrict__ best) {
+                          const int32_t* __restrict__ ar, bool direct, int64_t base, int64_t n,
+                          unsigned long long* __restrict__ best) {
     __shared__ long long warp_best[kThreads / 32];
+    __shared__ int32_t tail_keys[32];
     apsep::grid_dependency_wait();
+    const Tail<int32_t> t = load_tail(h, n, base, tail_keys);
     long long m = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t r = next_of(ar, direct, n, i);
+        const int64_t r = next_of(h, ar, direct, t, n, i);
         const int64_t w = (r < 0 ? n : r) - (int64_t)L[i] - 1;
         const long long area = (long long)h[i] * w;
         m = area > m ? area : m;
@@ -140,10 +187,13 @@ __global__ void rect_area(const int32_t* __restrict__ h, const int32_t* __restri
 // larger key, R on a tie; -1 for the root.
 template <typename T>
 __global__ void cartesian_parent(const T* __restrict__ a, const int32_t* __restrict__ L,
-                                 const int32_t* __restrict__ ar, bool direct, int32_t* __restrict__ out, int64_t n) {
+                                 const int32_t* __restrict__ ar, bool direct, int64_t base,
+                                 int32_t* __restrict__ out, int64_t n) {
+    __shared__ T tail_keys[32];
     apsep::grid_dependency_wait();
+    const Tail<T> t = load_tail(a, n, base, tail_keys);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t l = L[i], r = next_of(ar, direct, n, i);
+        const int64_t l = L[i], r = next_of(a, ar, direct, t, n, i);
         int64_t p;
         if (r < 0) p = l;
         else if (l < 0) p = r;
@@ -155,6 +205,16 @@ __global__ void cartesian_parent(const T* __restrict__ a, const int32_t* __restr
 bool overlaps(const void* a, size_t an, const void* b, size_t bn) {
     const uintptr_t a0 = (uintptr_t)a, b0 = (uintptr_t)b;
     return a0 < b0 + bn && b0 < a0 + an;
+}
+
+// The reversed run of the engine over the keys before the last n % 32, when it has
+// that form for the call (whole rows of 32 keys; *base: where they end), else
+// APSEP_ENOTSUP.
+apsep_status run_reversed(apsep_plan* plan, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp, void* stream,
+                          int64_t* base) {
+    *base = n / 32 * 32;
+    if (*base == 0 || overlaps(d_in, (size_t)n * 4, d_out, (size_t)n * 4)) return APSEP_ENOTSUP;
+    return plan_run_reversed(plan, d_in, d_out, *base, cmp, stream);
 }
 
 // Common argument checks; fills the plan's key type.
@@ -213,8 +273,17 @@ apsep_status apsep_run_next_smaller(apsep_plan* plan, const void* d_in, int32_t*
     if (s != APSEP_OK || n == 0) return s;
     // one engine run over the reversed array, answers mirrored as they leave,
     // when it has that form for the call; else reverse, run, mirror
-    if ((s = plan_run_reversed(plan, d_in, d_out, n, cmp, stream)) != APSEP_ENOTSUP) return s;
     const cudaStream_t st = (cudaStream_t)stream;
+    int64_t base = n;
+    if ((s = run_reversed(plan, d_in, d_out, n, cmp, stream, &base)) != APSEP_ENOTSUP) {
+        if (s != APSEP_OK || base == n) return s;
+        const bool le = cmp == APSEP_LE;
+        if (dtype == APSEP_INT32)
+            return launched(le ? next_with_tail<int32_t, true> : next_with_tail<int32_t, false>, n, st,
+                            (const int32_t*)d_in, d_out, n, base);
+        return launched(le ? next_with_tail<float, true> : next_with_tail<float, false>, n, st, (const float*)d_in,
+                        d_out, n, base);
+    }
     const Work w = carve(d_work, n, dtype);
     for_key_type(dtype, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
@@ -255,14 +324,16 @@ apsep_status apsep_largest_rectangle(apsep_plan* plan, const int32_t* d_heights,
     // next smaller: one reversed run when the engine has that form, else
     // reverse the heights and run (the answers then come mirrored)
     bool direct = true;
-    if ((s = plan_run_reversed(plan, d_heights, w.a, n, APSEP_LT, stream)) == APSEP_ENOTSUP) {
+    int64_t base = n;  // where the tail begins (none after a run over the whole reversed copy)
+    if ((s = run_reversed(plan, d_heights, w.a, n, APSEP_LT, stream, &base)) == APSEP_ENOTSUP) {
         direct = false;
+        base = n;
         s = launched(reverse_keys<int32_t>, n, st, d_heights, (int32_t*)w.keys, n);
         if (s != APSEP_OK) return s;
         s = apsep_run_cmp(plan, w.keys, w.a, n, APSEP_LT, stream);
     }
     if (s != APSEP_OK) return s;
-    s = launched(rect_area, n, st, d_heights, w.b, w.a, direct, n, (unsigned long long*)d_area);
+    s = launched(rect_area, n, st, d_heights, w.b, w.a, direct, base, n, (unsigned long long*)d_area);
     return s;
 }
 
@@ -275,8 +346,10 @@ apsep_status apsep_cartesian_parents(apsep_plan* plan, const void* d_in, int32_t
     const Work w = carve(d_work, n, dtype);
     if ((s = apsep_run_cmp(plan, d_in, w.b, n, APSEP_LE, stream)) != APSEP_OK) return s;
     bool direct = true;  // next smaller straight from a reversed run, else mirrored
-    if ((s = plan_run_reversed(plan, d_in, w.a, n, APSEP_LT, stream)) == APSEP_ENOTSUP) {
+    int64_t base = n;
+    if ((s = run_reversed(plan, d_in, w.a, n, APSEP_LT, stream, &base)) == APSEP_ENOTSUP) {
         direct = false;
+        base = n;
         for_key_type(dtype, [&](auto tag) {
             using T = std::remove_pointer_t<decltype(tag)>;
             s = launched(reverse_keys<T>, n, st, (const T*)d_in, (T*)w.keys, n);
@@ -287,7 +360,7 @@ apsep_status apsep_cartesian_parents(apsep_plan* plan, const void* d_in, int32_t
     if (s != APSEP_OK) return s;
     for_key_type(dtype, [&](auto tag) {
         using T = std::remove_pointer_t<decltype(tag)>;
-        s = launched(cartesian_parent<T>, n, st, (const T*)d_in, w.b, w.a, direct, d_out, n);
+        s = launched(cartesian_parent<T>, n, st, (const T*)d_in, w.b, w.a, direct, base, d_out, n);
     });
     return s;
 }
