@@ -77,6 +77,11 @@ __device__ __forceinline__ T map_key(T x) {
     else if constexpr (KMAP == KMAP_FLIP) return flip_key(x);
     else return x;
 }
+// The raw key that the key map takes to the pad.
+template <typename T, int KMAP>
+__device__ __forceinline__ T raw_pad() {
+    return KMAP == KMAP_FLIP ? flip_key(KeyTraits<T>::pad()) : KeyTraits<T>::pad();
+}
 // A key from global memory, through the key map.
 template <typename T, int KMAP>
 __device__ __forceinline__ T load_key(const T* p) {

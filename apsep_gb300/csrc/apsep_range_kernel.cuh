@@ -958,7 +958,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     uint32_t epoch = 0;
     if (lane == 0) {
         for (int s = 0; s < kStages; s++) mbar_init(&bar[s], 1);
-        for (int k = 0; k < 4; k++) sPad[k] = KeyTraits<T>::pad();
+        for (int k = 0; k < 4; k++) sPad[k] = raw_pad<T, MAPF>();
         fence_mbarrier_init();
         fence_proxy_async_smem();
     }
@@ -1021,33 +1021,26 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             T* V = sV + (size_t)slot * WT;
             const bool full = tile_full(t);
             const int tile_base = t * WT;
+            // Key e of the tile: the raw keys stay as they landed and go through the key map
+            // as they are read; a reversed run sees them, and writes O, from the end
+            // (reversing and mapping the tile in place cost 25-40 us at 2^25).
+            auto at = [](int e) { return REV ? WT - 1 - e : e; };
+            auto key = [&](int e) { return map_key<T, MAPF>(V[ks(at(e))]); };
+            // the lane's 16-byte groups in element order, and the key at each place of them
+            auto chunk = [&](int c) { return REV ? WT - (lane + 1) * IPT + c : lane * IPT + c; };
+            auto in_chunk = [](int c) { return REV ? IPT - 1 - c : c; };
+            // answers as they are written: reversed runs mirror them
+            auto mirror = [&](int p) { return REV ? a.n - 1 - p : p; };
             const int valid_keys = min(WT, a.n - tile_base);
 
             if (full) {
                 if (!mbar_wait_bounded(&bar[slot], par, a.spin_limit) && lane == 0) atomicOr(err, ERR_TMA_TIMEOUT);
-                if constexpr (REV) {  // the tile arrived in element order: reverse it in place
-                    T rv[IPT];
-#pragma unroll
-                    for (int j = 0; j < IPT; j++) rv[j] = V[ks(WT - 1 - (j * 32 + lane))];
-                    __syncwarp();
-#pragma unroll
-                    for (int j = 0; j < IPT; j++) V[ks(j * 32 + lane)] = rv[j];
-                    __syncwarp();
-                }
-                if constexpr (MAPF != KMAP_NONE) {  // the tile's keys through the key map, in place
-#pragma unroll
-                    for (int j = 0; j < IPT; j++) {
-                        const int e = j * 32 + lane;
-                        V[ks(e)] = map_key<T, MAPF>(V[ks(e)]);
-                    }
-                }
             } else {
 #pragma unroll
                 for (int j = 0; j < IPT; j++) {
                     const int e = j * 32 + lane;
                     const int g = tile_base + e;
-                    V[ks(e)] = g < a.n && (!head || g >= head) ? (MAPF != KMAP_NONE || REV ? key_at<T, MAPF, REV>(d_in, a.n, g) : d_in[g])
-                                                                : KeyTraits<T>::pad();
+                    V[ks(at(e))] = g < a.n && (!head || g >= head) ? d_in[REV ? a.n - 1 - g : g] : raw_pad<T, MAPF>();
                 }
                 // A view head makes tile 0 plain while tile kStages streams into its
                 // slot: the plain tile completes the slot barrier's phase by itself.
@@ -1111,11 +1104,11 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             if constexpr (KB == 4) {
 #pragma unroll
                 for (int q4 = 0; q4 < IPT / 4; q4++) {
-                    const uint4 rr = *reinterpret_cast<const uint4*>(&V[swz(lane * IPT + 4 * q4)]);
-                    v[4 * q4 + 0] = KeyTraits<T>::from_bits(rr.x);
-                    v[4 * q4 + 1] = KeyTraits<T>::from_bits(rr.y);
-                    v[4 * q4 + 2] = KeyTraits<T>::from_bits(rr.z);
-                    v[4 * q4 + 3] = KeyTraits<T>::from_bits(rr.w);
+                    const uint4 rr = *reinterpret_cast<const uint4*>(&V[swz(chunk(4 * q4))]);
+                    v[in_chunk(4 * q4 + 0)] = KeyTraits<T>::from_bits(rr.x);
+                    v[in_chunk(4 * q4 + 1)] = KeyTraits<T>::from_bits(rr.y);
+                    v[in_chunk(4 * q4 + 2)] = KeyTraits<T>::from_bits(rr.z);
+                    v[in_chunk(4 * q4 + 3)] = KeyTraits<T>::from_bits(rr.w);
                 }
             } else {  // two 8-byte keys per 16-byte chunk
 #pragma unroll
@@ -1124,6 +1117,10 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     v[2 * q2 + 0] = KeyTraits<T>::from_bits((uint64_t)rr.x);
                     v[2 * q2 + 1] = KeyTraits<T>::from_bits((uint64_t)rr.y);
                 }
+            }
+            if constexpr (MAPF != KMAP_NONE) {
+#pragma unroll
+                for (int k = 0; k < IPT; k++) v[k] = map_key<T, MAPF>(v[k]);
             }
             const int lb = tile_base + lane * IPT;  // position of this lane's first key
             const int nvalid = min(max(a.n - lb, 0), IPT);
@@ -1147,7 +1144,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                                 const int k = __ffs(m) - 1;
                                 m &= m - 1;
                                 sDefP[idx] = lb + k;
-                                sDefV[idx] = V[ks(lane * IPT + k)];
+                                sDefV[idx] = key(lane * IPT + k);
                                 idx++;
                             }
                         }
@@ -1190,36 +1187,6 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     }
                     return;
                 }
-                if constexpr (REV) {  // mirrored answers at the mirrored positions, in element order
-                    __syncwarp();     // every lane's answers are in O
-                    if (full) {
-                        int ro[IPT];
-#pragma unroll
-                        for (int j = 0; j < IPT; j++) {
-                            const int o = O[swz(WT - 1 - (j * 32 + lane))];
-                            ro[j] = o >= 0 ? a.n - 1 - o : -1;
-                        }
-                        __syncwarp();
-#pragma unroll
-                        for (int j = 0; j < IPT; j++) O[swz(j * 32 + lane)] = ro[j];
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            tma_store_2d(&map_out, 0, tile_row(t), O);
-                            bulk_commit();
-                        }
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < IPT; j++) {
-                            const int e = j * 32 + lane;
-                            if (e < valid_keys) {
-                                const int o = O[swz(e)];
-                                a.d_out[a.n - 1 - (tile_base + e)] = o >= 0 ? a.n - 1 - o : -1;
-                            }
-                        }
-                    }
-                    return;
-                }
                 if constexpr (OUTM == OUT_SPAN) {  // spans: position - answer
                     __syncwarp();                   // every lane's answers are in O
     #pragma unroll
@@ -1251,14 +1218,14 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 __syncwarp();
                 if (full) {
                     if (lane == 0) {
-                        tma_store_2d(&map_out, 0, t * W, O);
+                        tma_store_2d(&map_out, 0, REV ? tile_row(t) : t * W, O);
                         bulk_commit();
                     }
                 } else {
     #pragma unroll
                     for (int j = 0; j < IPT; j++) {
                         const int e = j * 32 + lane;
-                        if (e < valid_keys && (!head || tile_base + e >= head)) a.d_out[tile_base + e] = O[swz(e)];
+                        if (e < valid_keys && (!head || tile_base + e >= head)) a.d_out[mirror(tile_base + e)] = O[swz(at(e))];
                     }
                 }
             };
@@ -1266,13 +1233,13 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             // The four keys before the lane's first (lane 0: pads).
             T h[4];
             {
-                const T* hp = lane > 0 ? &V[ks(lane * IPT - 4)] : sPad;
+                const T* hp = lane > 0 ? &V[ks(REV ? WT - lane * IPT : lane * IPT - 4)] : sPad;
                 if constexpr (KB == 4) {
                     const uint4 rr = *reinterpret_cast<const uint4*>(hp);
-                    h[0] = KeyTraits<T>::from_bits(rr.x);
-                    h[1] = KeyTraits<T>::from_bits(rr.y);
-                    h[2] = KeyTraits<T>::from_bits(rr.z);
-                    h[3] = KeyTraits<T>::from_bits(rr.w);
+                    h[REV ? 3 : 0] = KeyTraits<T>::from_bits(rr.x);
+                    h[REV ? 2 : 1] = KeyTraits<T>::from_bits(rr.y);
+                    h[REV ? 1 : 2] = KeyTraits<T>::from_bits(rr.z);
+                    h[REV ? 0 : 3] = KeyTraits<T>::from_bits(rr.w);
                 } else {
                     const T* hq = lane > 0 ? &V[ks(lane * IPT - 2)] : sPad + 2;
                     const ulonglong2 r0 = *reinterpret_cast<const ulonglong2*>(hp);
@@ -1282,6 +1249,10 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     h[2] = KeyTraits<T>::from_bits((uint64_t)r1.x);
                     h[3] = KeyTraits<T>::from_bits((uint64_t)r1.y);
                 }
+            }
+            if constexpr (MAPF != KMAP_NONE) {
+#pragma unroll
+                for (int k = 0; k < 4; k++) h[k] = map_key<T, MAPF>(h[k]);
             }
             const T prev_last = h[3];
 
@@ -1342,7 +1313,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 if (same) {
                     const T tmin = __shfl_sync(FULL, v[IPT - 1], 31);
                     const int top = 31 - __clz(same);
-                    const int tp = max(sStkP[(wlo + top) & (K - 1)] - (OUTM == OUT_I32 ? head : 0), -1);
+                    const int tp = mirror(max(sStkP[(wlo + top) & (K - 1)] - (OUTM == OUT_I32 ? head : 0), -1));
 #pragma unroll
                     for (int q4 = 0; q4 < IPT / 4; q4++)
                         *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) = make_int4(tp, tp, tp, tp);
@@ -1396,7 +1367,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     const T tmin = __shfl_sync(FULL, v[IPT - 1], 31);
                     for (int e = lane; e < WT && def_total + e < kDefCap; e += 32) {
                         sDefP[def_total + e] = tile_base + e;
-                        sDefV[def_total + e] = V[ks(e)];
+                        sDefV[def_total + e] = key(e);
                     }
                     if (lane < W) __stcg(&a.s.tile_mask[(size_t)t * MW + lane], 0xffffffffu);
                     if (lane == 0) {
@@ -1459,11 +1430,12 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     // stack top here: a pad does not lie below the tile's first key)
                     const int top_pos = sStkP[(stk_hi - 1) & (K - 1)] - head;
                     const int hb = lb - head;
+                    auto up_ans = [&](int k) { return mirror(lane == 0 && k == 0 ? top_pos : hb + k - 1); };
 #pragma unroll
                     for (int q4 = 0; q4 < IPT / 4; q4++)
-                        *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) =
-                            make_int4(lane == 0 && q4 == 0 ? top_pos : hb + 4 * q4 - 1, hb + 4 * q4, hb + 4 * q4 + 1,
-                                      hb + 4 * q4 + 2);
+                        *reinterpret_cast<int4*>(&O[swz(chunk(4 * q4))]) =
+                            make_int4(up_ans(in_chunk(4 * q4)), up_ans(in_chunk(4 * q4 + 1)), up_ans(in_chunk(4 * q4 + 2)),
+                                      up_ans(in_chunk(4 * q4 + 3)));
                     if ((lane & (TPC - 1)) == 0) __stcg(&chunk_min_w[(size_t)t * W + lane / TPC], v[0]);
                     if (lane == 0) {
                         __stcg(&a.s.tile_flag[t], 0u);
@@ -1490,7 +1462,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
 #pragma unroll
                     for (int h = 0; h < kUpKeep / 32; h++) {  // the tile's last keys, one per lane and step
                         const int e = WT - kUpKeep + h * 32 + lane;
-                        sStkV[(base_idx + e) & (K - 1)] = V[ks(e)];
+                        sStkV[(base_idx + e) & (K - 1)] = key(e);
                         sStkP[(base_idx + e) & (K - 1)] = tile_base + e;
                     }
                     stk_hi = base_idx + WT;
@@ -1569,7 +1541,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 // run pays for the rolled loop instead, 0.88 -> 1.10 ms).
 #pragma unroll 1
                 for (int k = 0; k < IPT; k++) {
-                    const T vk = V[ks(lane * IPT + k)];
+                    const T vk = key(lane * IPT + k);
                     if (k > 0)
                         while (si >= stk_lo && !lt<INCL>(sStkV[si & (K - 1)], vk)) si--;
                     int rk = -1;
@@ -1604,26 +1576,26 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             unsigned umask = 0;  // keys without an in-thread answer: bit IPT - 1 - k for key k
             {
                 int res[IPT];  // absolute answers, -1 = none in the thread
-                const int lbo = lb - rel;
+                const int lbo = lb - rel, mbo = mirror(lbo);
                 if (mono == FULL) {  // monotone lanes need no ladder
-                    res[0] = lane > 0 && b_adj ? lbo - 1 : -1;
+                    res[0] = lane > 0 && b_adj ? mirror(lbo - 1) : -1;
 #pragma unroll
-                    for (int k = 1; k < IPT; k++) res[k] = adj ? lbo + k - 1 : -1;
+                    for (int k = 1; k < IPT; k++) res[k] = adj ? mirror(lbo + k - 1) : -1;
                 } else {
 #pragma unroll
                     for (int k = 0; k < IPT; k++) {
-                        int rk = -1 - lbo;  // relative to lbo
+                        int rk = REV ? mbo + 1 : -1 - lbo;  // relative to lbo
 #pragma unroll
                         for (int j = k; j < 4; j++) take_if_lt<INCL>(rk, h[j], v[k], zero, j - 4);
 #pragma unroll
                         for (int j = 0; j < k; j++) take_if_lt<INCL>(rk, v[j], v[k], zero, j);
-                        res[k] = rk + lbo;
+                        res[k] = REV ? mbo - rk : rk + lbo;
                     }
                     if constexpr (INCL) {  // lane 0's pads qualify for keys of the pad's value
                         if (lane == 0)
 #pragma unroll
                             for (int k = 0; k < 4; k++)
-                                if (res[k] < lbo) res[k] = -1;
+                                if (REV ? res[k] > mbo : res[k] < lbo) res[k] = -1;
                     }
                 }
 #pragma unroll
@@ -1632,8 +1604,9 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 // in-thread answers; every other key holds -1 until resolved below
 #pragma unroll
                 for (int q4 = 0; q4 < IPT / 4; q4++)
-                    *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) =
-                        make_int4(res[4 * q4], res[4 * q4 + 1], res[4 * q4 + 2], res[4 * q4 + 3]);
+                    *reinterpret_cast<int4*>(&O[swz(chunk(4 * q4))]) =
+                        make_int4(res[in_chunk(4 * q4)], res[in_chunk(4 * q4 + 1)], res[in_chunk(4 * q4 + 2)],
+                                  res[in_chunk(4 * q4 + 3)]);
             }
             // ---- 3. lane suffix minima, minima over lanes, the tile's strict suffix minima --
             T lmin, tab[5];
@@ -1719,7 +1692,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             }
             // A lane's listed keys do not increase: when no earlier lane qualifies for its
             // first, none does for any.  No such key at all (ramps): nothing to query.
-            const T q1 = V[ks(lane * IPT + (IPT - 1 - (31 - __clz(umask | 1u))))];
+            const T q1 = key(lane * IPT + (IPT - 1 - (31 - __clz(umask | 1u))));
             if (!__any_sync(FULL, umask && lane > 0 && lt<INCL>(before, q1))) {
                 smask = umask;
                 xtot = xoff = 0;
@@ -1727,7 +1700,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 // More than a round of keys: those no earlier lane qualifies for (most of
                 // them, when keys fall) need no query.
 #pragma unroll
-                for (int k = 0; k < IPT; k++) smask = (smask << 1) | (lane > 0 && lt<INCL>(before, V[ks(lane * IPT + k)]) ? 0u : 1u);
+                for (int k = 0; k < IPT; k++) smask = (smask << 1) | (lane > 0 && lt<INCL>(before, key(lane * IPT + k)) ? 0u : 1u);
                 smask &= umask;
                 xoff = warp_excl_sum(__popc(umask ^ smask), xtot);
             }
@@ -1745,7 +1718,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     }
 #pragma unroll
                     for (int i2 = 0; i2 < NQ; i2++) {
-                        q[i2] = V[ks(e[i2])];
+                        q[i2] = key(e[i2]);
                         pl[i2] = e[i2] / IPT;  // slot of the lane before the key's
                     }
                     // invariant: the answer's slot is <= pl and after each step pl - slot < 2^k;
@@ -1777,7 +1750,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
 #pragma unroll
                     for (int i2 = 0; i2 < NQ; i2++) {
                         const bool out = act[i2] && pl[i2] <= 0;
-                        if (act[i2] && !out) O[swz(e[i2])] = tile_base - rel + pb[i2] + j[i2];
+                        if (act[i2] && !out) O[swz(at(e[i2]))] = mirror(tile_base - rel + pb[i2] + j[i2]);
                         const unsigned om = __ballot_sync(FULL, out);
                         if (out) sList[ns + __popc(om & ((1u << lane) - 1u))] = (int16_t)e[i2];
                         ns += __popc(om);
@@ -1803,7 +1776,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             for (int b0 = 0; b0 < ns; b0 += 32) {
                 const bool act = b0 + lane < ns;
                 const int e = act ? (int)sList[b0 + lane] : 0;
-                const T q = V[ks(e)];
+                const T q = key(e);
                 int ans = -1;
                 if (__any_sync(FULL, act && has_rmin && lt<INCL>(rmin, q))) {
                     int lo = -1;  // the topmost qualifying entry of the window
@@ -1827,7 +1800,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         }
                     }
                 }
-                if (act && ans >= 0) O[swz(e)] = SEG && one_seg ? seg_rel(ans, rel) : ans;
+                if (act && ans >= 0) O[swz(at(e))] = SEG && one_seg ? seg_rel(ans, rel) : mirror(ans);
                 const bool miss = act && ans < 0;
                 if (__any_sync(FULL, miss)) {
                     const bool capd = miss && has_rmin && lt<INCL>(rmin, q);
@@ -1923,7 +1896,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     const unsigned all = (2u << (IPT - 1)) - 1u;
                     if (__all_sync(FULL, fmask == (k0 <= 0 ? all : k0 >= IPT ? 0u : all & (all << k0)))) {
                         for (int i2 = max(0, tot - K) + lane; i2 < tot; i2 += 32) {
-                            sStkV[(keep + i2) & (K - 1)] = V[ks(WT - tot + i2)];
+                            sStkV[(keep + i2) & (K - 1)] = key(WT - tot + i2);
                             sStkP[(keep + i2) & (K - 1)] = tile_base + WT - tot + i2;
                         }
                         m = 0;
@@ -1934,7 +1907,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     const int k = __ffs(m) - 1;
                     m &= m - 1;
                     if (idx >= newtop - K) {
-                        sStkV[idx & (K - 1)] = V[ks(lane * IPT + k)];
+                        sStkV[idx & (K - 1)] = key(lane * IPT + k);
                         sStkP[idx & (K - 1)] = lb + k;
                     }
                     idx++;
