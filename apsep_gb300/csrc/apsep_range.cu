@@ -49,7 +49,12 @@ cudaError_t range_prepare(int cfg) {
     int per_sm = 0;  // the smallest over the three modes, so every run fits
     e = prepare_mode<false, true>(cfg, &per_sm);
     if (e != cudaSuccess) return e;
-    e = prepare_segmented(cfg, &per_sm);
+    if (cfg == 0) {  // batches have their own CTA shape in this configuration
+        int seg_per_sm = 0;
+        e = prepare_segmented(cfg, &seg_per_sm);
+    } else {
+        e = prepare_segmented(cfg, &per_sm);
+    }
     if (e != cudaSuccess) return e;
     e = prepare_view(cfg, &per_sm);
     if (e != cudaSuccess) return e;

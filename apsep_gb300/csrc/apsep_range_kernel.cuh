@@ -64,16 +64,17 @@ template <int KB> constexpr int kStagesOf = KB == 8 ? 3 : 2;
 // Range-stack entries kept per warp.  Random keys leave ~ln(range) suffix minima
 // (10 of 13,800 keys), a random walk ~sqrt(range) (130): with 64 entries every
 // second range of a walk dropped some and sent its keys to phase 2 as capped.
-template <int KB> constexpr int kStackCapOf = KB == 8 ? 128 : 256;
+// (LEAN: the batches' 20-warp CTAs, whose shared memory leaves 128 entries.)
+template <int KB, bool LEAN> constexpr int kStackCapOf = KB == 8 || LEAN ? 128 : 256;
 constexpr int kUpKeep = 64;     // entries a wholly increasing tile leaves on the stack
 constexpr int kXQueries = 3;    // cross-lane queries per lane and round (32 * 3 keys per round)
 // Deferred keys listed in shared memory per range (a random walk's prefix
 // minima, ~sqrt(range) of them, fit; 8-byte keys: what shared memory leaves).
-template <int KB> constexpr int kDefCapOf = KB == 8 ? 128 : 192;
+template <int KB, bool LEAN> constexpr int kDefCapOf = LEAN ? 64 : KB == 8 ? 128 : 192;
 constexpr int kCapCap = 32;     // capped keys listed in shared memory per range
 
 // Shared memory of one warp (KB: bytes per key).
-template <int IPT, int KB = 4>
+template <int IPT, int KB = 4, bool LEAN = false>
 struct WLayout {
     static constexpr int WT = 32 * IPT;                              // keys per warp tile
     static constexpr size_t kV = 0;                                   // T[S][WT], swizzled (TMA dst)
@@ -81,10 +82,10 @@ struct WLayout {
     static constexpr size_t kSM = kO + (size_t)WT * 4;                // T[WT], swizzled: lane suffix minima
     static constexpr size_t kList = kSM + (size_t)WT * KB;            // int16[WT]: X keys in order
     static constexpr size_t kStkV = kList + (size_t)WT * 2;           // T[K]
-    static constexpr size_t kStkP = kStkV + (size_t)kStackCapOf<KB> * KB;   // int32[K]
-    static constexpr size_t kDefP = kStkP + (size_t)kStackCapOf<KB> * 4;    // int32[kDefCap]
-    static constexpr size_t kDefV = kDefP + (size_t)kDefCapOf<KB> * 4;  // T[kDefCap]
-    static constexpr size_t kCapP = kDefV + (size_t)kDefCapOf<KB> * KB;  // int32[kCapCap]
+    static constexpr size_t kStkP = kStkV + (size_t)kStackCapOf<KB, LEAN> * KB;   // int32[K]
+    static constexpr size_t kDefP = kStkP + (size_t)kStackCapOf<KB, LEAN> * 4;    // int32[kDefCap]
+    static constexpr size_t kDefV = kDefP + (size_t)kDefCapOf<KB, LEAN> * 4;  // T[kDefCap]
+    static constexpr size_t kCapP = kDefV + (size_t)kDefCapOf<KB, LEAN> * KB;  // int32[kCapCap]
     static constexpr size_t kCapS = kCapP + (size_t)kCapCap * 4;      // int32[kCapCap]: segment starts
     static constexpr size_t kPad = (kCapS + (size_t)kCapCap * 4 + 15) / 16 * 16;  // T[4]: pads (lane 0's earlier keys)
     static constexpr size_t kBar = kPad + 4 * KB;  // uint64[S]
@@ -96,8 +97,8 @@ struct WLayout {
     static_assert(kStkV % 8 == 0 && kDefV % 8 == 0, "8-byte keys need 8-byte aligned arrays");
 };
 
-template <int IPT, int WPC, int KB = 4>
-constexpr size_t kernel_smem_bytes() { return WLayout<IPT, KB>::kBytes * WPC + 1024 + 64; }  // + CTA words
+template <int IPT, int WPC, int KB = 4, bool LEAN = false>
+constexpr size_t kernel_smem_bytes() { return WLayout<IPT, KB, LEAN>::kBytes * WPC + 1024 + 64; }  // + CTA words
 
 __device__ __forceinline__ uint32_t make_tag(uint32_t epoch, uint32_t flag) { return (epoch << 2) | flag; }
 
@@ -468,10 +469,12 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
 // start order), so no wait depends on a warp that may not start.  Every wait
 // is bounded and reports ERR_LOOKBACK_TIMEOUT when it gives up.
 // ---------------------------------------------------------------------------
-// A launch of at most kDirectRanges ranges skips the global step: range r polls
-// the tagged minima of the ranges before it directly (a few words), which ends
-// sooner than waiting for every range of the launch to publish.
-constexpr int kDirectRanges = 256;
+// A launch of at most kDirectRanges ranges skips the count: range r polls
+// the tagged minima of the ranges before it directly (two words a lane), which ends
+// sooner than waiting for every range of the launch to publish (32 ranges 7.9
+// against 8.9 us a run, 64 ranges 8.7 against 9.5); with 256 ranges the pollers'
+// own traffic costs more (12.3 against 10.2 us).
+constexpr int kDirectRanges = 64;
 
 template <typename T>
 __device__ void range_publish(int r, uint32_t epoch, T rmin, const RangeArgs& a) {
@@ -597,13 +600,13 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, int* sRe
 // lane) then cost phase 1 none (inlined, the 8-byte kernels spilled there: 125 ->
 // 142 us at 2^24 int64 keys).
 // ---------------------------------------------------------------------------
-template <typename T, int IPT, bool INCL, bool SEG, int MAPF, int OUTM, bool REV>
+template <typename T, int IPT, bool INCL, bool SEG, bool LEAN, int MAPF, int OUTM, bool REV>
 __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, const int r, const int t0, const int t1,
                                     const int def_total, const int cap_total, const int first_start, const T P,
                                     const bool has_p, const T win) {
     constexpr int KB = (int)sizeof(T);
-    using L = WLayout<IPT, KB>;
-    constexpr int WT = L::WT, W = WT / 32, RPT = W * KB / 4, MW = kMaxTileKeys / 32, kDefCap = kDefCapOf<KB>;
+    using L = WLayout<IPT, KB, LEAN>;
+    constexpr int WT = L::WT, W = WT / 32, RPT = W * KB / 4, MW = kMaxTileKeys / 32, kDefCap = kDefCapOf<KB, LEAN>;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr bool OUT64 = OUTM == OUT_I64;
     const int lane = threadIdx.x & 31;
@@ -891,24 +894,30 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
 // land -- and writes each answer mirrored back, n - 1 - answer (-1 for none)
 // at element n - 1 - position: the next smaller key, in one run.
 
+// Batches of 4-byte keys in 512-key tiles: less shared memory per warp, 20 warps per
+// SM in configuration 0 (the segmented unit launches it so).
+template <typename T, int IPT, bool SEG, bool EP>
+constexpr bool kIsLean = SEG && !EP && IPT == 16 && sizeof(T) == 4;
+
 // 16 warps per SM in every configuration: without the bound the 4-warp CTAs took
 // 205 registers a thread and 8 warps fitted; with it, and a deferred list that
 // lets four of their CTAs share an SM, 2^20 random-walk keys 34.7 -> 28.5 us.
 template <typename T, int IPT, int WPC, bool INCL, bool SEG, bool EP, int MAPF = KMAP_NONE, int OUTM = OUT_I32,
           bool REV = false>
-__global__ void __launch_bounds__(WPC * 32, 16 / WPC)
+__global__ void __launch_bounds__(WPC * 32, WPC > 8 ? 1 : 16 / WPC)
 apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_constant__ CUtensorMap map_out,
                  const RangeArgs a) {
     constexpr int KB = (int)sizeof(T);  // bytes per key
-    using L = WLayout<IPT, KB>;
+    constexpr bool LEAN = kIsLean<T, IPT, SEG, EP>;
+    using L = WLayout<IPT, KB, LEAN>;
     constexpr int WT = L::WT;      // keys per warp tile
     constexpr int W = WT / 32;     // 32-key chunks (and answer TMA rows) per warp tile
     constexpr int RPT = W * KB / 4;  // key TMA rows (128 bytes) per warp tile
     static_assert(KB == 4 || (KB == 8 && IPT == 8), "8-byte keys run with 8 keys per lane");
     constexpr int TPC = 32 / IPT;  // lanes per chunk
-    constexpr int K = kStackCapOf<KB>;
+    constexpr int K = kStackCapOf<KB, LEAN>;
     constexpr int kStages = kStagesOf<KB>;
-    constexpr int kDefCap = kDefCapOf<KB>;
+    constexpr int kDefCap = kDefCapOf<KB, LEAN>;
     constexpr int MW = kMaxTileKeys / 32;  // flag-mask words per tile in global
     static_assert(IPT == 8 || IPT == 16, "IPT must be 8 or 16");
     auto ks = [](int e) { return kswz<KB>(e); };  // swizzled index of key e in V / sSM
@@ -1953,7 +1962,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
         range_prefix<T>(r, epoch, a, sCta + 2, P, has_p, win);
         __syncwarp();  // lane 0's acquire and wait before every lane's reads and writes
 
-        phase2<T, IPT, INCL, SEG, MAPF, OUTM, REV>(a, wsm, r, t0, t1, def_total, cap_total, first_start, P, has_p, win);
+        phase2<T, IPT, INCL, SEG, LEAN, MAPF, OUTM, REV>(a, wsm, r, t0, t1, def_total, cap_total, first_start, P, has_p, win);
     }
 
     // ---- run bookkeeping: the last warp resets the control block --------------------------
@@ -1985,7 +1994,7 @@ template <typename T, int IPT, int WPC, bool INCL, bool SEG, bool EP, int MAPF =
           bool REV = false>
 inline cudaError_t launch_t(RangeArgs& a, const CUtensorMap& mi, const CUtensorMap& mo, cudaStream_t st,
                             int max_warps) {
-    constexpr size_t smem = kernel_smem_bytes<IPT, WPC, (int)sizeof(T)>();
+    constexpr size_t smem = kernel_smem_bytes<IPT, WPC, (int)sizeof(T), kIsLean<T, IPT, SEG, EP>>();
     int tpr = (a.num_tiles + max_warps - 1) / max_warps;
     if (tpr < 1) tpr = 1;
     a.tiles_per_range = tpr;
@@ -1997,7 +2006,7 @@ inline cudaError_t launch_t(RangeArgs& a, const CUtensorMap& mi, const CUtensorM
 template <typename T, int IPT, int WPC, bool INCL, bool SEG, bool EP, int MAPF = KMAP_NONE, int OUTM = OUT_I32,
           bool REV = false>
 inline cudaError_t prepare_t(int* ctas_per_sm) {
-    constexpr size_t smem = kernel_smem_bytes<IPT, WPC, (int)sizeof(T)>();
+    constexpr size_t smem = kernel_smem_bytes<IPT, WPC, (int)sizeof(T), kIsLean<T, IPT, SEG, EP>>();
     auto k = apse_warp_kernel<T, IPT, WPC, INCL, SEG, EP, MAPF, OUTM, REV>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
@@ -2007,6 +2016,9 @@ inline cudaError_t prepare_t(int* ctas_per_sm) {
     if (*ctas_per_sm == 0 || n < *ctas_per_sm) *ctas_per_sm = n;
     return cudaSuccess;
 }
+
+// Warps per CTA of a batch in configuration 0.
+constexpr int kSegWarps = 20;
 
 // Shared-memory attributes and occupancy of every kernel of one mode and
 // configuration (the smallest CTAs-per-SM over the four key/comparison types).
@@ -2022,7 +2034,9 @@ inline cudaError_t prepare_mode(int cfg, int* per_sm) {
             if (rr[q] != cudaSuccess) return rr[q];                                    \
     }
     switch (cfg) {
-    case 0: P_(16, 16); break;
+    case 0:
+        if constexpr (SEG && !EP) P_(16, kSegWarps) else P_(16, 16);
+        break;
     case 1: P_(8, 8); break;
     case 2: P_(16, 8); break;
     case 3: P_(8, 16); break;
@@ -2045,7 +2059,12 @@ inline cudaError_t launch_mode(int dtype, int incl, int cfg, RangeArgs& a, const
         return incl ? launch_t<float, IPT, WPC, true, SEG, EP>(a, mi, mo, st, max_warps)    \
                     : launch_t<float, IPT, WPC, false, SEG, EP>(a, mi, mo, st, max_warps);
     switch (cfg) {
-    case 0: L_(16, 16);
+    case 0:
+        if constexpr (SEG && !EP) {
+            L_(16, kSegWarps)
+        } else {
+            L_(16, 16)
+        }
     case 1: L_(8, 8);
     case 2: L_(16, 8);
     case 3: L_(8, 16);

@@ -17,8 +17,27 @@ cudaError_t prepare_segmented(int cfg, int* ctas_per_sm) { return prepare_mode<t
 cudaError_t launch_range_segmented(int dtype, int incl, int cfg, RangeArgs& a, const CUtensorMap& mi,
                                    const CUtensorMap& mo, cudaStream_t st) {
     int max_warps = 0;
-    const cudaError_t e = range_max_warps(cfg, &max_warps);
+    cudaError_t e = range_max_warps(cfg, &max_warps);
     if (e != cudaSuccess) return e;
+    if (cfg == 0) {
+        // One CTA of 20 warps per SM instead of 16: a batch has no whole-tile paths for
+        // sorted keys, which lose to the finer ranges (2^25 descending 54 -> 58 us as a
+        // single array), and hides more of its dependent steps: 1.03e8 keys in 1024
+        // arrays, mixed 410 -> 379 us, uniform 316 -> 305, sawtooth 338 -> 305.  Below
+        // six tiles a range the finer ranges cost more than they hide (8.2e6 keys 69.6
+        // us; 1.35e7 keys 95.0): those take configuration 2, 16 warps per SM in two CTAs
+        // (67.0; 97.7).
+        int dev = 0, sms = 0;
+        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        const int seg_warps = sms * kSegWarps < kMaxRanges ? sms * kSegWarps : kMaxRanges;
+        if (a.num_tiles >= 6 * seg_warps) {
+            max_warps = seg_warps;
+        } else {
+            cfg = 2;  // the same 512-key tiles
+            if ((e = range_max_warps(cfg, &max_warps)) != cudaSuccess) return e;
+        }
+    }
     if (!a.offsets || a.nseg < 1) return cudaErrorInvalidValue;
     return launch_mode<true, false>(dtype, incl, cfg, a, mi, mo, st, max_warps);
 }
