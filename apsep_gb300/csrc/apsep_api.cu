@@ -220,7 +220,8 @@ apsep_status run_impl(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n
     DeviceGuard g(p->device);
     if (!g.ok) return APSEP_ECUDA;
     if (wide(p->dtype)) {  // 8-byte keys: TMA when both arrays are 16-byte aligned
-        const int B = kWideTileKeys, key_rows_per_tile = B * 8 / 128;
+        const int B = wide_tile_keys(n, offsets != nullptr), key_rows_per_tile = B * 8 / 128;
+        if (B == 0) return APSEP_ECUDA;
         int rows = (int)(n / 16);  // 128-byte rows of keys
         CUtensorMap mi, mo;
         memset(&mi, 0, sizeof(mi));
@@ -247,7 +248,7 @@ apsep_status run_impl(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n
         a.s = p->rs;
         p->dbg_skip_range = -1;
         p->dbg_spin_limit = 0;
-        const cudaError_t e = launch_range_wide(p->dtype, cmp == APSEP_LE ? 1 : 0, a, mi, mo, (cudaStream_t)stream);
+        const cudaError_t e = launch_range_wide(p->dtype, cmp == APSEP_LE ? 1 : 0, B, a, mi, mo, (cudaStream_t)stream);
         return e == cudaSuccess ? APSEP_OK : APSEP_ECUDA;
     }
 

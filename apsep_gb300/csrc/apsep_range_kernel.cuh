@@ -56,11 +56,11 @@
 
 namespace apsep {
 
-// TMA ring depth per warp (tiles): two for 4-byte keys, one landing while one is
-// worked on (a third measured no gain, and its shared memory holds the longer
-// stack and lists); three for 8-byte keys, whose tiles are 256 keys (ascending
-// float64 keys, 2^26 of them: 207 us with two, 173 us with three).
-template <int KB> constexpr int kStagesOf = KB == 8 ? 3 : 2;
+// TMA ring depth per warp (tiles): two, one landing while one is worked on (a
+// third measured no gain for 4-byte keys, and its shared memory holds the longer
+// stack and lists); three for 8-byte keys in tiles of 256 (ascending float64
+// keys, 2^26 of them: 207 us with two, 173 us with three).
+template <int KB, int IPT> constexpr int kStagesOf = KB == 8 && IPT == 8 ? 3 : 2;
 // Range-stack entries kept per warp.  Random keys leave ~ln(range) suffix minima
 // (10 of 13,800 keys), a random walk ~sqrt(range) (130): with 64 entries every
 // second range of a walk dropped some and sent its keys to phase 2 as capped.
@@ -70,7 +70,7 @@ constexpr int kUpKeep = 64;     // entries a wholly increasing tile leaves on th
 constexpr int kXQueries = 3;    // cross-lane queries per lane and round (32 * 3 keys per round)
 // Deferred keys listed in shared memory per range (a random walk's prefix
 // minima, ~sqrt(range) of them, fit; 8-byte keys: what shared memory leaves).
-template <int KB, bool LEAN> constexpr int kDefCapOf = LEAN ? 64 : KB == 8 ? 128 : 192;
+template <int KB, int IPT, bool LEAN> constexpr int kDefCapOf = LEAN ? 64 : KB == 4 ? 192 : IPT == 8 ? 128 : 96;
 constexpr int kCapCap = 32;     // capped keys listed in shared memory per range
 
 // Shared memory of one warp (KB: bytes per key).
@@ -78,18 +78,18 @@ template <int IPT, int KB = 4, bool LEAN = false>
 struct WLayout {
     static constexpr int WT = 32 * IPT;                              // keys per warp tile
     static constexpr size_t kV = 0;                                   // T[S][WT], swizzled (TMA dst)
-    static constexpr size_t kO = kV + (size_t)kStagesOf<KB> * WT * KB;      // int32[WT], swizzled (TMA src)
+    static constexpr size_t kO = kV + (size_t)kStagesOf<KB, IPT> * WT * KB;      // int32[WT], swizzled (TMA src)
     static constexpr size_t kSM = kO + (size_t)WT * 4;                // T[WT], swizzled: lane suffix minima
     static constexpr size_t kList = kSM + (size_t)WT * KB;            // int16[WT]: X keys in order
     static constexpr size_t kStkV = kList + (size_t)WT * 2;           // T[K]
     static constexpr size_t kStkP = kStkV + (size_t)kStackCapOf<KB, LEAN> * KB;   // int32[K]
     static constexpr size_t kDefP = kStkP + (size_t)kStackCapOf<KB, LEAN> * 4;    // int32[kDefCap]
-    static constexpr size_t kDefV = kDefP + (size_t)kDefCapOf<KB, LEAN> * 4;  // T[kDefCap]
-    static constexpr size_t kCapP = kDefV + (size_t)kDefCapOf<KB, LEAN> * KB;  // int32[kCapCap]
+    static constexpr size_t kDefV = kDefP + (size_t)kDefCapOf<KB, IPT, LEAN> * 4;  // T[kDefCap]
+    static constexpr size_t kCapP = kDefV + (size_t)kDefCapOf<KB, IPT, LEAN> * KB;  // int32[kCapCap]
     static constexpr size_t kCapS = kCapP + (size_t)kCapCap * 4;      // int32[kCapCap]: segment starts
     static constexpr size_t kPad = (kCapS + (size_t)kCapCap * 4 + 15) / 16 * 16;  // T[4]: pads (lane 0's earlier keys)
     static constexpr size_t kBar = kPad + 4 * KB;  // uint64[S]
-    static constexpr size_t kFlag = kBar + (size_t)kStagesOf<KB> * 8;  // int32: phase 2's group minima are staged
+    static constexpr size_t kFlag = kBar + (size_t)kStagesOf<KB, IPT> * 8;  // int32: phase 2's group minima are staged
     static constexpr size_t kEnd = kFlag + 8;
     static constexpr size_t kBytes = (kEnd + 1023) / 1024 * 1024;     // keeps every warp 1024-aligned
     static_assert(kO % 1024 == 0 && kSM % 1024 == 0 && (WT * KB) % 1024 == 0,
@@ -606,7 +606,7 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
                                     const bool has_p, const T win) {
     constexpr int KB = (int)sizeof(T);
     using L = WLayout<IPT, KB, LEAN>;
-    constexpr int WT = L::WT, W = WT / 32, RPT = W * KB / 4, MW = kMaxTileKeys / 32, kDefCap = kDefCapOf<KB, LEAN>;
+    constexpr int WT = L::WT, W = WT / 32, RPT = W * KB / 4, MW = kMaxTileKeys / 32, kDefCap = kDefCapOf<KB, IPT, LEAN>;
     constexpr unsigned FULL = 0xffffffffu;
     constexpr bool OUT64 = OUTM == OUT_I64;
     const int lane = threadIdx.x & 31;
@@ -913,11 +913,10 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     constexpr int WT = L::WT;      // keys per warp tile
     constexpr int W = WT / 32;     // 32-key chunks (and answer TMA rows) per warp tile
     constexpr int RPT = W * KB / 4;  // key TMA rows (128 bytes) per warp tile
-    static_assert(KB == 4 || (KB == 8 && IPT == 8), "8-byte keys run with 8 keys per lane");
     constexpr int TPC = 32 / IPT;  // lanes per chunk
     constexpr int K = kStackCapOf<KB, LEAN>;
-    constexpr int kStages = kStagesOf<KB>;
-    constexpr int kDefCap = kDefCapOf<KB, LEAN>;
+    constexpr int kStages = kStagesOf<KB, IPT>;
+    constexpr int kDefCap = kDefCapOf<KB, IPT, LEAN>;
     constexpr int MW = kMaxTileKeys / 32;  // flag-mask words per tile in global
     static_assert(IPT == 8 || IPT == 16, "IPT must be 8 or 16");
     auto ks = [](int e) { return kswz<KB>(e); };  // swizzled index of key e in V / sSM
