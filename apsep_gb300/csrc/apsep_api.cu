@@ -410,6 +410,7 @@ apsep_status plan_run_out64(apsep_plan* p, const void* d_in, int64_t* d_out, int
     if (chunk_min) a.s.chunk_min = chunk_min;
     a.d_out64 = d_out;
     a.out_base = out_base;
+    a.unanswered64 = out_base > 0 ? UNRESOLVED64 : -1;  // (-1: nothing before the first piece)
     p->dbg_skip_range = -1;
     p->dbg_spin_limit = 0;
     const cudaError_t e = launch_range_out64(p->dtype, cmp == APSEP_LE ? 1 : 0, a, mi, (cudaStream_t)stream);

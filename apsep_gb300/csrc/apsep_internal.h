@@ -137,10 +137,12 @@ struct RangeArgs {
     RangeScratch s;
     int64_t* d_out64 = nullptr;  // int64 answers (the int64-position path's kernels): out_base + answer
     int64_t out_base = 0;
+    int64_t unanswered64 = -1;  // what a key that no key of the run answers reads there
 };
 
 // Runs with int64 answers (RangeArgs::d_out64): a key that no key of the run
-// answers reads UNRESOLVED64, and a tile whose keys are all unanswered within
+// answers reads RangeArgs::unanswered64 (UNRESOLVED64 when keys before the run may
+// answer it, else -1), and a tile whose keys are all unanswered within
 // their range is not written at all; its tile_flag word carries
 // TILE_NOT_STORED (phase 2 still writes the keys that it answers).
 constexpr int64_t UNRESOLVED64 = -2;
@@ -194,7 +196,7 @@ cudaError_t prepare_segmented(int cfg, int* ctas_per_sm);
 cudaError_t range_max_warps(int cfg, int* warps);  // persistent warps of one launch, current device
 // A single array (no view head) with int64 answers a.out_base + answer into
 // a.d_out64 (4-byte keys in configuration 0, 8-byte keys in theirs); flagged keys
-// get UNRESOLVED64 and all-deferred tiles are not written (TILE_NOT_STORED).
+// get a.unanswered64 and all-deferred tiles are not written (TILE_NOT_STORED).
 cudaError_t launch_range_out64(int dtype, int incl, RangeArgs& a, const CUtensorMap& map_in, cudaStream_t st);
 // A single array (no view head, 4-byte keys) through the order-reversing key
 // map in configuration 0: previous-greater answers (int32), or with span != 0

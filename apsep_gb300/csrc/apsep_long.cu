@@ -209,17 +209,30 @@ __global__ void __launch_bounds__(kPrologue)
 }
 
 // The fix-up of piece [b0, b1) after its engine run (int64 answers): every key
-// the run left unanswered gets its answer before b0, or -1.  One warp per 32
-// tiles of the run at a time: a ballot over their flag words, then each flagged
-// tile in turn.  A tile written by the engine names its unanswered keys by its
-// mask words and UNRESOLVED64; a tile left unwritten (TILE_NOT_STORED: its keys
-// are all prefix minima of their range, and never increase) has its keys
-// answered by phase 2 exactly when the range's prefix minimum qualifies.
+// the run left unanswered gets its answer before b0, or -1.  One warp per
+// `tiles_per_warp` tiles of the run at a time: a ballot over their flag words,
+// then each flagged tile in turn.  A tile written by the engine names its
+// unanswered keys by its mask words and UNRESOLVED64; a tile left unwritten
+// (TILE_NOT_STORED: its keys are all prefix minima of their range, and never
+// increase) has its keys answered by phase 2 exactly when the range's prefix
+// minimum qualifies.
+//
+// Bound by chains of dependent L2 reads (flags, masks, answers, then a query's
+// descent), so: a warp takes as few tiles as still occupy the chip; a flagged
+// tile's answers are read in one go; and a query's answer serves the smaller keys
+// after it: with key x at p the nearest before b0 to qualify for q, a key q2 <= q
+// that x qualifies for has the answer p (what lies between did not qualify for
+// q).  Unanswered keys never increase along a piece, so the first one asks for
+// all.  With a query for every key, 32 tiles a warp and chunk after chunk the whole
+// call took, int32 keys: 2^22 uniform in four pieces 405 us (now 117), in one 74 (36);
+// a walk in four 982 (261); 40.8M descending in four pieces, a key in 50,000 out of
+// place, 31.2 ms (0.33); 2^27 in two: uniform 549 (546), 16 values 1556 (778; 953 when
+// the first piece's unanswered keys were still marked and rewritten here).
 template <typename K, bool MAPF, bool INCL>
 __global__ void __launch_bounds__(kThreads)
     fixup_kernel(const K* __restrict__ keys, int64_t* __restrict__ out, int64_t b0, int64_t b1, Levels<K> lv,
                  const Frontier<K>* __restrict__ fr, bool look_before, const K* __restrict__ rpre, RangeScratch rs,
-                 const K* __restrict__ cmin, int num_tiles, int tiles_per_range, uint32_t* err) {
+                 const K* __restrict__ cmin, int num_tiles, int tiles_per_range, int tiles_per_warp, uint32_t* err) {
     constexpr int WT = sizeof(K) == 8 ? kWideTileKeys : 512;  // keys per engine tile
     constexpr int W = WT / 32;                                 // 32-key chunks per tile
     constexpr int MW = kMaxTileKeys / 32;                      // mask words per tile
@@ -242,58 +255,74 @@ __global__ void __launch_bounds__(kThreads)
     const K* tmin = (const K*)rs.tile_min;
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
+    // the last query: key cx at position cp answers cq (cp < 0: none yet)
+    K cq = KeyTraits<K>::pad(), cx = KeyTraits<K>::pad();
+    int64_t cp = -1;
+    // cp is the answer of every key between lo and hi
+    auto served = [&](K lo, K hi) { return cp >= 0 && lt<INCL>(cx, lo) && !lt<false>(cq, hi); };
+    auto put = [&](int64_t i, int64_t o) { __stcs(reinterpret_cast<long long*>(out) + i, (long long)o); };
     // the answer before b0 of the keys `need` marks (uniform call), written
     auto resolve = [&](bool need, K q, int64_t i) {
         int64_t o = -1;
-        int lvl = -1;  // the nearest frontier whose minimum qualifies
-        if (need && has && lt<INCL>(pm, q)) {
-            for (int l = 0; l < kLevels; l++)
-                if (((has >> l) & 1u) && lt<INCL>(su[l], q)) {
-                    lvl = l;
-                    break;
-                }
+        bool open = need && has && lt<INCL>(pm, q);  // an answer is still to be found
+        if (open && served(q, q)) {
+            o = cp;
+            open = false;
         }
-        unsigned qm = __ballot_sync(FULL, lvl >= 0);
-        while (qm) {
+        unsigned qm;
+        while ((qm = __ballot_sync(FULL, open))) {
             const int src = __ffs(qm) - 1;
-            qm &= qm - 1;
             const K qs = __shfl_sync(FULL, q, src);
-            const int l = __shfl_sync(FULL, lvl, src);
+            int l = 0;  // the nearest frontier whose minimum qualifies (pm is one of them)
+            while (l < kLevels - 1 && (!((has >> l) & 1u) || !lt<INCL>(su[l], qs))) l++;
             const int64_t ans = answer_before<K, MAPF, INCL>(keys, lv, qs, l, b0, err);
-            if (lane == src) o = ans;
+            cq = qs;
+            cp = ans;
+            if (ans >= 0) cx = entry<K, MAPF>(keys, lv, 0, ans);
+            if (open && (lane == src || served(q, q))) {
+                o = ans;
+                open = false;
+            }
         }
-        if (need) __stcs(reinterpret_cast<long long*>(out) + i, (long long)o);
+        if (need) put(i, o);
     };
-    const int ngroups = (num_tiles + 31) >> 5;
+    const int ngroups = (num_tiles + tiles_per_warp - 1) / tiles_per_warp;
     for (int tg = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); tg < ngroups; tg += nw) {
-        const int tl = (tg << 5) + lane;
-        const uint32_t myf = tl < num_tiles ? __ldcg(&rs.tile_flag[tl]) : 0u;
+        const int tl = tg * tiles_per_warp + lane;
+        const uint32_t myf = lane < tiles_per_warp && tl < num_tiles ? __ldcg(&rs.tile_flag[tl]) : 0u;
         unsigned fm = __ballot_sync(FULL, (myf & 0x3fffffffu) != 0);
         while (fm) {
             const int src = __ffs(fm) - 1;
             fm &= fm - 1;
-            const int t = (tg << 5) + src;
+            const int t = tg * tiles_per_warp + src;
             const uint32_t tf = __shfl_sync(FULL, myf, src);
+            if (!has && !(tf & TILE_NOT_STORED)) continue;  // nothing before the piece: the run's -1 stands
             const int r = t / tiles_per_range;
             const bool has_p = r > 0;  // the piece's ranges before r
             const K P = has_p ? rpre[r] : KeyTraits<K>::pad();
             const int64_t tb = b0 + (int64_t)t * WT;  // the tile's first position
             if (tf & TILE_NOT_STORED) {
-                // chunk c's keys are at most the minimum of chunk c - 1, and chunk
-                // 0's at most the previous tile's minimum (the range's minimum
-                // before the tile is >= its first key); lane c holds chunk c's bound
-                bool dec = false;
-                if (lane < W && (lane > 0 || t % tiles_per_range != 0)) {
-                    const K ub = lane > 0 ? __ldcg(&cmin[(size_t)t * W + lane - 1]) : __ldcg(&tmin[t - 1]);
-                    dec = !(has_p && lt<INCL>(P, ub)) && !(has && lt<INCL>(pm, ub));
-                }
-                const unsigned decm = __ballot_sync(FULL, dec);
+                // lane c bounds chunk c's keys: from its minimum up to the minimum of
+                // chunk c - 1, and chunk 0's up to the previous tile's minimum (the
+                // range's minimum before the tile is >= its first key)
+                const bool bounded = lane < W && (lane > 0 || t % tiles_per_range != 0);
+                K ub = KeyTraits<K>::pad(), lb = ub;
+                if (lane < W) lb = __ldcg(&cmin[(size_t)t * W + lane]);
+                if (bounded) ub = lane > 0 ? __ldcg(&cmin[(size_t)t * W + lane - 1]) : __ldcg(&tmin[t - 1]);
+                const bool none_p = bounded && !(has_p && lt<INCL>(P, ub));  // phase 2 answered no key of the chunk
+                const unsigned decm = __ballot_sync(FULL, none_p && !(has && lt<INCL>(pm, ub)));
+                const unsigned donem = __ballot_sync(FULL, has_p && lt<INCL>(P, lb));  // ... and here every key
 #pragma unroll 1
                 for (int c = 0; c < W; c++) {
+                    if ((donem >> c) & 1u) continue;
                     const int64_t i = tb + 32 * c + lane;
                     const bool valid = i < b1;
                     if ((decm >> c) & 1u) {  // no key of the chunk has an answer
-                        if (valid) __stcs(reinterpret_cast<long long*>(out) + i, -1ll);
+                        if (valid) put(i, -1);
+                        continue;
+                    }
+                    if ((__ballot_sync(FULL, none_p && served(lb, ub)) >> c) & 1u) {  // they share the last one
+                        if (valid) put(i, cp);
                         continue;
                     }
                     const K q = valid ? load_key<K, MAPF>(keys + i) : KeyTraits<K>::pad();
@@ -301,15 +330,23 @@ __global__ void __launch_bounds__(kThreads)
                 }
             } else {
                 const uint32_t mw = lane < W ? __ldcg(&rs.tile_mask[(size_t)t * MW + lane]) : 0u;
-#pragma unroll 1
-                for (int c = 0; c < W; c++) {
+                unsigned cm = __ballot_sync(FULL, mw != 0u);  // chunks with flagged keys
+                unsigned need = 0u;                           // bit c: the lane's key of chunk c is unanswered
+#pragma unroll
+                for (int c = 0; c < W; c++) {  // (all reads in flight together)
                     const uint32_t m = __shfl_sync(FULL, mw, c);
-                    if (!m) continue;
                     const int64_t i = tb + 32 * c + lane;
-                    const bool need = ((m >> lane) & 1u) && i < b1 &&
-                                      __ldcg(reinterpret_cast<const long long*>(out) + i) == (long long)UNRESOLVED64;
-                    const K q = need ? load_key<K, MAPF>(keys + i) : KeyTraits<K>::pad();
-                    resolve(need, q, i);
+                    if (((m >> lane) & 1u) && i < b1 &&
+                        __ldcg(reinterpret_cast<const long long*>(out) + i) == (long long)UNRESOLVED64)
+                        need |= 1u << c;
+                }
+                while (cm) {
+                    const int c = __ffs(cm) - 1;
+                    cm &= cm - 1;
+                    const int64_t i = tb + 32 * c + lane;
+                    const bool nd = (need >> c) & 1u;
+                    const K q = nd ? load_key<K, MAPF>(keys + i) : KeyTraits<K>::pad();
+                    resolve(nd, q, i);
                 }
             }
         }
@@ -374,11 +411,14 @@ apsep_status run_long(apsep_plan* plan, const K* keys, int64_t* out, int64_t n, 
         if (launch_pdl(prologue_kernel<K, MAPF>, 1, kPrologue, 0, st, keys, lv, b0, look, ra.s, ra.num_ranges, rpre, fr) !=
             cudaSuccess)
             return APSEP_ECUDA;
-        const int groups = (ra.num_tiles + 31) / 32;  // 32 tiles per warp and step
+        // tiles per warp and step: as few as fill the chip once (a warp's flag ballot takes 32)
+        const int resident = sms * std::max(per_sm, 1) * (kThreads / 32);
+        const int tpw = std::min(32, (ra.num_tiles + resident - 1) / resident);
+        const int groups = (ra.num_tiles + tpw - 1) / tpw;
         const int grid = (int)std::min<int64_t>(std::max<int64_t>(ceil_div(groups, kThreads / 32), 1),
                                                 (int64_t)sms * std::max(per_sm, 1));
         if (launch_pdl(fix, grid, kThreads, 0, st, keys, out, b0, b1, lv, fr, look, rpre, ra.s,
-                       (const K*)ra.s.chunk_min, ra.num_tiles, ra.tiles_per_range, &ra.s.ctr->err) != cudaSuccess)
+                       (const K*)ra.s.chunk_min, ra.num_tiles, ra.tiles_per_range, tpw, &ra.s.ctr->err) != cudaSuccess)
             return APSEP_ECUDA;
         if (!pieces || b1 == n) continue;
         // level entries that complete inside this piece (level 1 came with the run)

@@ -1,11 +1,11 @@
 // apsep_out64.cu -- the range engine with int64 answers, for the
 // int64-position path (apsep_run64): single arrays on a 16-byte boundary,
 // 4-byte keys in configuration 0 (16 warps per CTA, 512-key warp tiles),
-// 8-byte keys in their one configuration (8 warps per CTA, 256-key tiles).
+// 8-byte keys in their short tiles (8 warps per CTA, 256 keys).
 // Each piece of a long array writes out_base + answer straight into the
 // int64 output, so no int32 scratch is written and read back; keys the piece
-// leaves unanswered are marked (UNRESOLVED64, or a tile flagged as not
-// stored) for the int64-position path's fix-up.
+// leaves unanswered are marked (UNRESOLVED64; -1, the answer, in the first
+// piece; or a tile flagged as not stored) for the int64-position path's fix-up.
 #include "apsep_range_kernel.cuh"
 
 namespace apsep {

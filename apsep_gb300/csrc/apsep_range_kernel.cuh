@@ -625,10 +625,10 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
     auto seg_idx = [&](int pos) { return a.offsets ? seg_find(a.offsets, a.nseg, pos, err) : 0; };
     auto tile_full = [&](int t) { return a.tma_rows > 0 && (t + 1) * RPT <= a.tma_rows && (t > 0 || head == 0); };
     // a final answer v of position pos (phase 2); int64 answers: out_base + v, and
-    // UNRESOLVED64 for none (the key is left to the int64-position path); spans:
+    // a.unanswered64 for none (the int64-position path's mark); spans:
     // pos - v
     auto put = [&](int pos, int v) {
-        if constexpr (OUT64) a.d_out64[pos] = v >= 0 ? (int64_t)v + a.out_base : UNRESOLVED64;
+        if constexpr (OUT64) a.d_out64[pos] = v >= 0 ? (int64_t)v + a.out_base : a.unanswered64;
         else if constexpr (REV) a.d_out[a.n - 1 - pos] = v >= 0 ? a.n - 1 - v : -1;
         else if constexpr (OUTM == OUT_SPAN) a.d_out[pos] = pos - v;
         else a.d_out[pos] = v;
@@ -884,14 +884,14 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
 // f64_order, or the order-reversing flip for previous-greater queries.
 // OUTM (single arrays, no view head, except OUT_I32): OUT_I64 -- answers as
 // int64, a.out_base + answer, into a.d_out64, for the int64-position path: a
-// flagged key gets UNRESOLVED64 (phase 2 overwrites the ones it answers), and a
+// flagged key gets a.unanswered64 (phase 2 overwrites the ones it answers), and a
 // tile whose keys are all deferred is not written at all (its flag word says
 // so); the int64-position path answers what is left.  OUT_SPAN -- int32
 // position - answer (position + 1 for none): the stock span, with the flip.
 // REV (single arrays, no view head, 4-byte keys): the run sees the array
 // reversed -- tile t holds elements n - 1 - (t * WT + e), its TMA rows counted
-// from the end (n a multiple of 32) and reversed in shared memory as they
-// land -- and writes each answer mirrored back, n - 1 - answer (-1 for none)
+// from the end (n a multiple of 32) and read mirrored from shared
+// memory -- and writes each answer mirrored back, n - 1 - answer (-1 for none)
 // at element n - 1 - position: the next smaller key, in one run.
 
 // Batches of 4-byte keys in 512-key tiles: less shared memory per warp, 20 warps per
@@ -1190,7 +1190,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         const int e = j * 32 + lane;
                         if (e < valid_keys) {
                             const int o = O[swz(e)];
-                            a.d_out64[tile_base + e] = o >= 0 ? (int64_t)o + a.out_base : UNRESOLVED64;
+                            a.d_out64[tile_base + e] = o >= 0 ? (int64_t)o + a.out_base : a.unanswered64;
                         }
                     }
                     return;
