@@ -255,20 +255,39 @@ __global__ void __launch_bounds__(kThreads)
     const K* tmin = (const K*)rs.tile_min;
     const int lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    // the last query: key cx at position cp answers cq (cp < 0: none yet)
-    K cq = KeyTraits<K>::pad(), cx = KeyTraits<K>::pad();
+    // the last query: key cx at position cp answers cq (cp < 0: none yet), and the
+    // window of 32 keys up to cp: lane j holds the minimum of its entries j .. 31
+    K cq = KeyTraits<K>::pad(), cx = KeyTraits<K>::pad(), wm = KeyTraits<K>::pad();
     int64_t cp = -1;
     // cp is the answer of every key between lo and hi
     auto served = [&](K lo, K hi) { return cp >= 0 && lt<INCL>(cx, lo) && !lt<false>(cq, hi); };
+    // the window entry that answers q, -1 for none (uniform call; q <= cq): the entries
+    // whose suffix minimum qualifies are its first ones, and the last of those qualifies
+    auto in_window = [&](K q) {
+        int j = -1;
+#pragma unroll
+        for (int step = 16; step > 0; step >>= 1) {
+            const K m = __shfl_sync(FULL, wm, j + step);
+            if (lt<INCL>(m, q)) j += step;
+        }
+        const K m = __shfl_sync(FULL, wm, j + 1);
+        return lt<INCL>(m, q) ? j + 1 : j;
+    };
     auto put = [&](int64_t i, int64_t o) { __stcs(reinterpret_cast<long long*>(out) + i, (long long)o); };
     // the answer before b0 of the keys `need` marks (uniform call), written
     auto resolve = [&](bool need, K q, int64_t i) {
         int64_t o = -1;
         bool open = need && has && lt<INCL>(pm, q);  // an answer is still to be found
-        if (open && served(q, q)) {
-            o = cp;
-            open = false;
-        }
+        // the open keys that the window serves
+        auto from_window = [&]() {
+            if (cp < 0 || !__any_sync(FULL, open)) return;
+            const int j = in_window(q);
+            if (open && j >= 0 && !lt<false>(cq, q)) {
+                o = cp - 31 + j;
+                open = false;
+            }
+        };
+        from_window();
         unsigned qm;
         while ((qm = __ballot_sync(FULL, open))) {
             const int src = __ffs(qm) - 1;
@@ -278,11 +297,19 @@ __global__ void __launch_bounds__(kThreads)
             const int64_t ans = answer_before<K, MAPF, INCL>(keys, lv, qs, l, b0, err);
             cq = qs;
             cp = ans;
-            if (ans >= 0) cx = entry<K, MAPF>(keys, lv, 0, ans);
-            if (open && (lane == src || served(q, q))) {
+            const int64_t wp = ans - 31 + lane;
+            wm = wp >= 0 ? entry<K, MAPF>(keys, lv, 0, wp) : KeyTraits<K>::pad();
+            cx = __shfl_sync(FULL, wm, 31);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {  // (past the end: the lane's own value)
+                const K u = __shfl_down_sync(FULL, wm, d);
+                wm = KeyTraits<K>::vmin(wm, u);
+            }
+            if (lane == src) {
                 o = ans;
                 open = false;
             }
+            from_window();
         }
         if (need) put(i, o);
     };

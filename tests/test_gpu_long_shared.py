@@ -18,10 +18,12 @@ def _shape(kind, n, piece):
         return i // piece * (piece // 2) - i % piece
     if kind == "steps":  # long runs of equal keys, going down
         return (n - i) // 1500
+    if kind == "mountain":  # up, then down: an answer of its own for every key of the falling half
+        return np.minimum(2 * i, 2 * (n - i) - 1) + i % 7
     return keys(kind, n, n)
 
 
-@pytest.mark.parametrize("kind", ["down_few", "walk_down", "noisy_down", "falling_pieces", "steps"])
+@pytest.mark.parametrize("kind", ["down_few", "walk_down", "noisy_down", "falling_pieces", "steps", "mountain"])
 @pytest.mark.parametrize("dtype", ["int32", "float32", "int64", "float64"])
 @pytest.mark.parametrize("n,piece,off", [(70_001, 4096, 0), (70_001, 33_333, 1), (1_500_007, 511_999, 0),
                                          (3_000_000, 1 << 20, 1)])
