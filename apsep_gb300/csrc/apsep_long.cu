@@ -32,12 +32,12 @@
 //
 // The frontier minima of a piece and the prefix minima of its ranges come from
 // one small prologue kernel; the fix-up's queries are warp-cooperative (one at
-// a time per warp, every lane on one entry).  Keys that need a query are the
-// prefix minima of their piece that something before the piece qualifies for:
-// a few dozen per piece on random keys, none on descending keys; an input whose
-// every piece descends while the pieces rise makes every key a query (a few
-// dependent L2 reads each, one query at a time per warp), the slow case of
-// this path.
+// a time per warp, every lane on one entry).  Keys that need an answer here are
+// the prefix minima of their piece that something before the piece qualifies
+// for: a few dozen per piece on random keys, every key of a piece that descends
+// above what came before.  They never increase along the piece, so their
+// answers only move back, and a query's answer and the keys just before it
+// serve the keys after it too.
 #include <stdint.h>
 
 #include <type_traits>
@@ -219,15 +219,16 @@ __global__ void __launch_bounds__(kPrologue)
 //
 // Bound by chains of dependent L2 reads (flags, masks, answers, then a query's
 // descent), so: a warp takes as few tiles as still occupy the chip; a flagged
-// tile's answers are read in one go; and a query's answer serves the smaller keys
-// after it: with key x at p the nearest before b0 to qualify for q, a key q2 <= q
-// that x qualifies for has the answer p (what lies between did not qualify for
-// q).  Unanswered keys never increase along a piece, so the first one asks for
-// all.  With a query for every key, 32 tiles a warp and chunk after chunk the whole
-// call took, int32 keys: 2^22 uniform in four pieces 405 us (now 117), in one 74 (36);
-// a walk in four 982 (261); 40.8M descending in four pieces, a key in 50,000 out of
-// place, 31.2 ms (0.33); 2^27 in two: uniform 549 (546), 16 values 1556 (778; 953 when
-// the first piece's unanswered keys were still marked and rewritten here).
+// tile's answers are read in one go; and a query serves the smaller keys after it:
+// with p the nearest key before b0 to qualify for q, what lies between does not
+// qualify for any q2 <= q either, so the answer of q2 is the last of the 32 keys up
+// to p that qualifies, if one does.  Unanswered keys never increase along a piece, so
+// the first one asks for all.  With a query for every key, 32 tiles a warp and chunk
+// after chunk the whole call took, int32 keys: 2^22 uniform in four pieces 405 us (now
+// 116), in one 74 (35); a walk in four 982 (199; 260 with p alone serving others);
+// 40.8M descending in four, a key in 50,000 out of place, 31.2 ms (0.33); 2^27 in two:
+// uniform 549 (541), 16 values 1556 (790; 953 when the first piece's unanswered keys
+// were still marked and rewritten here), keys that rise and then fall 20.5 ms (1.3).
 template <typename K, bool MAPF, bool INCL>
 __global__ void __launch_bounds__(kThreads)
     fixup_kernel(const K* __restrict__ keys, int64_t* __restrict__ out, int64_t b0, int64_t b1, Levels<K> lv,
