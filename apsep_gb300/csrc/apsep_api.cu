@@ -298,28 +298,24 @@ apsep_status run_impl(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n
 
 }  // namespace
 
-apsep_status plan_run_flipped(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp, int span,
-                              void* stream) {
-    if (!p || n <= 0 || n > p->capacity || !d_in || !d_out || (cmp != APSEP_LT && cmp != APSEP_LE)) return APSEP_EINVAL;
-    if (wide(p->dtype) || (span && cmp != APSEP_LT)) return APSEP_ENOTSUP;
-    if ((uintptr_t)d_in % 4 != 0 || (uintptr_t)d_out % 4 != 0) return APSEP_EINVAL;
-    // answers over the keys themselves (in place) take the general route, which
-    // reads the keys into the workspace first
-    if (ranges_overlap(d_in, (size_t)n * 4, d_out, (size_t)n * 4)) return APSEP_ENOTSUP;
-    // a view head would need the view instantiation: those runs take the general route
-    if ((uintptr_t)d_in % 16 != (uintptr_t)d_out % 16 || (uintptr_t)d_in % 16 != 0) return APSEP_ENOTSUP;
-    DeviceGuard g(p->device);
-    if (!g.ok) return APSEP_ECUDA;
-    const int B = 32 * kTileConfigs[0].ipt;  // keys per warp tile
-    const int tile_rows = B / 32;
-    int rows = (int)(n / 32);
-    CUtensorMap mi, mo;
-    memset(&mi, 0, sizeof(mi));
-    memset(&mo, 0, sizeof(mo));
+// The arguments of a flipped or reversed run and its TMA maps: the whole array in
+// tiles of 512 keys (APSEP_ENOTSUP: the engine has no such form for the call).
+namespace {
+apsep_status mapped_args(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n, RangeArgs* out, CUtensorMap* mi,
+                         CUtensorMap* mo) {
+    const int kb = key_bytes(p->dtype);
+    const int B = wide(p->dtype) ? kWideMappedTileKeys : 32 * kTileConfigs[0].ipt;  // keys per warp tile
+    // 8-byte keys: these forms exist in the tiles of long arrays
+    if (wide(p->dtype) && wide_tile_keys(n, false) != B) return APSEP_ENOTSUP;
+    const int tile_rows = B * kb / 128;  // 128-byte rows per tile
+    int rows = (int)(n * kb / 128);
+    memset(mi, 0, sizeof(*mi));
+    memset(mo, 0, sizeof(*mo));
     if (rows < tile_rows) rows = 0;
-    if (rows > 0 && (!encode_rows(&mi, d_in, rows, tile_rows, p->dtype) || !encode_rows(&mo, d_out, rows, tile_rows, 0)))
+    if (rows > 0 && (!encode_rows(mi, d_in, rows, tile_rows, p->dtype) ||
+                     !encode_rows(mo, d_out, (int)(n / 32), B / 32, APSEP_INT32)))
         return APSEP_ECUDA;
-    RangeArgs a;
+    RangeArgs& a = *out;
     a.d_in = d_in;
     a.d_out = d_out;
     a.n = (int)n;
@@ -335,45 +331,49 @@ apsep_status plan_run_flipped(apsep_plan* p, const void* d_in, int32_t* d_out, i
     a.s = p->rs;
     p->dbg_skip_range = -1;
     p->dbg_spin_limit = 0;
-    const cudaError_t e =
-        launch_range_flipped(p->dtype, cmp == APSEP_LE ? 1 : 0, span, a, mi, mo, (cudaStream_t)stream);
+    return APSEP_OK;
+}
+}  // namespace
+
+apsep_status plan_run_flipped(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp, int span,
+                              void* stream) {
+    if (!p || n <= 0 || n > p->capacity || !d_in || !d_out || (cmp != APSEP_LT && cmp != APSEP_LE)) return APSEP_EINVAL;
+    if (span && cmp != APSEP_LT) return APSEP_ENOTSUP;
+    const int kb = key_bytes(p->dtype);
+    if ((uintptr_t)d_in % kb != 0 || (uintptr_t)d_out % 4 != 0) return APSEP_EINVAL;
+    // answers over the keys themselves (in place) take the general route, which
+    // reads the keys into the workspace first
+    if (ranges_overlap(d_in, (size_t)n * kb, d_out, (size_t)n * 4)) return APSEP_ENOTSUP;
+    // a view head would need the view instantiation: those runs take the general route
+    if ((uintptr_t)d_in % 16 != 0 || (uintptr_t)d_out % 16 != 0) return APSEP_ENOTSUP;
+    DeviceGuard g(p->device);
+    if (!g.ok) return APSEP_ECUDA;
+    RangeArgs a;
+    CUtensorMap mi, mo;
+    const apsep_status s = mapped_args(p, d_in, d_out, n, &a, &mi, &mo);
+    if (s != APSEP_OK) return s;
+    const int incl = cmp == APSEP_LE ? 1 : 0;
+    const cudaError_t e = wide(p->dtype) ? launch_wide_flipped(p->dtype, incl, span, a, mi, mo, (cudaStream_t)stream)
+                                         : launch_range_flipped(p->dtype, incl, span, a, mi, mo, (cudaStream_t)stream);
     return e == cudaSuccess ? APSEP_OK : APSEP_ECUDA;
 }
 
 apsep_status plan_run_reversed(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp,
                                void* stream) {
     if (!p || n <= 0 || n > p->capacity || !d_in || !d_out || (cmp != APSEP_LT && cmp != APSEP_LE)) return APSEP_EINVAL;
-    if (wide(p->dtype) || n % 32 != 0) return APSEP_ENOTSUP;
+    if (n % 32 != 0) return APSEP_ENOTSUP;
     if ((uintptr_t)d_in % 16 != 0 || (uintptr_t)d_out % 16 != 0) return APSEP_ENOTSUP;
-    if (ranges_overlap(d_in, (size_t)n * 4, d_out, (size_t)n * 4)) return APSEP_ENOTSUP;  // in place: general route
+    // in place: general route
+    if (ranges_overlap(d_in, (size_t)n * key_bytes(p->dtype), d_out, (size_t)n * 4)) return APSEP_ENOTSUP;
     DeviceGuard g(p->device);
     if (!g.ok) return APSEP_ECUDA;
-    const int B = 32 * kTileConfigs[0].ipt;  // keys per warp tile
-    const int tile_rows = B / 32;
-    int rows = (int)(n / 32);
-    CUtensorMap mi, mo;
-    memset(&mi, 0, sizeof(mi));
-    memset(&mo, 0, sizeof(mo));
-    if (rows < tile_rows) rows = 0;
-    if (rows > 0 && (!encode_rows(&mi, d_in, rows, tile_rows, p->dtype) || !encode_rows(&mo, d_out, rows, tile_rows, 0)))
-        return APSEP_ECUDA;
     RangeArgs a;
-    a.d_in = d_in;
-    a.d_out = d_out;
-    a.n = (int)n;
-    a.head = 0;
-    a.num_tiles = (int)((n + B - 1) / B);
-    a.tiles_per_range = 0;
-    a.num_ranges = 0;
-    a.tma_rows = rows;
-    a.spin_limit = p->dbg_spin_limit ? p->dbg_spin_limit : kDefaultSpinLimit;
-    a.skip_publish_range = p->dbg_skip_range;
-    a.offsets = nullptr;
-    a.nseg = 1;
-    a.s = p->rs;
-    p->dbg_skip_range = -1;
-    p->dbg_spin_limit = 0;
-    const cudaError_t e = launch_range_reversed(p->dtype, cmp == APSEP_LE ? 1 : 0, a, mi, mo, (cudaStream_t)stream);
+    CUtensorMap mi, mo;
+    const apsep_status s = mapped_args(p, d_in, d_out, n, &a, &mi, &mo);
+    if (s != APSEP_OK) return s;
+    const int incl = cmp == APSEP_LE ? 1 : 0;
+    const cudaError_t e = wide(p->dtype) ? launch_wide_reversed(p->dtype, incl, a, mi, mo, (cudaStream_t)stream)
+                                         : launch_range_reversed(p->dtype, incl, a, mi, mo, (cudaStream_t)stream);
     return e == cudaSuccess ? APSEP_OK : APSEP_ECUDA;
 }
 

@@ -10,8 +10,9 @@
 //   largest rectangle = max over i of h[i] * (next smaller - previous smaller - 1)
 //   Cartesian parent  = of previous smaller-or-equal and next smaller, the one
 //                       with the larger key (ties: the next one)
-// With 4-byte keys on a 16-byte boundary the engine does the flips and
-// reversals itself (apsep_mapped.cu): previous greater and the stock span are
+// With 4-byte keys on a 16-byte boundary, and 8-byte ones in arrays of long tiles,
+// the engine does the flips and reversals itself (apsep_mapped.cu,
+// apsep_wide_mapped.cu): previous greater and the stock span are
 // one run each with the keys flipped as they load (and position - answer as
 // the answers leave), next smaller one run over the reversed array with its
 // answers mirrored as they leave (the last n % 32 keys apart: a pass over the answers
@@ -26,6 +27,7 @@
 #include <type_traits>
 
 #include "apsep.h"
+#include "apsep_device.cuh"
 #include "apsep_internal.h"
 
 namespace {
@@ -105,28 +107,39 @@ __global__ void reverse_keys(const T* __restrict__ in, T* __restrict__ out, int6
 // The next-smaller answer from its mirror image, a previous-smaller answer of the
 // reversed array (-1: none).
 __device__ __forceinline__ int64_t next_from_reversed(int32_t a, int64_t n) { return a >= 0 ? n - 1 - a : -1; }
+// A key as these passes compare it: float64 keys by the order-preserving map of their
+// bits (each thread's minimum over a tail of 25 keys, compared as doubles, took next
+// smaller of 5M float64 keys from 56 to 83 us).
+template <typename T>
+__device__ __forceinline__ T ordered(T x) {
+    return x;
+}
+__device__ __forceinline__ int64_t ordered(double x) { return apsep::f64_order(__double_as_longlong(x)); }
+template <typename T>
+using Ordered = std::conditional_t<std::is_same_v<T, double>, int64_t, T>;
 // The keys after the last multiple of 32 (the engine's reversed run takes whole
 // 32-key rows): at most 31 of them, in shared memory, with their minimum.
-template <typename T>
+template <typename K>
 struct Tail {
-    const T* v;
-    T least;
+    const K* v;
+    K least;
     int count;
     int64_t base;  // position of the first (n when there is none)
 };
 // Called by every thread of the block; v: 32 keys of its shared memory.
 template <typename T>
-__device__ __forceinline__ Tail<T> load_tail(const T* __restrict__ a, int64_t n, int64_t base, T* v) {
+__device__ __forceinline__ Tail<Ordered<T>> load_tail(const T* __restrict__ a, int64_t n, int64_t base,
+                                                      Ordered<T>* v) {
     const int count = (int)(n - base);
-    if ((int)threadIdx.x < count) v[threadIdx.x] = a[base + threadIdx.x];
+    if ((int)threadIdx.x < count) v[threadIdx.x] = ordered(a[base + threadIdx.x]);
     __syncthreads();
-    T least = count > 0 ? v[0] : T(0);
+    Ordered<T> least = count > 0 ? v[0] : Ordered<T>(0);
     for (int j = 1; j < count; j++) least = v[j] < least ? v[j] : least;
     return {v, least, count, base};
 }
 // The first tail key at or after position i that is smaller (or equal) than q, or -1.
-template <bool LE, typename T>
-__device__ __forceinline__ int64_t next_in_tail(const Tail<T>& t, T q, int64_t i) {
+template <bool LE, typename K>
+__device__ __forceinline__ int64_t next_in_tail(const Tail<K>& t, K q, int64_t i) {
     if (t.count == 0 || !(LE ? t.least <= q : t.least < q)) return -1;
     for (int j = i > t.base ? (int)(i - t.base) : 0; j < t.count; j++)
         if (LE ? t.v[j] <= q : t.v[j] < q) return t.base + j;
@@ -135,30 +148,30 @@ __device__ __forceinline__ int64_t next_in_tail(const Tail<T>& t, T q, int64_t i
 // What next-smaller answer of key i to load (next_word) and its meaning (next_of): R
 // holds the answers themselves over the keys before the tail (direct, a reversed run of
 // the engine), or the reversed array's previous-smaller answers (no tail).
-template <typename T>
-__device__ __forceinline__ int32_t next_word(const int32_t* __restrict__ R, bool direct, const Tail<T>& t, int64_t n,
+template <typename K>
+__device__ __forceinline__ int32_t next_word(const int32_t* __restrict__ R, bool direct, const Tail<K>& t, int64_t n,
                                              int64_t i) {
     return !direct ? R[n - 1 - i] : i < t.base ? R[i] : -1;
 }
 template <typename T>
-__device__ __forceinline__ int64_t next_of(const T* __restrict__ a, int32_t word, bool direct, const Tail<T>& t,
-                                           int64_t n, int64_t i) {
+__device__ __forceinline__ int64_t next_of(const T* __restrict__ a, int32_t word, bool direct,
+                                           const Tail<Ordered<T>>& t, int64_t n, int64_t i) {
     if (!direct) return next_from_reversed(word, n);
-    return word >= 0 || t.count == 0 ? word : next_in_tail<false>(t, a[i], i + 1);
+    return word >= 0 || t.count == 0 ? word : next_in_tail<false>(t, ordered(a[i]), i + 1);
 }
 
 // Completes next-smaller answers of a reversed run over the keys before the tail:
 // its unanswered keys and the tail's own.
 template <typename T, bool LE>
 __global__ void next_with_tail(const T* __restrict__ a, int32_t* __restrict__ out, int64_t n, int64_t base) {
-    __shared__ T tail_keys[32];
+    __shared__ Ordered<T> tail_keys[32];
     apsep::grid_dependency_wait();
-    const Tail<T> t = load_tail(a, n, base, tail_keys);
+    const Tail<Ordered<T>> t = load_tail(a, n, base, tail_keys);
     for_batches(
         n, [&](int64_t i) { return i < base ? out[i] : -1; },
         [&](int64_t i, int32_t r) {
             if (r >= 0) return;
-            const int64_t o = next_in_tail<LE>(t, a[i], i + 1);
+            const int64_t o = next_in_tail<LE>(t, ordered(a[i]), i + 1);
             if (o >= 0 || i >= base) out[i] = (int32_t)o;  // (a key without one reads -1 already)
         });
 }
@@ -215,14 +228,14 @@ template <typename T>
 __global__ void cartesian_parent(const T* __restrict__ a, const int32_t* __restrict__ L,
                                  const int32_t* __restrict__ ar, bool direct, int64_t base,
                                  int32_t* __restrict__ out, int64_t n) {
-    __shared__ T tail_keys[32];
+    __shared__ Ordered<T> tail_keys[32];
     apsep::grid_dependency_wait();
-    const Tail<T> t = load_tail(a, n, base, tail_keys);
+    const Tail<Ordered<T>> t = load_tail(a, n, base, tail_keys);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kBatch * stride) {
         // kBatch keys of a thread side by side: the answers' reads, then their keys'
         int32_t l[kBatch], r[kBatch];
-        T kl[kBatch], kr[kBatch];
+        Ordered<T> kl[kBatch], kr[kBatch];
 #pragma unroll
         for (int u = 0; u < kBatch; u++) {
             const int64_t i = i0 + u * stride;
@@ -236,8 +249,8 @@ __global__ void cartesian_parent(const T* __restrict__ a, const int32_t* __restr
         }
 #pragma unroll
         for (int u = 0; u < kBatch; u++) {
-            kl[u] = a[l[u] < 0 ? 0 : l[u]];
-            kr[u] = a[r[u] < 0 ? 0 : r[u]];
+            kl[u] = ordered(a[l[u] < 0 ? 0 : l[u]]);
+            kr[u] = ordered(a[r[u] < 0 ? 0 : r[u]]);
         }
 #pragma unroll
         for (int u = 0; u < kBatch; u++) {
@@ -255,10 +268,10 @@ bool overlaps(const void* a, size_t an, const void* b, size_t bn) {
 // The reversed run of the engine over the keys before the last n % 32, when it has
 // that form for the call (whole rows of 32 keys; *base: where they end), else
 // APSEP_ENOTSUP.
-apsep_status run_reversed(apsep_plan* plan, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp, void* stream,
-                          int64_t* base) {
+apsep_status run_reversed(apsep_plan* plan, int dtype, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp,
+                          void* stream, int64_t* base) {
     *base = n / 32 * 32;
-    if (*base == 0 || overlaps(d_in, (size_t)n * 4, d_out, (size_t)n * 4)) return APSEP_ENOTSUP;
+    if (*base == 0 || overlaps(d_in, (size_t)n * key_bytes(dtype), d_out, (size_t)n * 4)) return APSEP_ENOTSUP;
     return plan_run_reversed(plan, d_in, d_out, *base, cmp, stream);
 }
 
@@ -299,8 +312,8 @@ apsep_status apsep_run_prev_greater(apsep_plan* plan, const void* d_in, int32_t*
     int dtype = 0;
     apsep_status s = check_args(plan, d_in, d_out, (size_t)n * 4, n, d_work, &dtype);
     if (s != APSEP_OK || n == 0) return s;
-    // one engine run that flips the keys as it loads them (4-byte keys on a
-    // 16-byte boundary), else a flip pass into the workspace and a plain run
+    // one engine run that flips the keys as it loads them, when it has that form for
+    // the call, else a flip pass into the workspace and a plain run
     if ((s = plan_run_flipped(plan, d_in, d_out, n, cmp, 0, stream)) != APSEP_ENOTSUP) return s;
     const cudaStream_t st = (cudaStream_t)stream;
     for_key_type(dtype, [&](auto tag) {
@@ -320,14 +333,14 @@ apsep_status apsep_run_next_smaller(apsep_plan* plan, const void* d_in, int32_t*
     // when it has that form for the call; else reverse, run, mirror
     const cudaStream_t st = (cudaStream_t)stream;
     int64_t base = n;
-    if ((s = run_reversed(plan, d_in, d_out, n, cmp, stream, &base)) != APSEP_ENOTSUP) {
+    if ((s = run_reversed(plan, dtype, d_in, d_out, n, cmp, stream, &base)) != APSEP_ENOTSUP) {
         if (s != APSEP_OK || base == n) return s;
         const bool le = cmp == APSEP_LE;
-        if (dtype == APSEP_INT32)
-            return launched(le ? next_with_tail<int32_t, true> : next_with_tail<int32_t, false>, n, st,
-                            (const int32_t*)d_in, d_out, n, base);
-        return launched(le ? next_with_tail<float, true> : next_with_tail<float, false>, n, st, (const float*)d_in,
-                        d_out, n, base);
+        for_key_type(dtype, [&](auto tag) {
+            using T = std::remove_pointer_t<decltype(tag)>;
+            s = launched(le ? next_with_tail<T, true> : next_with_tail<T, false>, n, st, (const T*)d_in, d_out, n, base);
+        });
+        return s;
     }
     const Work w = carve(d_work, n, dtype);
     for_key_type(dtype, [&](auto tag) {
@@ -370,7 +383,7 @@ apsep_status apsep_largest_rectangle(apsep_plan* plan, const int32_t* d_heights,
     // reverse the heights and run (the answers then come mirrored)
     bool direct = true;
     int64_t base = n;  // where the tail begins (none after a run over the whole reversed copy)
-    if ((s = run_reversed(plan, d_heights, w.a, n, APSEP_LT, stream, &base)) == APSEP_ENOTSUP) {
+    if ((s = run_reversed(plan, dtype, d_heights, w.a, n, APSEP_LT, stream, &base)) == APSEP_ENOTSUP) {
         direct = false;
         base = n;
         s = launched(reverse_keys<int32_t>, n, st, d_heights, (int32_t*)w.keys, n);
@@ -392,7 +405,7 @@ apsep_status apsep_cartesian_parents(apsep_plan* plan, const void* d_in, int32_t
     if ((s = apsep_run_cmp(plan, d_in, w.b, n, APSEP_LE, stream)) != APSEP_OK) return s;
     bool direct = true;  // next smaller straight from a reversed run, else mirrored
     int64_t base = n;
-    if ((s = run_reversed(plan, d_in, w.a, n, APSEP_LT, stream, &base)) == APSEP_ENOTSUP) {
+    if ((s = run_reversed(plan, dtype, d_in, w.a, n, APSEP_LT, stream, &base)) == APSEP_ENOTSUP) {
         direct = false;
         base = n;
         for_key_type(dtype, [&](auto tag) {

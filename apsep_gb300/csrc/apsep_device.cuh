@@ -66,8 +66,8 @@ __device__ __forceinline__ int64_t f64_order(int64_t b) {
 // KMAP template parameter): KMAP_F64 -- int64 slots holding float64 bit
 // patterns, compared through f64_order; KMAP_FLIP -- the order-reversing map
 // (integers ~x = -x - 1, floats -x; the two zeros stay equal), so that a
-// previous-smaller run answers previous-greater queries.
-constexpr int KMAP_NONE = 0, KMAP_F64 = 1, KMAP_FLIP = 2;
+// previous-smaller run answers previous-greater queries; KMAP_F64_FLIP -- both.
+constexpr int KMAP_NONE = 0, KMAP_F64 = 1, KMAP_FLIP = 2, KMAP_F64_FLIP = 3;
 __device__ __forceinline__ int32_t flip_key(int32_t x) { return ~x; }
 __device__ __forceinline__ float flip_key(float x) { return -x; }
 __device__ __forceinline__ int64_t flip_key(int64_t x) { return ~x; }
@@ -75,12 +75,14 @@ template <typename T, int KMAP>
 __device__ __forceinline__ T map_key(T x) {
     if constexpr (KMAP == KMAP_F64) return (T)f64_order((int64_t)x);
     else if constexpr (KMAP == KMAP_FLIP) return flip_key(x);
+    else if constexpr (KMAP == KMAP_F64_FLIP) return flip_key((T)f64_order((int64_t)x));
     else return x;
 }
 // The raw key that the key map takes to the pad.
 template <typename T, int KMAP>
 __device__ __forceinline__ T raw_pad() {
-    return KMAP == KMAP_FLIP ? flip_key(KeyTraits<T>::pad()) : KeyTraits<T>::pad();
+    if constexpr (KMAP == KMAP_F64_FLIP) return (T)-1;  // f64_order's smallest value, which the flip makes the pad
+    else return KMAP == KMAP_FLIP ? flip_key(KeyTraits<T>::pad()) : KeyTraits<T>::pad();
 }
 // A key from global memory, through the key map.
 template <typename T, int KMAP>

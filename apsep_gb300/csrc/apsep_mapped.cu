@@ -4,8 +4,8 @@
 //     previous-smaller engine over the unchanged input answers previous
 //     greater (or greater-or-equal under <=), and with the span output form
 //     it writes the stock span (position - previous strictly greater);
-//   * the reversed array: tiles counted from the end and reversed as they
-//     land, answers mirrored as they leave, so one run answers next smaller
+//   * the reversed array: tiles counted from the end and read mirrored from
+//     shared memory, answers mirrored as they leave, so one run answers next smaller
 //     (or smaller-or-equal).
 // Single arrays on a 16-byte boundary (keys and answers), 4-byte keys,
 // configuration 0 (16 warps per CTA, 512-key warp tiles).

@@ -888,7 +888,7 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
 // tile whose keys are all deferred is not written at all (its flag word says
 // so); the int64-position path answers what is left.  OUT_SPAN -- int32
 // position - answer (position + 1 for none): the stock span, with the flip.
-// REV (single arrays, no view head, 4-byte keys): the run sees the array
+// REV (single arrays, no view head): the run sees the array
 // reversed -- tile t holds elements n - 1 - (t * WT + e), its TMA rows counted
 // from the end (n a multiple of 32) and read mirrored from shared
 // memory -- and writes each answer mirrored back, n - 1 - answer (-1 for none)
@@ -961,7 +961,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
     };
     auto seg_idx = [&](int pos) { return a.offsets ? seg_find(a.offsets, a.nseg, pos, err) : 0; };
     static_assert(OUTM == OUT_I32 || (!SEG && EP), "int64 and span answers: single arrays only");
-    static_assert(!REV || (!SEG && EP && OUTM == OUT_I32 && KB == 4), "reversed runs: single arrays of 4-byte keys");
+    static_assert(!REV || (!SEG && EP && OUTM == OUT_I32), "reversed runs: single arrays");
     constexpr bool OUT64 = OUTM == OUT_I64;
     uint32_t epoch = 0;
     if (lane == 0) {
@@ -1121,9 +1121,9 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             } else {  // two 8-byte keys per 16-byte chunk
 #pragma unroll
                 for (int q2 = 0; q2 < IPT / 2; q2++) {
-                    const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(&V[ks(lane * IPT + 2 * q2)]);
-                    v[2 * q2 + 0] = KeyTraits<T>::from_bits((uint64_t)rr.x);
-                    v[2 * q2 + 1] = KeyTraits<T>::from_bits((uint64_t)rr.y);
+                    const ulonglong2 rr = *reinterpret_cast<const ulonglong2*>(&V[ks(chunk(2 * q2))]);
+                    v[in_chunk(2 * q2 + 0)] = KeyTraits<T>::from_bits((uint64_t)rr.x);
+                    v[in_chunk(2 * q2 + 1)] = KeyTraits<T>::from_bits((uint64_t)rr.y);
                 }
             }
             if constexpr (MAPF != KMAP_NONE) {
@@ -1226,7 +1226,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 __syncwarp();
                 if (full) {
                     if (lane == 0) {
-                        tma_store_2d(&map_out, 0, REV ? tile_row(t) : t * W, O);
+                        tma_store_2d(&map_out, 0, REV ? a.tma_rows * 4 / KB - (t + 1) * W : t * W, O);
                         bulk_commit();
                     }
                 } else {
@@ -1249,13 +1249,13 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     h[REV ? 1 : 2] = KeyTraits<T>::from_bits(rr.z);
                     h[REV ? 0 : 3] = KeyTraits<T>::from_bits(rr.w);
                 } else {
-                    const T* hq = lane > 0 ? &V[ks(lane * IPT - 2)] : sPad + 2;
+                    const T* hq = lane > 0 ? &V[ks(REV ? WT - lane * IPT + 2 : lane * IPT - 2)] : sPad + 2;
                     const ulonglong2 r0 = *reinterpret_cast<const ulonglong2*>(hp);
                     const ulonglong2 r1 = *reinterpret_cast<const ulonglong2*>(hq);
-                    h[0] = KeyTraits<T>::from_bits((uint64_t)r0.x);
-                    h[1] = KeyTraits<T>::from_bits((uint64_t)r0.y);
-                    h[2] = KeyTraits<T>::from_bits((uint64_t)r1.x);
-                    h[3] = KeyTraits<T>::from_bits((uint64_t)r1.y);
+                    h[REV ? 3 : 0] = KeyTraits<T>::from_bits((uint64_t)r0.x);
+                    h[REV ? 2 : 1] = KeyTraits<T>::from_bits((uint64_t)r0.y);
+                    h[REV ? 1 : 2] = KeyTraits<T>::from_bits((uint64_t)r1.x);
+                    h[REV ? 0 : 3] = KeyTraits<T>::from_bits((uint64_t)r1.y);
                 }
             }
             if constexpr (MAPF != KMAP_NONE) {
