@@ -335,10 +335,15 @@ __global__ void __launch_bounds__(kThreads)
                 // range's minimum before the tile is >= its first key)
                 const bool bounded = lane < W && (lane > 0 || t % tiles_per_range != 0);
                 K ub = KeyTraits<K>::pad(), lb = ub;
-                if (lane < W) lb = __ldcg(&cmin[(size_t)t * W + lane]);
                 if (bounded) ub = lane > 0 ? __ldcg(&cmin[(size_t)t * W + lane - 1]) : __ldcg(&tmin[t - 1]);
                 const bool none_p = bounded && !(has_p && lt<INCL>(P, ub));  // phase 2 answered no key of the chunk
                 const unsigned decm = __ballot_sync(FULL, none_p && !(has && lt<INCL>(pm, ub)));
+                if (decm == (unsigned)((1ull << W) - 1) && tb + WT <= b1) {  // no key of the tile has an answer
+#pragma unroll
+                    for (int c = 0; c < W; c++) put(tb + 32 * c + lane, -1);
+                    continue;
+                }
+                if (lane < W) lb = __ldcg(&cmin[(size_t)t * W + lane]);
                 const unsigned donem = __ballot_sync(FULL, has_p && lt<INCL>(P, lb));  // ... and here every key
 #pragma unroll 1
                 for (int c = 0; c < W; c++) {
