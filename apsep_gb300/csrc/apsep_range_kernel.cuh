@@ -1057,6 +1057,14 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             }
             if (lane == 0) bulk_wait_read0();  // the previous tile's store has read O
             __syncwarp();
+            // Every lane is done with V: the load of the tile kStages on goes there.
+            auto load_ahead = [&]() {
+                __syncwarp();
+                if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
+                    mbar_arrive_expect_tx(&bar[slot], (uint32_t)(WT * KB));
+                    tma_load_2d(V, &map_in, 0, tile_row(t + kStages), &bar[slot]);
+                }
+            };
 
             // ---- 0. segmented runs: where segments start among the tile's keys ----------
             unsigned bword = 0;  // segment starts among this lane's keys (bit k: key k)
@@ -1360,23 +1368,26 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                         dropped = true;
                     }
                     rmin = KeyTraits<T>::vmin(rmin, tmin);
-                    __syncwarp();
-                    if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
-                        mbar_arrive_expect_tx(&bar[slot], (uint32_t)(WT * KB));
-                        tma_load_2d(V, &map_in, 0, tile_row(t + kStages), &bar[slot]);
-                    }
+                    load_ahead();
                     continue;
                 }
                 if (never && (!has_rmin || !lt<INCL>(rmin, first))) {
-                    const int4 m1 = make_int4(-1, -1, -1, -1);
-#pragma unroll
-                    for (int q4 = 0; q4 < IPT / 4; q4++) *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) = m1;
-                    if (((lane + 1) & (TPC - 1)) == 0) __stcg(&chunk_min_w[(size_t)t * W + lane / TPC], v[IPT - 1]);
-                    const T tmin = __shfl_sync(FULL, v[IPT - 1], 31);
                     for (int e = lane; e < WT && def_total + e < kDefCap; e += 32) {
                         sDefP[def_total + e] = tile_base + e;
                         sDefV[def_total + e] = key(e);
                     }
+                    // With nothing to store the loads set the pace, and the next one leaves
+                    // here (2^28 keys in two pieces 636 -> 620 us); where the tile is stored
+                    // too, loads this early made it slower (a run of 2^28: 372 -> 382 us).
+                    if constexpr (OUT64) {
+                        load_ahead();
+                    } else {
+                        const int4 m1 = make_int4(-1, -1, -1, -1);
+#pragma unroll
+                        for (int q4 = 0; q4 < IPT / 4; q4++) *reinterpret_cast<int4*>(&O[swz(lane * IPT + 4 * q4)]) = m1;
+                    }
+                    if (((lane + 1) & (TPC - 1)) == 0) __stcg(&chunk_min_w[(size_t)t * W + lane / TPC], v[IPT - 1]);
+                    const T tmin = __shfl_sync(FULL, v[IPT - 1], 31);
                     if (lane < W) __stcg(&a.s.tile_mask[(size_t)t * MW + lane], 0xffffffffu);
                     if (lane == 0) {
                         __stcg(&a.s.tile_flag[t], (uint32_t)WT | (OUT64 ? TILE_NOT_STORED : 0u));
@@ -1406,11 +1417,8 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     stk_hi = stk_lo + 1;
                     rmin = tmin;
                     has_rmin = true;
-                    __syncwarp();
-                    if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
-                        mbar_arrive_expect_tx(&bar[slot], (uint32_t)(WT * KB));
-                        tma_load_2d(V, &map_in, 0, tile_row(t + kStages), &bar[slot]);
-                    }
+                    if constexpr (OUT64) __syncwarp();
+                    else load_ahead();
                     continue;
                 }
             }
@@ -1477,11 +1485,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     stk_lo = stk_hi - kUpKeep;
                     dropped = true;  // the older entries are gone
                     rmin = KeyTraits<T>::vmin(rmin, first);
-                    __syncwarp();
-                    if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
-                        mbar_arrive_expect_tx(&bar[slot], (uint32_t)(WT * KB));
-                        tma_load_2d(V, &map_in, 0, tile_row(t + kStages), &bar[slot]);
-                    }
+                    load_ahead();
                     continue;
                 }
             }
@@ -1931,11 +1935,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
             if (lane == 0) __stcg(&tile_min_w[t], tile_min_t);
             rmin = has_rmin ? KeyTraits<T>::vmin(rmin, tile_min_t) : tile_min_t;
             has_rmin = true;
-            __syncwarp();
-            if (lane == 0 && i + kStages < ntr && tile_full(t + kStages)) {
-                mbar_arrive_expect_tx(&bar[slot], (uint32_t)(WT * KB));
-                tma_load_2d(V, &map_in, 0, tile_row(t + kStages), &bar[slot]);
-            }
+            load_ahead();
         }
 
         // ======================= publish the range, its prefix ======================
