@@ -1319,7 +1319,8 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 unsigned same = 0u;  // the window entries that qualify for every key
                 const int wlo = max(stk_lo, stk_hi - 32);
                 T wtop = KeyTraits<T>::pad();
-                if (never && has_rmin) {
+                const bool below = !has_rmin || !lt<INCL>(rmin, first);  // nothing in the range qualifies
+                if (never && !below) {
                     const bool in = wlo + lane < stk_hi;
                     const T last = __shfl_sync(FULL, v[IPT - 1], 31);
                     wtop = in ? sStkV[(wlo + lane) & (K - 1)] : KeyTraits<T>::pad();
@@ -1371,7 +1372,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                     load_ahead();
                     continue;
                 }
-                if (never && (!has_rmin || !lt<INCL>(rmin, first))) {
+                if (never && below) {
                     for (int e = lane; e < WT && def_total + e < kDefCap; e += 32) {
                         sDefP[def_total + e] = tile_base + e;
                         sDefV[def_total + e] = key(e);
