@@ -44,12 +44,14 @@
 //  (find_in_tiles).
 //
 //  On random keys the kernel is bound by the latency of its dependent steps
-//  and by issue (4 warps a scheduler; 58 % of issue slots and 50 % of the ALU
-//  pipe busy at 2^25 int32 keys): seeing four predecessors before any query,
+//  and by issue (4 warps a scheduler; 62 % of issue slots busy in the steady
+//  state at 2^25 int32 keys): seeing four predecessors before any query,
 //  one list and one prefix sum per tile, no prefix scan and one query round
-//  took 2^25 uniform keys from 136 to 117 us (2.3 TB/s of useful bytes), the
-//  one-key-per-lane phase 2 with the longer stack and lists a random walk of
-//  2^24 keys (stock span) from 783 to 202 us and of 2^20 keys from 176 to 40.
+//  took 2^25 uniform keys from 136 to 117 us and, with launches that overlap the
+//  previous kernel and the shorter handshake, to 111 (2.4 TB/s of useful bytes);
+//  the one-key-per-lane phase 2 with the longer stack and lists, and each stack top
+//  copied once, took a random walk of 2^24 keys (stock span) from 783 to 140 us and
+//  of 2^20 keys from 176 to 28.
 #pragma once
 #include "apsep_device.cuh"
 #include "apsep_internal.h"

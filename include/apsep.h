@@ -66,7 +66,9 @@ typedef struct apsep_plan apsep_plan;
 typedef struct apsep_plan_info {
     int64_t capacity;       /* largest n a run may use                      */
     int64_t scratch_bytes;  /* device scratch owned by the plan             */
-    int32_t tile_keys;      /* keys per tile of the selected configuration  */
+    int32_t tile_keys;      /* keys per tile of the selected configuration
+                               (8-byte keys: of short arrays and batches;
+                               long arrays run in tiles of twice as many)   */
     int32_t config;         /* index of the selected kernel configuration   */
     int32_t device;         /* CUDA device the plan lives on                */
     int32_t dtype;
