@@ -220,13 +220,14 @@ apsep_status run_impl(apsep_plan* p, const void* d_in, int32_t* d_out, int64_t n
     DeviceGuard g(p->device);
     if (!g.ok) return APSEP_ECUDA;
     if (wide(p->dtype)) {  // 8-byte keys: TMA when both arrays are 16-byte aligned
-        const int B = wide_tile_keys(n, offsets != nullptr), key_rows_per_tile = B * 8 / 128;
+        const bool aligned = (uintptr_t)d_in % 16 == 0 && (uintptr_t)d_out % 16 == 0;
+        const int B = wide_tile_keys(n, offsets != nullptr, aligned), key_rows_per_tile = B * 8 / 128;
         if (B == 0) return APSEP_ECUDA;
         int rows = (int)(n / 16);  // 128-byte rows of keys
         CUtensorMap mi, mo;
         memset(&mi, 0, sizeof(mi));
         memset(&mo, 0, sizeof(mo));
-        if ((uintptr_t)d_in % 16 != 0 || (uintptr_t)d_out % 16 != 0 || rows < key_rows_per_tile) rows = 0;
+        if (!aligned || rows < key_rows_per_tile) rows = 0;
         if (rows > 0) {
             if (!encode_rows(&mi, d_in, rows, key_rows_per_tile, p->dtype) ||
                 !encode_rows(&mo, d_out, (int)(n / 32), B / 32, APSEP_INT32))
@@ -306,7 +307,7 @@ apsep_status mapped_args(apsep_plan* p, const void* d_in, int32_t* d_out, int64_
     const int kb = key_bytes(p->dtype);
     const int B = wide(p->dtype) ? kWideMappedTileKeys : 32 * kTileConfigs[0].ipt;  // keys per warp tile
     // 8-byte keys: these forms exist in the tiles of long arrays
-    if (wide(p->dtype) && wide_tile_keys(n, false) != B) return APSEP_ENOTSUP;
+    if (wide(p->dtype) && wide_tile_keys(n, false, true) != B) return APSEP_ENOTSUP;
     const int tile_rows = B * kb / 128;  // 128-byte rows per tile
     int rows = (int)(n * kb / 128);
     memset(mi, 0, sizeof(*mi));

@@ -179,11 +179,11 @@ cudaError_t range_prepare(int cfg);  // smem attributes + occupancy, current dev
 cudaError_t launch_range_segmented(int dtype, int incl, int cfg, RangeArgs& a, const CUtensorMap& map_in,
                                    const CUtensorMap& map_out, cudaStream_t stream);
 // 8-byte keys (dtype 2: int64, 3: float64), single arrays and segmented batches
-// (RangeArgs::offsets): warp tiles of wide_tile_keys(n, segmented) keys, which the
-// launch is given back; the int64-position path's pieces run in kWideTileKeys.
+// (RangeArgs::offsets): warp tiles of wide_tile_keys(...) keys, which the launch is
+// given back (aligned: keys and answers on a 16-byte boundary); the int64-position path's pieces run in kWideTileKeys.
 constexpr int kWideTileKeys = 256;
 cudaError_t prepare_wide();
-int wide_tile_keys(int64_t n, bool segmented);
+int wide_tile_keys(int64_t n, bool segmented, bool aligned);
 cudaError_t launch_range_wide(int dtype, int incl, int tile_keys, RangeArgs& a, const CUtensorMap& map_in,
                               const CUtensorMap& map_out, cudaStream_t st);
 

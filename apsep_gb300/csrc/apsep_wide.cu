@@ -79,13 +79,16 @@ cudaError_t prepare_wide() {
 // 15.3 | 15.0 and 31.1 | 24.9; 2^19 18.7 | 15.1 and 40.3 | 29.7; 2^22 43.6 | 35.3
 // and 56.2 | 49.0; 2^25 218 | 168 and 128 | 119; random walks, whose long lists of
 // phase 2 have fewer warps to share, 2^20 35 | 42, 2^22 76 | 70, 2^25 365 | 329.
+// Arrays off a 16-byte boundary, which take plain loads, keep shape 0 and its 16 warps
+// (2^24 int64 keys, shape 0 against shape 1, us: uniform 201 | 226, descending
+// 139 | 169, ascending 144 | 175).
 // Batches keep shape 0 (2^25 keys in 1024 segments: uniform 237 | 184, but a walk
 // 404 | 486), as do the pieces of the int64-position path (2^27 keys in two: uniform
 // 970 | 800, walk 1816 | 1906; 2^24 in two: descending 163 | 197).
-int wide_tile_keys(int64_t n, bool segmented) {
+int wide_tile_keys(int64_t n, bool segmented, bool aligned) {
     int dev = 0;
     if (prepare_wide() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (segmented) return 32 * kIpt0;
+    if (segmented || !aligned) return 32 * kIpt0;
     return n > (int64_t)32 * kIpt0 * kWpc0 * g_wide_sms[dev] ? 32 * kIpt1 : 32 * kIpt0;
 }
 
