@@ -40,8 +40,9 @@ struct RangeScratch {
     Counters* ctr;
     uint64_t* group_min;    // [max_ranges/32] atomic min of (EPOCH_LIMIT - epoch) << 32 | ordered key
                             //   over each group of 32 ranges; all-ones when created
-    uint64_t* range_state;  // [max_ranges] tag<<32 | key bits: min of a finished range
-    uint64_t* range_key;    // [max_ranges] 8-byte keys: the range minimum (range_state holds the tag)
+    uint64_t* range_state;  // [max_ranges] tag<<32 | key bits (4-byte keys): min of a finished range, for a
+                            //   reader that waits on this word itself
+    uint64_t* range_key;    // key[max_ranges] (packed): the range minima, for readers of the count too
     void* top_key;          // [max_ranges * kTopEntries] key: top of each range's final stack, bottom first
     int32_t* top_pos;       // [max_ranges * kTopEntries] their positions
     uint32_t* top_cnt;      // [max_ranges] entries published | bit 31: they are the whole stack

@@ -171,12 +171,7 @@ __global__ void __launch_bounds__(kPrologue)
     for (int j = 0; j < 4; j++) {
         const int r = 4 * threadIdx.x + j;
         v[j] = KeyTraits<K>::pad();
-        if (r < num_ranges) {
-            if constexpr (sizeof(K) == 8)
-                v[j] = KeyTraits<K>::from_bits((uint64_t)__ldcg((const unsigned long long*)&rs.range_key[r]));
-            else
-                v[j] = KeyTraits<K>::from_bits((uint32_t)__ldcg((const unsigned long long*)&rs.range_state[r]));
-        }
+        if (r < num_ranges) v[j] = __ldcg((const K*)rs.range_key + r);
     }
     const K tot = KeyTraits<K>::vmin(KeyTraits<K>::vmin(v[0], v[1]), KeyTraits<K>::vmin(v[2], v[3]));
     K inc = tot;  // inclusive scan over the warp's threads
