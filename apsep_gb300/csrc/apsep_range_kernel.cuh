@@ -563,6 +563,7 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, int* sRe
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) m = KeyTraits<T>::vmin(m, __shfl_xor_sync(FULL, m, o));
             p = m;
+            __syncwarp();  // the window's ranges are ones that other lanes acquired (a vote orders nothing)
             const int wi = r - 1 - lane;
             win = wi >= 0 ? range_min<T>(a, wi) : KeyTraits<T>::pad();
             return;

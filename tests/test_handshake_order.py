@@ -60,6 +60,12 @@ def test_readers_of_the_count_read_released_words(reader):
     assert read <= released | {"group_min"}
 
 
+def test_lanes_are_ordered_before_they_read_what_others_acquired():
+    body = _block(_code(), r"void range_prefix\(")
+    won = _block(body[body.index("range_state"):], r"if \(__all_sync\(FULL, ok\)\) \{")
+    assert "__syncwarp()" in won[:won.index("range_min<")]
+
+
 def test_tagged_words_are_acquired():
     code = _code()
     loads = [m.start() for m in re.finditer(r"a\.s\.range_state\b", code)]
