@@ -480,7 +480,8 @@ __device__ void range_publish(int r, uint32_t epoch, T rmin, const RangeArgs& a)
 }
 
 // p: the minimum over ranges [0, r); win (lane i): the minimum of range r-1-i
-// (pad below range 0), the window phase 2 searches first.
+// (pad below range 0), the window phase 2 searches first.  has_p: there is a p (not
+// in range 0, nor when the wait gave up).
 template <typename T>
 __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, int* sReady, T& p, bool& has_p, T& win) {
     constexpr unsigned FULL = 0xffffffffu;
@@ -575,6 +576,7 @@ __device__ void range_prefix(int r, uint32_t epoch, const RangeArgs& a, int* sRe
         }
         if (spins >= a.spin_limit) {
             if (lane == 0) atomicOr(&a.s.ctr->err, ERR_LOOKBACK_TIMEOUT);
+            has_p = false;  // what those ranges would publish may be an older run's: phase 2 leaves it alone
             return;
         }
         __nanosleep(spins < 128 ? 64 : 256);
