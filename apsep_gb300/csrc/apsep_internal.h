@@ -194,6 +194,16 @@ cudaError_t prepare_view(int cfg, int* ctas_per_sm);
 cudaError_t launch_range_view(int dtype, int incl, int cfg, RangeArgs& a, const CUtensorMap& map_in,
                               const CUtensorMap& map_out, cudaStream_t st);
 cudaError_t prepare_segmented(int cfg, int* ctas_per_sm);
+// Batches in configuration 0 have CTAs of their own, of kSegWarps warps.
+constexpr int kSegWarps = 20;
+// Persistent warps of such a batch of num_tiles tiles where ctas_per_sm of those
+// CTAs are resident on each of sms SMs; 0: it takes configuration 2's kernel (fewer
+// than six tiles a warp, measured in apsep_segmented.cu, or no CTA fits).
+constexpr int batch_warps(int ctas_per_sm, int sms, int num_tiles) {
+    const int w = ctas_per_sm * sms * kSegWarps < kMaxRanges ? ctas_per_sm * sms * kSegWarps : kMaxRanges;
+    return w > 0 && num_tiles >= 6 * w ? w : 0;
+}
+cudaError_t batch_ctas_per_sm(int* ctas);  // their occupancy, current device (range_prepare(0))
 cudaError_t range_max_warps(int cfg, int* warps);  // persistent warps of one launch, current device
 // A single array (no view head) with int64 answers a.out_base + answer into
 // a.d_out64 (4-byte keys in configuration 0, 8-byte keys in theirs); flagged keys

@@ -39,6 +39,7 @@ size_t carve_scratch(void* base, int64_t capacity, RangeScratch* s, int kb) {
 namespace {
 constexpr int kMaxDev = 64;
 int g_warps[kMaxDev][kNumTileConfigs];  // resident warps per device and configuration
+int g_batch_ctas[kMaxDev];              // resident CTAs per SM of configuration 0's batches
 }
 
 cudaError_t range_prepare(int cfg) {
@@ -47,11 +48,11 @@ cudaError_t range_prepare(int cfg) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= kMaxDev || cfg < 0 || cfg >= kNumTileConfigs) return cudaErrorInvalidValue;
     int per_sm = 0;  // the smallest over the three modes, so every run fits
+    int batch_ctas = 0;
     e = prepare_mode<false, true>(cfg, &per_sm);
     if (e != cudaSuccess) return e;
     if (cfg == 0) {  // batches have their own CTA shape in this configuration
-        int seg_per_sm = 0;
-        e = prepare_segmented(cfg, &seg_per_sm);
+        e = prepare_segmented(cfg, &batch_ctas);
     } else {
         e = prepare_segmented(cfg, &per_sm);
     }
@@ -64,6 +65,7 @@ cudaError_t range_prepare(int cfg) {
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     int warps = per_sm * sms * kTileConfigs[cfg].wpc;
     if (warps > kMaxRanges) warps = kMaxRanges;
+    if (cfg == 0) g_batch_ctas[dev] = batch_ctas;
     g_warps[dev][cfg] = warps;
     return cudaSuccess;
 }
@@ -78,6 +80,15 @@ cudaError_t range_max_warps(int cfg, int* warps) {
         if (e != cudaSuccess) return e;
     }
     *warps = g_warps[dev][cfg];
+    return cudaSuccess;
+}
+
+cudaError_t batch_ctas_per_sm(int* ctas) {
+    int warps = 0, dev = 0;
+    cudaError_t e = range_max_warps(0, &warps);  // (prepared once per device)
+    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    *ctas = g_batch_ctas[dev];
     return cudaSuccess;
 }
 

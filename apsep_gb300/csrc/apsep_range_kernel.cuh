@@ -2006,9 +2006,6 @@ inline cudaError_t prepare_t(int* ctas_per_sm) {
     return cudaSuccess;
 }
 
-// Warps per CTA of a batch in configuration 0.
-constexpr int kSegWarps = 20;
-
 // Shared-memory attributes and occupancy of every kernel of one mode and
 // configuration (the smallest CTAs-per-SM over the four key/comparison types).
 template <bool SEG, bool EP>

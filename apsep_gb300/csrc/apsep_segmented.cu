@@ -27,13 +27,12 @@ cudaError_t launch_range_segmented(int dtype, int incl, int cfg, RangeArgs& a, c
         // six tiles a range the finer ranges cost more than they hide (8.2e6 keys 69.6
         // us; 1.35e7 keys 95.0): those take configuration 2, 16 warps per SM in two CTAs
         // (67.0; 97.7).
-        int dev = 0, sms = 0;
+        int dev = 0, sms = 0, ctas = 0;
+        if ((e = batch_ctas_per_sm(&ctas)) != cudaSuccess) return e;
         if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
         if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-        const int seg_warps = sms * kSegWarps < kMaxRanges ? sms * kSegWarps : kMaxRanges;
-        if (a.num_tiles >= 6 * seg_warps) {
-            max_warps = seg_warps;
-        } else {
+        max_warps = batch_warps(ctas, sms, a.num_tiles);
+        if (max_warps == 0) {
             cfg = 2;  // the same 512-key tiles
             if ((e = range_max_warps(cfg, &max_warps)) != cudaSuccess) return e;
         }
