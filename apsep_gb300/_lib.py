@@ -103,10 +103,14 @@ def check(status: int, what: str = "") -> None:
 
 
 def copy_spans(srcs, dsts, nbytes, stream_handle: int) -> None:
-    """apsep_copy_spans over Python lists of addresses and byte counts."""
+    """apsep_copy_spans over Python lists of addresses (None: a null one) and byte counts."""
     n = len(srcs)
     if n == 0:
         return
-    a, b, c = array.array("Q", srcs), array.array("Q", dsts), array.array("q", nbytes)
+    if len(dsts) != n or len(nbytes) != n:  # the call reads n entries of each
+        raise ValueError("%d sources, %d destinations, %d byte counts" % (n, len(dsts), len(nbytes)))
+    a = array.array("Q", [p or 0 for p in srcs])
+    b = array.array("Q", [p or 0 for p in dsts])
+    c = array.array("q", nbytes)
     check(load().apsep_copy_spans(a.buffer_info()[0], b.buffer_info()[0], c.buffer_info()[0], n,
                                   ctypes.c_void_p(stream_handle)), "apsep_copy_spans")
