@@ -274,15 +274,15 @@ class PoolServer:
             srcs, dsts, nb = [], [], []
             a0 = ans_ring.data_ptr()
             for r in batch:
-                n = r._n
-                if r.out is None or n == 0:
+                n, out = r._n, r.out  # (its buffer as it is now: on_done may have set another one)
+                if out is None or n == 0:
                     continue
-                if r._out_ptr is not None:  # device answers: one gathered copy for the batch
+                if out.is_cuda:  # device answers: one gathered copy for the batch
                     srcs.append(a0 + 4 * r.slot)
-                    dsts.append(r._out_ptr)
+                    dsts.append(out.data_ptr())
                     nb.append(4 * n)
                 else:
-                    r.out[:n].copy_(ans_ring[r.slot:r.slot + n], non_blocking=True)
+                    out[:n].copy_(ans_ring[r.slot:r.slot + n], non_blocking=True)
             _lib.copy_spans(srcs, dsts, nb, ln.stream.cuda_stream)
         self._finish_launch(ln)
 
@@ -414,7 +414,6 @@ class PoolServer:
             r._span = pools[kind].span_size(n)
             r._dev = keys.is_cuda
             r._ptr = keys.data_ptr()
-            r._out_ptr = out.data_ptr() if out is not None and out.is_cuda else None
             r._direct = direct
         self._pools = pools
         order = sorted(requests, key=lambda r: r.arrival if realtime else 0.0)
