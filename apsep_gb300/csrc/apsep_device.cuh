@@ -224,10 +224,6 @@ __device__ __forceinline__ void copy_async16(void* smem_dst, const void* src) {
 }
 __device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-__device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)map) : "memory");
-}
-
 // ---------------------------------------------------------------------------
 // gpu-scope acquire / release on 64-bit status words, L2-only loads.
 // ---------------------------------------------------------------------------
@@ -236,19 +232,10 @@ __device__ __forceinline__ uint64_t ld_acquire_u64(const uint64_t* p) {
     asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-__device__ __forceinline__ void st_release_u64(uint64_t* p, uint64_t v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
 __device__ __forceinline__ uint32_t ld_acquire_u32(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
-}
-// Atomic add with acquire + release semantics at gpu scope; returns the old value.
-__device__ __forceinline__ uint32_t atom_add_acq_rel_u32(uint32_t* p, uint32_t v) {
-    uint32_t old;
-    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
 }
 // Fire-and-forget atomic minimum (relaxed, gpu scope).
 __device__ __forceinline__ void red_min_u64(uint64_t* p, uint64_t v) {

@@ -17,8 +17,8 @@ enum : uint32_t {
     ERR_BAD_OFFSETS = 8u,       // segment offsets not 0 = off[0] <= ... <= off[nseg] = n
 };
 
-// Look-back flag values (low 2 bits of a status word's tag).
-enum : uint32_t { FLAG_AGG = 1u, FLAG_INCL = 2u };
+// Look-back flag value (low 2 bits of a status word's tag).
+constexpr uint32_t FLAG_AGG = 1u;
 constexpr uint32_t EPOCH_LIMIT = (1u << 30) - 1u;
 
 // Run-to-run control block at the head of a plan's scratch.  Zeroed once at
@@ -45,7 +45,7 @@ struct RangeScratch {
     uint64_t* range_key;    // key[max_ranges] (packed): the range minima, for readers of the count too
     void* top_key;          // [max_ranges * kTopEntries] key: top of each range's final stack, bottom first
     int32_t* top_pos;       // [max_ranges * kTopEntries] their positions
-    uint32_t* top_cnt;      // [max_ranges] entries published | bit 31: they are the whole stack
+    uint32_t* top_cnt;      // [max_ranges] entries published
     void* tile_min;         // [cap_tiles]  key: min of each tile
     void* chunk_min;        // [cap_chunks] key: min of each 32-key chunk
     uint32_t* tile_flag;    // [cap_tiles]  flagged keys of the tile | bit 31: some are capped

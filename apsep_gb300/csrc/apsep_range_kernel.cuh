@@ -102,8 +102,6 @@ struct WLayout {
 template <int IPT, int WPC, int KB = 4, bool LEAN = false>
 constexpr size_t kernel_smem_bytes() { return WLayout<IPT, KB, LEAN>::kBytes * WPC + 1024 + 64; }  // + CTA words
 
-__device__ __forceinline__ uint32_t make_tag(uint32_t epoch, uint32_t flag) { return (epoch << 2) | flag; }
-
 // Key of a group word (the low half of an atomic minimum over ordered keys).
 template <typename T>
 __device__ __forceinline__ T group_key(const uint64_t* w) {
@@ -395,7 +393,7 @@ __device__ __noinline__ int answer_before(T q, bool want, int r, T wpm, T* sg, i
         int cnt = 0;
         __syncwarp();
         if (slot >= 0 && slot < kSlots && first == lane) {
-            cnt = (int)(__ldcg(&a.s.top_cnt[rq]) & 0xffu);
+            cnt = (int)__ldcg(&a.s.top_cnt[rq]);
             const char* tk = (const char*)((const T*)a.s.top_key + (size_t)rq * kTopEntries);
             const char* tp = (const char*)(a.s.top_pos + (size_t)rq * kTopEntries);
 #pragma unroll
@@ -1938,7 +1936,7 @@ apse_warp_kernel(const __grid_constant__ CUtensorMap map_in, const __grid_consta
                 __stcg(&top_key[lane], sStkV[(tb + lane) & (K - 1)]);
                 __stcg(&top_pos[lane], sStkP[(tb + lane) & (K - 1)]);
             }
-            if (lane == 0) __stcg(&a.s.top_cnt[r], (uint32_t)tc | ((!dropped && tb == stk_lo) ? 0x80000000u : 0u));
+            if (lane == 0) __stcg(&a.s.top_cnt[r], (uint32_t)tc);
         }
         __syncwarp();  // every lane's words before lane 0's release in range_publish
         range_publish<T>(r, epoch, rmin, a);
