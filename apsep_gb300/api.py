@@ -24,7 +24,7 @@ from ._lib import ApsepError, PlanInfo  # noqa: F401
 
 _DTYPES = {torch.int32: _lib.INT32, torch.float32: _lib.FLOAT32, torch.int64: _lib.INT64,
            torch.float64: _lib.FLOAT64}
-_WIDE = (torch.int64, torch.float64)  # 8-byte keys: single arrays, one configuration
+_WIDE = (torch.int64, torch.float64)  # 8-byte keys: one configuration index, tiles by the array's length
 
 
 # The current stream's handle without building a Stream object (2 us a call on
@@ -60,7 +60,7 @@ class Plan:
         self._h = ctypes.c_void_p()
         self._cfg = 1 if dtype in _WIDE else 0
         if dtype in _WIDE:
-            tuning = None  # one configuration for 8-byte keys
+            tuning = None  # nothing to choose for 8-byte keys
         if tuning == "default":
             from . import autotune
             tuning = autotune.load()

@@ -141,7 +141,7 @@ apsep_status apsep_plan_create(apsep_plan** out, apsep_dtype dtype, apsep_cmp cm
     p->dtype = dtype;
     p->cmp = cmp;
     p->capacity = capacity;
-    p->cfg = wide(dtype) ? 1 : 0;  // 8-byte keys: the one configuration their kernels have (8 keys per lane)
+    p->cfg = wide(dtype) ? 1 : 0;  // 8-byte keys: the one index they have (wide_tile_keys picks the tiles)
     const size_t total = carve_scratch(nullptr, capacity, nullptr, key_bytes(dtype));
     if (cudaMalloc(&p->scratch, total) != cudaSuccess) {
         cudaGetLastError();
@@ -194,7 +194,7 @@ apsep_status apsep_plan_get_info(const apsep_plan* p, apsep_plan_info* info) {
 
 apsep_status apsep_plan_set_config(apsep_plan* p, int32_t config) {
     if (!p || config < 0 || config >= kNumTileConfigs) return APSEP_EINVAL;
-    if (wide(p->dtype) && config != 1) return APSEP_ENOTSUP;  // 8-byte keys: 8 keys per lane only
+    if (wide(p->dtype) && config != 1) return APSEP_ENOTSUP;  // 8-byte keys: one index for both of their shapes
     p->cfg = config;
     return APSEP_OK;
 }

@@ -62,7 +62,7 @@ template <> struct KeyTraits<int64_t> {
 __device__ __forceinline__ int64_t f64_order(int64_t b) {
     return (b << 1) == 0 ? 0 : (b ^ ((b >> 63) & 0x7fffffffffffffffLL));
 }
-// Key maps, applied as keys enter registers or shared memory (the engine's
+// Key maps, applied as keys are read into registers (the engine's
 // KMAP template parameter): KMAP_F64 -- int64 slots holding float64 bit
 // patterns, compared through f64_order; KMAP_FLIP -- the order-reversing map
 // (integers ~x = -x - 1, floats -x; the two zeros stay equal), so that a

@@ -206,7 +206,7 @@ constexpr int batch_warps(int ctas_per_sm, int sms, int num_tiles) {
 cudaError_t batch_ctas_per_sm(int* ctas);  // their occupancy, current device (range_prepare(0))
 cudaError_t range_max_warps(int cfg, int* warps);  // persistent warps of one launch, current device
 // A single array (no view head) with int64 answers a.out_base + answer into
-// a.d_out64 (4-byte keys in configuration 0, 8-byte keys in theirs); flagged keys
+// a.d_out64 (4-byte keys in configuration 0, 8-byte keys in tiles of kWideTileKeys); flagged keys
 // get a.unanswered64 and all-deferred tiles are not written (TILE_NOT_STORED).
 cudaError_t launch_range_out64(int dtype, int incl, RangeArgs& a, const CUtensorMap& map_in, cudaStream_t st);
 // A single array (no view head, 4-byte keys) through the order-reversing key
@@ -231,17 +231,11 @@ void noalloc_debug_inject(int32_t range, uint32_t spin_limit);
 }  // namespace apsep
 
 struct apsep_plan;
-// One single-array run of the plan with int64 answers (out_base + answer into
-// d_out; see launch_range_out64): 4-byte keys in configuration 0, 8-byte keys
-// in theirs, tiles by TMA when d_in is 16-byte aligned, else by plain loads.
-// chunk_min, when not null, takes the run's minima of every 32 keys (in key
-// order, up to the end of the last tile) instead of the plan's scratch.
-// *layout returns the run's arguments: tile and range layout, scratch words.
 // One single-array run of the plan through the order-reversing key map
 // (launch_range_flipped): previous greater (span = 0) or the stock span
 // (span = 1, APSEP_LT).  APSEP_ENOTSUP when the engine has no such form for
-// the call (8-byte keys, keys or answers off a 16-byte boundary, answers over
-// the keys): the caller then takes its general route.
+// the call (8-byte keys in an array of short tiles, keys or answers off a 16-byte
+// boundary, answers over the keys): the caller then takes its general route.
 apsep_status plan_run_flipped(struct apsep_plan* plan, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp,
                               int span, void* stream);
 // One single-array run of the plan over the reversed array
@@ -252,5 +246,11 @@ apsep_status plan_run_flipped(struct apsep_plan* plan, const void* d_in, int32_t
 // its general route.
 apsep_status plan_run_reversed(struct apsep_plan* plan, const void* d_in, int32_t* d_out, int64_t n, apsep_cmp cmp,
                                void* stream);
+// One single-array run of the plan with int64 answers (out_base + answer into
+// d_out; see launch_range_out64): 4-byte keys in configuration 0, 8-byte keys
+// in tiles of kWideTileKeys, by TMA when d_in is 16-byte aligned, else by plain loads.
+// chunk_min, when not null, takes the run's minima of every 32 keys (in key
+// order, up to the end of the last tile) instead of the plan's scratch.
+// *layout returns the run's arguments: tile and range layout, scratch words.
 apsep_status plan_run_out64(struct apsep_plan* plan, const void* d_in, int64_t* d_out, int64_t n, int64_t out_base,
                             apsep_cmp cmp, void* chunk_min, void* stream, apsep::RangeArgs* layout);

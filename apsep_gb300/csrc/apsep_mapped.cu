@@ -1,6 +1,6 @@
 // apsep_mapped.cu -- the range engine in the forms the consumers ask for:
-//   * the order-reversing key map: keys are flipped as they enter shared
-//     memory or registers (integers ~x, floats -x), so one run of the
+//   * the order-reversing key map: keys are flipped as they are read from
+//     shared memory (integers ~x, floats -x), so one run of the
 //     previous-smaller engine over the unchanged input answers previous
 //     greater (or greater-or-equal under <=), and with the span output form
 //     it writes the stock span (position - previous strictly greater);

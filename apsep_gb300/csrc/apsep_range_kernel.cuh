@@ -866,8 +866,8 @@ __device__ __noinline__ void phase2(const RangeArgs& a, unsigned char* wsm, cons
     }
 }
 
-// MAPF: the key map (KMAP_*): keys pass through it as they enter shared memory
-// or registers -- float64 bit patterns in int64 slots compared through
+// MAPF: the key map (KMAP_*): keys stay as they landed in shared memory and pass
+// through it as they are read -- float64 bit patterns in int64 slots compared through
 // f64_order, or the order-reversing flip for previous-greater queries.
 // OUTM (single arrays, no view head, except OUT_I32): OUT_I64 -- answers as
 // int64, a.out_base + answer, into a.d_out64, for the int64-position path: a

@@ -2,10 +2,10 @@
 //
 // The same kernel template with 8-byte keys, keys streamed as 128-byte TMA rows
 // of 16 keys, answers as int32 positions (n < 2^31).
-// Range minima sit beside their tag words (no 64-bit key fits beside a tag
-// in one atomic word), and group minima are read from the ranges' words.
+// No 64-bit key fits beside a tag in one atomic word, so the tagged words hold
+// the tag alone and group minima are read from the ranges' minima.
 // float64 keys run as int64 through an order-preserving map of their bits
-// (applied as keys enter shared memory or registers): the FP64 compare rate
+// (applied as keys are read into registers): the FP64 compare rate
 // of this part would make every comparison the bottleneck.
 // Single arrays and segmented batches; two shapes, chosen by the length
 // (wide_tile_keys); no view head (arrays off a 16-byte boundary take plain

@@ -65,7 +65,7 @@ def main() -> None:
         def run():
             plan.run(x, out=out)
     if dt in (torch.int32, torch.float32):
-        plan.set_config(a.config)  # (8-byte keys have one configuration)
+        plan.set_config(a.config)  # (8-byte keys: one index, the length picks the tiles)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     times = []
     for _ in range(a.reps):

@@ -53,7 +53,8 @@ typedef enum apsep_status {
  * src/apsep.cuh:62-70) keep int32 positions (n <= APSEP_MAX_KEYS) and run
  * single arrays, segmented batches and the consumers (the histogram takes
  * int32 heights); apsep_run_noalloc refuses them (APSEP_EINVAL), and their
- * plans have one configuration (1). */
+ * plans have one configuration (1): tiles of 256 keys, of 512 for long
+ * arrays on a 16-byte boundary. */
 typedef enum apsep_dtype { APSEP_INT32 = 0, APSEP_FLOAT32 = 1, APSEP_INT64 = 2, APSEP_FLOAT64 = 3 } apsep_dtype;
 
 typedef enum apsep_cmp {
@@ -179,10 +180,11 @@ apsep_status apsep_noalloc_check(void* stream);
 /* ---- Consumers of APSE ------------------------------------------------------
  * The classic callers the reference names for its output (README.md:3,
  * src/bench_spt_le.cu:1-3), each one or two runs on `plan` (whose key type
- * they use; n <= its capacity) -- with 4-byte keys and 16-byte aligned keys
- * and answers the engine flips or reverses the keys as it loads them (next
- * smaller: n a multiple of 32), else memory-bound flip / reverse / mirror
- * passes around plain runs -- asynchronous on `stream` like apsep_run.  d_work: a 16-byte aligned device workspace of
+ * they use; n <= its capacity) -- with 16-byte aligned keys and answers (and,
+ * for 8-byte keys, an array long enough for their 512-key tiles) the engine
+ * reads the keys flipped or from the end (next smaller: the last n % 32 keys
+ * apart), else memory-bound flip / reverse / mirror passes around plain
+ * runs -- asynchronous on `stream` like apsep_run.  d_work: a 16-byte aligned device workspace of
  * apsep_consumer_workspace_bytes(n) bytes, not overlapping the inputs or
  * outputs.  Device-side errors of the inner runs surface through
  * apsep_plan_check. */
